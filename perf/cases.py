@@ -381,7 +381,7 @@ def _basis():
                                x * y, y * z, x * z, (y * y - z * z) * x, (z * z - x * x) * y, (x * x - y * y) * z)):
             r.append(v)
     M = _t(rows)
-    return M, torch.linalg.inv(M)
+    return M, M.T / (M * M).sum(1)   # its rows are orthogonal
 
 
 def _meq(model, rho, j):
