@@ -95,46 +95,96 @@ __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float
 #endif
 }
 
-/* random-phase solenoidal field: u = sum_m a_m e_m cos(2 pi k_m.x / n + phi_m);
- * the equilibrium at rho = 1 and u into both buffers */
-__global__ void k_ens_init(const Table T, const Mode* __restrict__ modes, float* __restrict__ fA,
-                           float* __restrict__ fB, float* __restrict__ u_out) {
-    const int g = blockIdx.x;
-    if (g >= T.ntiles) return;
-    const int mi = find_member(T, g);
+/* random-phase solenoidal field: u = sum_m a_m e_m cos(2 pi k_m.x / n + phi_m),
+ * the equilibrium at rho = 1 and u into the first buffer (a step overwrites
+ * the whole of the second before anything reads it).
+ *
+ * Bound by the FP64 pipe (2 operations per clock and SM on this chip), so the
+ * sum is factored by the x wavenumber: a block takes rows of one z plane and
+ *   1. adds, per row and kx, the amplitudes (A + iB) e^{i 2 pi (ky y + kz z)/n}
+ *      of its modes (sorted by kx) into a complex Z[kx], one thread per (row,
+ *      kx) with the rows in adjacent lanes, so that a warp's lanes share their
+ *      mode list;
+ *   2. forms u(x) = sum_kx Re Z cos - Im Z sin, and u(n - x) from the same two
+ *      sums (C - S, C + S).
+ * The angles are multiples of 2 pi / n: one table of n cosines and sines per
+ * block, no cosine per node and mode.  About 3 (kmax + 1) + 12 modes / n FP64
+ * operations per node instead of a cosine and 3 products for every mode:
+ * eight boxes of sides 48 to 128 (7.1 M nodes, some 300 modes each) took
+ * 143 ms that way. */
+constexpr int INIT_THREADS = 256;
+__global__ void __launch_bounds__(INIT_THREADS) k_ens_init(const Table T, const KMode* __restrict__ modes,
+                                                           float* __restrict__ fA, int mi, int rows) {
+    extern __shared__ double ism[];
     const Member& M = T.m[mi];
-    const int local = g - M.tile0, per_z = M.tiles_x * M.tiles_y;
-    const int z = local / per_z, r = local - z * per_z;
-    const int y = (r / M.tiles_x) * T.ty + (threadIdx.x >> 5), x = (r % M.tiles_x) * 32 + (threadIdx.x & 31);
-    const int n = M.n;
-    if (x >= n || y >= n) return;
-    double u[3] = {0, 0, 0};
-    for (int k = M.mode0; k < M.mode0 + M.nmodes; ++k) {
-        const Mode md = modes[k];
-        long long ph = (long long)md.k[0] * x + (long long)md.k[1] * y + (long long)md.k[2] * z;
-        ph %= n;
-        if (ph < 0) ph += n;
-        const double c = cospi(2.0 * double(ph) / n + md.phase);
-        u[0] += md.a[0] * c;
-        u[1] += md.a[1] * c;
-        u[2] += md.a[2] * c;
+    const int n = M.n, nk = M.kmax + 1;
+    double2* tab = reinterpret_cast<double2*>(ism); /* cos, sin of 2 pi i / n */
+    double* Z = ism + 2 * n;                        /* [kx][6][rows]: Re x y z, Im x y z */
+    const int z = blockIdx.y, y0 = blockIdx.x * rows;
+    for (int i = threadIdx.x; i < n; i += INIT_THREADS) {
+        double sn, cs;
+        sincospi(2.0 * i / n, &sn, &cs);
+        tab[i] = make_double2(cs, sn);
     }
-    const unsigned pitch = unsigned(M.pitch), plane = unsigned(n) * pitch, qs = plane * unsigned(n);
-    const unsigned c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
-    const float ux = float(u[0]), uy = float(u[1]), uz = float(u[2]);
-    const float usq = ux * ux + uy * uy + uz * uz;
+    __syncthreads();
+    for (int i = threadIdx.x; i < nk * rows; i += INIT_THREADS) {
+        const int kx = i / rows, r = i - kx * rows, y = min(y0 + r, n - 1);
+        double re[3] = {0, 0, 0}, im[3] = {0, 0, 0};
+        /* the member's modes of this kx: [lower bound, upper bound) of the sorted list */
+        int lo = M.mode0, hi = M.mode0 + M.nmodes;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (modes[mid].k[0] < kx) lo = mid + 1;
+            else hi = mid;
+        }
+        for (int m = lo; m < M.mode0 + M.nmodes && modes[m].k[0] == kx; ++m) {
+            int ph = int(((long long)modes[m].k[1] * y + (long long)modes[m].k[2] * z) % n);
+            if (ph < 0) ph += n;
+            const double2 w = tab[ph];
 #pragma unroll
-    for (int q = 0; q < 19; ++q) {
-        const float cu = float(cx(q)) * ux + float(cy(q)) * uy + float(cz(q)) * uz;
-        const float fe = wq(q) * (1.f + 3.f * cu + 4.5f * cu * cu - 1.5f * usq);
-        fA[M.off + q * qs + c] = fe;
-        fB[M.off + q * qs + c] = fe;
+            for (int k = 0; k < 3; ++k) {
+                const double a = modes[m].re[k], b = modes[m].im[k];
+                re[k] += a * w.x - b * w.y;
+                im[k] += a * w.y + b * w.x;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            Z[(6 * kx + k) * rows + r] = re[k];
+            Z[(6 * kx + 3 + k) * rows + r] = im[k];
+        }
     }
-    if (u_out) {
-        const size_t o = M.uoff + (size_t(z) * n + y) * n + x, nn = size_t(n) * n * n;
-        u_out[o] = ux;
-        u_out[o + nn] = uy;
-        u_out[o + 2 * nn] = uz;
+    __syncthreads();
+    const unsigned pitch = unsigned(M.pitch), plane = unsigned(n) * pitch, qs = plane * unsigned(n);
+    const int half = n / 2 + 1;
+    for (int i = threadIdx.x; i < rows * half; i += INIT_THREADS) {
+        const int r = i / half, x = i - r * half, y = y0 + r;
+        if (y >= n) break;
+        double C[3] = {0, 0, 0}, S[3] = {0, 0, 0};
+        int ph = 0;
+        for (int kx = 0; kx < nk; ++kx) {
+            const double2 w = tab[ph];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                C[k] += Z[(6 * kx + k) * rows + r] * w.x;
+                S[k] += Z[(6 * kx + 3 + k) * rows + r] * w.y;
+            }
+            ph += x;
+            if (ph >= n) ph -= n;
+        }
+        for (int side = 0; side < 2; ++side) {
+            const int xx = side ? n - x : x;
+            if (side && (x == 0 || xx == x)) break;
+            const double sg = side ? 1.0 : -1.0;
+            const float ux = float(C[0] + sg * S[0]), uy = float(C[1] + sg * S[1]), uz = float(C[2] + sg * S[2]);
+            const float usq = ux * ux + uy * uy + uz * uz;
+            const unsigned c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(xx);
+#pragma unroll
+            for (int q = 0; q < 19; ++q) {
+                const float cu = float(cx(q)) * ux + float(cy(q)) * uy + float(cz(q)) * uz;
+                fA[M.off + q * qs + c] = wq(q) * (1.f + 3.f * cu + 4.5f * cu * cu - 1.5f * usq);
+            }
+        }
     }
 }
 
@@ -165,6 +215,19 @@ __global__ void k_ens_init_from(const Table T, const float* __restrict__ u, floa
     }
 }
 
+/* density and momentum of the node whose population 0 is at f */
+__device__ __forceinline__ void node_moments(const float* __restrict__ f, unsigned qs, float& rho, float j[3]) {
+    rho = j[0] = j[1] = j[2] = 0;
+#pragma unroll
+    for (int q = 0; q < 19; ++q) {
+        const float v = f[q * qs];
+        rho += v;
+        if (cx(q)) j[0] += float(cx(q)) * v;
+        if (cy(q)) j[1] += float(cy(q)) * v;
+        if (cz(q)) j[2] += float(cz(q)) * v;
+    }
+}
+
 /* velocity j / rho of every member into the compact buffer at Member::uoff */
 __global__ void k_ens_velocity(const Table T, const float* __restrict__ f, float* __restrict__ u) {
     const int g = blockIdx.x;
@@ -178,41 +241,48 @@ __global__ void k_ens_velocity(const Table T, const float* __restrict__ f, float
     if (x >= n || y >= n) return;
     const unsigned pitch = unsigned(M.pitch), plane = unsigned(n) * pitch, qs = plane * unsigned(n);
     const unsigned c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
-    float rho = 0, jx = 0, jy = 0, jz = 0;
-#pragma unroll
-    for (int q = 0; q < 19; ++q) {
-        const float v = f[M.off + q * qs + c];
-        rho += v;
-        if (cx(q)) jx += float(cx(q)) * v;
-        if (cy(q)) jy += float(cy(q)) * v;
-        if (cz(q)) jz += float(cz(q)) * v;
-    }
+    float rho, j[3];
+    node_moments(f + M.off + c, qs, rho, j);
     const size_t o = M.uoff + (size_t(z) * n + y) * n + x, nn = size_t(n) * n * n;
-    u[o] = jx / rho;
-    u[o + nn] = jy / rho;
-    u[o + 2 * nn] = jz / rho;
+    u[o] = j[0] / rho;
+    u[o + nn] = j[1] / rho;
+    u[o + 2 * nn] = j[2] / rho;
 }
 
 /* per-member kinetic energy 1/2 <|u|^2> over the nodes, FP64, from the
- * compact velocities: one block per member, fixed order */
-__global__ void k_ens_energy(const Table T, const float* __restrict__ u, double* __restrict__ out) {
-    const int mi = blockIdx.x;
-    if (mi >= T.count) return;
-    const Member& M = T.m[mi];
-    const size_t nn = size_t(M.n) * M.n * M.n;
+ * populations (u = j / rho in FP32, as k_ens_velocity): ENERGY_BLOCKS block
+ * partials per member, one warp per row, summed by k_ens_energy_final in a
+ * fixed order.  Bound by the one read of the populations */
+__global__ void __launch_bounds__(256) k_ens_energy(const Table T, const float* __restrict__ f,
+                                                    double* __restrict__ part) {
+    const Member& M = T.m[blockIdx.y];
+    const int n = M.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned pitch = unsigned(M.pitch), qs = unsigned(n) * unsigned(n) * pitch;
     double s = 0;
-    for (size_t i = threadIdx.x; i < nn; i += blockDim.x) {
-        const double a = u[M.uoff + i], b = u[M.uoff + nn + i], c = u[M.uoff + 2 * nn + i];
-        s += a * a + b * b + c * c;
-    }
-    __shared__ double red[256];
-    red[threadIdx.x] = s;
+    for (int row = blockIdx.x * 8 + warp; row < n * n; row += ENERGY_BLOCKS * 8)
+        for (int x = lane; x < n; x += 32) {
+            float rho, j[3];
+            node_moments(f + M.off + unsigned(row) * pitch + x, qs, rho, j);
+            const double a = j[0] / rho, b = j[1] / rho, c = j[2] / rho;
+            s += a * a + b * b + c * c;
+        }
+    __shared__ double red[8];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) red[warp] = s;
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (int(threadIdx.x) < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = 0;
+        for (int w = 0; w < 8; ++w) v += red[w];
+        part[blockIdx.y * ENERGY_BLOCKS + blockIdx.x] = v;
     }
-    if (threadIdx.x == 0) out[mi] = 0.5 * red[0] / double(nn);
+}
+__global__ void __launch_bounds__(32) k_ens_energy_final(const Table T, const double* __restrict__ part,
+                                                         double* __restrict__ out) {
+    const int mi = blockIdx.x, n = T.m[mi].n;
+    double s = 0;
+    for (int i = threadIdx.x; i < ENERGY_BLOCKS; i += 32) s += part[mi * ENERGY_BLOCKS + i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[mi] = 0.5 * s / (double(n) * n * n);
 }
 
 /* 2x2x2 box filter of one fine member's velocity (compact [3][n][n][n]) onto
@@ -371,9 +441,20 @@ int ens_step_occupancy(int ty, int sgs) {
     return nb < 1 ? 1 : nb;
 }
 
-cudaError_t launch_ens_init(const ens::Table& T, const ens::Mode* modes, float* fA, float* fB, float* u_out,
-                            cudaStream_t s) {
-    ens::k_ens_init<<<T.ntiles, 32 * T.ty, 0, s>>>(T, modes, fA, fB, u_out);
+cudaError_t launch_ens_init(const ens::Table& T, const ens::KMode* modes, float* fA, cudaStream_t s) {
+    /* rows of a block: as many as 64 KB hold, so that three blocks share an
+     * SM (32 at kmax 16; one row always fits: n <= 1024, kmax <= 512) */
+    constexpr size_t BUDGET = 64 * 1024;
+    cudaError_t e = cudaFuncSetAttribute(ens::k_ens_init, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BUDGET));
+    if (e != cudaSuccess) return e;
+    for (int m = 0; m < T.count; ++m) {
+        const ens::Member& M = T.m[m];
+        const size_t table = size_t(M.n) * 2 * sizeof(double), row = size_t(M.kmax + 1) * 6 * sizeof(double);
+        int rows = 32;
+        while (rows > 1 && table + rows * row > BUDGET) rows /= 2;
+        ens::k_ens_init<<<dim3((M.n + rows - 1) / rows, M.n), ens::INIT_THREADS, table + rows * row, s>>>(T, modes, fA,
+                                                                                                    m, rows);
+    }
     return cudaGetLastError();
 }
 cudaError_t launch_ens_init_from(const ens::Table& T, const float* u, float* fA, float* fB, cudaStream_t s) {
@@ -384,8 +465,9 @@ cudaError_t launch_ens_velocity(const ens::Table& T, const float* f, float* u, c
     ens::k_ens_velocity<<<T.ntiles, 32 * T.ty, 0, s>>>(T, f, u);
     return cudaGetLastError();
 }
-cudaError_t launch_ens_energy(const ens::Table& T, const float* u, double* out, cudaStream_t s) {
-    ens::k_ens_energy<<<T.count, 256, 0, s>>>(T, u, out);
+cudaError_t launch_ens_energy(const ens::Table& T, const float* f, double* part, double* out, cudaStream_t s) {
+    ens::k_ens_energy<<<dim3(ens::ENERGY_BLOCKS, T.count), 256, 0, s>>>(T, f, part);
+    ens::k_ens_energy_final<<<T.count, 32, 0, s>>>(T, part, out);
     return cudaGetLastError();
 }
 cudaError_t launch_box_filter(const float* u, int n, double* ubar, double* uu, cudaStream_t s) {

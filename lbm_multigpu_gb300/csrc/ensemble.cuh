@@ -18,7 +18,8 @@ struct Member {
     unsigned long long uoff;/* element offset in the compact velocity buffer [3][n][n][n] */
     int tile0;              /* first global tile index */
     int tiles_x, tiles_y;   /* tiles per z plane */
-    int mode0, nmodes;      /* the member's rows of the mode table */
+    int mode0, nmodes;      /* the member's rows of the mode tables */
+    int kmax;               /* the largest x wavenumber of its modes */
     float tau0, omega;
 };
 
@@ -37,16 +38,27 @@ struct Mode {
     double a[3];
 };
 
+/* the same mode as the initial field's kernel reads it (a member's rows
+ * sorted by k[0], which is never negative): the velocity is the sum of
+ * Re((re + i im) e^{i 2 pi k.x / n}) */
+struct KMode {
+    int k[3];
+    double re[3], im[3];
+};
+
+/* block partials per member of the energy sum */
+constexpr int ENERGY_BLOCKS = 256;
+
 }  // namespace ens
 
 cudaError_t launch_ens_step(const ens::Table& T, const float* fA, float* fB, int sgs, const void* blob, float cs,
                             int* err, int grid, cudaStream_t s);
 int ens_step_occupancy(int ty, int sgs);
-cudaError_t launch_ens_init(const ens::Table& T, const ens::Mode* modes, float* fA, float* fB, float* u_out,
-                            cudaStream_t s);
+cudaError_t launch_ens_init(const ens::Table& T, const ens::KMode* modes, float* fA, cudaStream_t s);
 cudaError_t launch_ens_init_from(const ens::Table& T, const float* u, float* fA, float* fB, cudaStream_t s);
 cudaError_t launch_ens_velocity(const ens::Table& T, const float* f, float* u, cudaStream_t s);
-cudaError_t launch_ens_energy(const ens::Table& T, const float* u, double* out, cudaStream_t s);
+/* part: T.count * ENERGY_BLOCKS doubles */
+cudaError_t launch_ens_energy(const ens::Table& T, const float* f, double* part, double* out, cudaStream_t s);
 cudaError_t launch_box_filter(const float* u, int n, double* ubar, double* uu, cudaStream_t s);
 cudaError_t launch_d2f(const double* a, float* b, size_t n, cudaStream_t s);
 /* two passes: per-cell strain and contractions into s8 (8 * nc^3 doubles),

@@ -41,7 +41,8 @@ struct lbm_ensemble {
     double* ubar = nullptr; /* filter scratch, sized for the largest member */
     double* uu = nullptr;
     double* s8 = nullptr;
-    ens::Mode* modes = nullptr;
+    std::vector<ens::Mode> modes;
+    ens::KMode* kmodes = nullptr; /* the same, sorted by kx per member */
     unsigned char* blob = nullptr;
     int* err = nullptr;
     double* energy = nullptr;
@@ -252,7 +253,7 @@ int lbm_ensemble_create(int count, const int* sizes, const float* tau0, int sgs,
         cudaMalloc(&e->ubar, maxc * 3 * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&e->uu, maxc * 6 * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&e->s8, maxc * 8 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&e->err, sizeof(int)) != cudaSuccess || cudaMalloc(&e->energy, ens::MAXM * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&e->err, sizeof(int)) != cudaSuccess || cudaMalloc(&e->energy, size_t(count) * (1 + ens::ENERGY_BLOCKS) * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&e->blob, sgs::BLOB_BYTES) != cudaSuccess)
         return bail(set_error(LBM_ERR_CUDA, "ensemble: buffers", cudaGetLastError()));
     cudaMemset(e->err, 0, sizeof(int));
@@ -277,7 +278,7 @@ int lbm_ensemble_destroy(lbm_ensemble* e) {
     cudaFree(e->ubar);
     cudaFree(e->uu);
     cudaFree(e->s8);
-    cudaFree(e->modes);
+    cudaFree(e->kmodes);
     cudaFree(e->blob);
     cudaFree(e->err);
     cudaFree(e->energy);
@@ -291,17 +292,30 @@ int lbm_ensemble_destroy(lbm_ensemble* e) {
 int lbm_ensemble_init_turbulence(lbm_ensemble* e, uint32_t seed, float u_rms, int kmax_div, int per_shell) {
     if (!e || !(u_rms >= 0) || kmax_div < 2 || per_shell < 1) return set_error(LBM_ERR_ARG, "bad argument", cudaSuccess);
     std::vector<ens::Mode> all;
+    std::vector<ens::KMode> sorted;
     for (int m = 0; m < e->T.count; ++m) {
         ens::Member& M = e->T.m[m];
         M.mode0 = int(all.size());
         make_modes(M.n, std::max(1, M.n / kmax_div), per_shell, (uint64_t(seed) << 8) + uint64_t(m), u_rms, all);
         M.nmodes = int(all.size()) - M.mode0;
+        M.kmax = 0;
+        for (int i = M.mode0; i < int(all.size()); ++i) {
+            const ens::Mode& md = all[i];
+            const double c = std::cos(M_PI * md.phase), s = std::sin(M_PI * md.phase);
+            sorted.push_back({{md.k[0], md.k[1], md.k[2]},
+                              {md.a[0] * c, md.a[1] * c, md.a[2] * c},
+                              {md.a[0] * s, md.a[1] * s, md.a[2] * s}});
+            M.kmax = std::max(M.kmax, md.k[0]);
+        }
+        std::stable_sort(sorted.begin() + M.mode0, sorted.end(),
+                         [](const ens::KMode& a, const ens::KMode& b) { return a.k[0] < b.k[0]; });
     }
-    cudaFree(e->modes);
-    e->modes = nullptr;
-    ENS_TRY(cudaMalloc(&e->modes, std::max<size_t>(1, all.size()) * sizeof(ens::Mode)), "modes");
-    ENS_TRY(cudaMemcpy(e->modes, all.data(), all.size() * sizeof(ens::Mode), cudaMemcpyHostToDevice), "modes");
-    ENS_TRY(launch_ens_init(e->T, e->modes, e->f[0], e->f[1], e->u, e->stream), "turbulence init");
+    cudaFree(e->kmodes);
+    e->kmodes = nullptr;
+    ENS_TRY(cudaMalloc(&e->kmodes, std::max<size_t>(1, sorted.size()) * sizeof(ens::KMode)), "modes");
+    ENS_TRY(cudaMemcpy(e->kmodes, sorted.data(), sorted.size() * sizeof(ens::KMode), cudaMemcpyHostToDevice), "modes");
+    e->modes = std::move(all);
+    ENS_TRY(launch_ens_init(e->T, e->kmodes, e->f[0], e->stream), "turbulence init");
     e->cur = 0;
     e->steps = 0;
     return sync_check(e);
@@ -311,9 +325,7 @@ int lbm_ensemble_modes(const lbm_ensemble* e, int member, int* k3, double* phase
     if (!e || member < 0 || member >= e->T.count || !n) return set_error(LBM_ERR_ARG, "bad argument", cudaSuccess);
     const ens::Member& M = e->T.m[member];
     *n = M.nmodes;
-    if (!e->modes || M.nmodes == 0) return LBM_OK;
-    std::vector<ens::Mode> mm(M.nmodes);
-    ENS_TRY(cudaMemcpy(mm.data(), e->modes + M.mode0, M.nmodes * sizeof(ens::Mode), cudaMemcpyDeviceToHost), "modes");
+    const ens::Mode* mm = e->modes.data() + M.mode0;
     for (int i = 0; i < M.nmodes && i < cap; ++i) {
         for (int j = 0; j < 3; ++j) {
             if (k3) k3[3 * i + j] = mm[i].k[j];
@@ -441,8 +453,7 @@ int lbm_ensemble_info(const lbm_ensemble* e, int* ty, int* grid, long long* cell
 
 int lbm_ensemble_energy(lbm_ensemble* e, double* E) {
     if (!e || !E) return set_error(LBM_ERR_ARG, "bad argument", cudaSuccess);
-    ENS_TRY(launch_ens_velocity(e->T, e->f[e->cur], e->u, e->stream), "velocity");
-    ENS_TRY(launch_ens_energy(e->T, e->u, e->energy, e->stream), "energy");
+    ENS_TRY(launch_ens_energy(e->T, e->f[e->cur], e->energy + e->T.count, e->energy, e->stream), "energy");
     ENS_TRY(cudaMemcpyAsync(E, e->energy, e->T.count * sizeof(double), cudaMemcpyDeviceToHost, e->stream), "read");
     return sync_check(e);
 }

@@ -46,6 +46,21 @@ def test_turbulence_init_matches_modes(product):
             assert abs(slope + 5 / 3) < 0.05, slope
 
 
+@pytest.mark.parametrize("n,kmax_div,per_shell", [(8, 2, 40), (10, 5, 1), (34, 2, 24), (100, 8, 24), (32, 16, 3)])
+def test_turbulence_init_and_energy_over_sizes(product, n, kmax_div, per_shell):
+    """the factored sum over the modes (block rows that do not divide n, many
+    and single x wavenumbers) and the energy of two unequal members"""
+    with product.Ensemble([n, 16], 0.52) as e:
+        e.init_turbulence(seed=11, u_rms=0.04, kmax_div=kmax_div, per_shell=per_shell)
+        want = _field(n, *e.modes(0))
+        u = [e.velocity(m) for m in range(2)]
+        np.testing.assert_allclose(u[0], want, atol=2e-7)
+        e.step(3)
+        u = [e.velocity(m).astype(np.float64) for m in range(2)]
+        # the same FP32 velocities, summed in FP64 in another order
+        np.testing.assert_allclose(e.energy(), [0.5 * (v ** 2).sum(0).mean() for v in u], rtol=1e-12)
+
+
 @pytest.mark.parametrize("sgs,les", [("none", 0), ("smagorinsky", 1)])
 def test_ensemble_step_matches_oracle(product, sgs, les):
     lbm = product
