@@ -97,6 +97,34 @@ def test_mlp_predict_matches_oracle(product):
     np.testing.assert_allclose(nu.cpu().numpy(), want, rtol=2e-5, atol=1e-10)
 
 
+@pytest.mark.parametrize("n,shift", [(1, 0), (63, 1), (65, 0), (64 * 304 + 17, 3)])
+def test_mlp_tiles_match_oracle(product, n, shift):
+    """gradient and prediction where a tile of samples ends, where a block
+    takes a second tile, and with samples off a 16-byte boundary"""
+    torch = pytest.importorskip("torch")
+    lib = product.library()
+    P = _params(lib, 13)
+    P[NH * NIN + NH * NH: NH * NIN + NH * NH + NH] = 0.05
+    X, T = _data(n, 21)
+    room = torch.zeros(n * NIN + shift, dtype=torch.float32, device="cuda")
+    dX = room[shift:].copy_(_dev(torch, X).reshape(-1))
+    dP, dT = _dev(torch, P), _dev(torch, T)
+    g = torch.zeros(NPARAM + 1, dtype=torch.float32, device="cuda")
+    nu = torch.zeros(n, dtype=torch.float32, device="cuda")
+    at = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert lib.lbm_mlp_grad(at(dP), at(dX), at(dT), n, at(g), at(g[NPARAM:]), None) == 0, lib.lbm_last_error()
+    assert lib.lbm_mlp_predict(at(dP), at(dX), n, at(nu), None) == 0
+    torch.cuda.synchronize()
+    go, lo, want = np.zeros(NPARAM), ctypes.c_double(), np.zeros(n)
+    oracle().orc_mlp_grad(ptr(P), ptr(X), ptr(T), n, ptr(go), ctypes.byref(lo))
+    oracle().orc_mlp_forward(ptr(P), ptr(X), n, ptr(want))
+    gg = g.cpu().numpy().astype(np.float64)
+    # dot products of 16 and 64 FP32 terms: a few 1e-6 relative; the bounds of the tests above
+    assert np.linalg.norm(gg[:NPARAM] - go) <= 1e-4 * np.linalg.norm(go)
+    assert abs(gg[NPARAM] - lo.value) <= 1e-5 * lo.value
+    np.testing.assert_allclose(nu.cpu().numpy(), want, rtol=2e-5, atol=1e-10)
+
+
 def test_training_reduces_loss(product):
     torch = pytest.importorskip("torch")
     lib = product.library()
