@@ -1,8 +1,8 @@
 """Build liblbm_gb300.so in-tree (lbm_multigpu_gb300/_build/) with nvcc for sm_103a.
 
 Translation units compiled in parallel and linked into one shared library:
-the CUDA kernels (csrc/lbm_kernels.cu, and csrc/lbm_blocked.cu for the
-blocked population layout), the C ABI host side
+the CUDA kernels (csrc/lbm_kernels.cu, and csrc/sc_instance.cu once for each
+storage format and population layout of the stream-collide), the C ABI host side
 (csrc/lbm_host.cpp), the allocation-free force entry point
 (csrc/lbm_noalloc.cu), and the learned subgrid closure (csrc/sgs_mlp.cu
 kernels, csrc/lbm_sgs.cpp host side), and the ensemble of periodic boxes
@@ -38,8 +38,13 @@ def nvcc() -> str:
     raise RuntimeError("nvcc not found")
 
 
+# the stream-collide instances: name, element type, population layouts
+INSTANCES = [("f32", "float", 0), ("f16", "__half", 0), ("bf16", "__nv_bfloat16", 0), ("f64", "double", 0),
+             ("f32", "float", 1), ("f16", "__half", 1), ("bf16", "__nv_bfloat16", 1)]
+
+
 def sources() -> list[Path]:
-    return [CSRC / "lbm_kernels.cu", CSRC / "lbm_blocked.cu", CSRC / "lbm_host.cpp", CSRC / "lbm_noalloc.cu", CSRC / "sgs_mlp.cu",
+    return [CSRC / "lbm_kernels.cu", CSRC / "sc_instance.cu", CSRC / "lbm_host.cpp", CSRC / "lbm_noalloc.cu", CSRC / "sgs_mlp.cu",
             CSRC / "lbm_sgs.cpp", CSRC / "ensemble.cu", CSRC / "lbm_ensemble.cpp", CSRC / "lbm_post.cpp"]
 
 
@@ -70,20 +75,25 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(parents=True, exist_ok=True)
     cc = nvcc()
 
-    def compile_one(src: Path) -> Path:
-        obj = BUILD / (src.name + ".o")
-        cmd = [cc, *ARCH, *NVCC_FLAGS, "-c", str(src), "-o", str(obj)]
+    units = [(src, "", []) for src in sources() if src.name != "sc_instance.cu"]
+    units += [(CSRC / "sc_instance.cu", f".{name}_{lay}", [f"-DLBM_SC_NAME={name}", f"-DLBM_SC_TYPE={typ}",
+                                                          f"-DLBM_SC_LAY={lay}"]) for name, typ, lay in INSTANCES]
+
+    def compile_one(unit) -> Path:
+        src, tag, defs = unit
+        obj = BUILD / (src.name + tag + ".o")
+        cmd = [cc, *ARCH, *NVCC_FLAGS, *defs, "-c", str(src), "-o", str(obj)]
         if src.suffix == ".cpp":
             cmd = [cc, *NVCC_FLAGS, "-x", "c++", "-c", str(src), "-o", str(obj)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {src.name}:\n{r.stdout}{r.stderr}")
+            raise RuntimeError(f"nvcc failed on {src.name}{tag}:\n{r.stdout}{r.stderr}")
         if verbose:
             print(r.stderr)
         return obj
 
-    with ThreadPoolExecutor(len(sources())) as ex:
-        objs = list(ex.map(compile_one, sources()))
+    with ThreadPoolExecutor(len(units)) as ex:
+        objs = list(ex.map(compile_one, units))
     tmp = LIB.with_suffix(f".so.{os.getpid()}.tmp")
     r = subprocess.run([cc, *ARCH, "-shared", "-o", str(tmp), *map(str, objs)], capture_output=True, text=True)
     if r.returncode != 0:

@@ -42,20 +42,58 @@ __host__ __device__ constexpr float wq(int q) {
     return q == 0 ? 1.f / 3.f : (q <= 4 || q == 9 || q == 14) ? 1.f / 18.f : 1.f / 36.f;
 }
 
-/* square root and reciprocal of the LES closure: on the device in FP32 the
+/* square root and reciprocal of the LES closure.  On the device in FP32 the
  * hardware approximations (a few ulp, far below the FP32 step-to-step
- * rounding the parity tolerance allows), IEEE otherwise */
+ * rounding the parity tolerance allows); in FP64 Newton's iteration from the
+ * FP32 approximation, which takes 5 (square root) and 4 (reciprocal)
+ * operations of the FP64 pipe.  That pipe does 2 operations per clock and SM
+ * on this chip and bounds the FP64 kernels, so the seeds change format by
+ * integer instructions (same exponent range, mantissa cut to 23 bits).
+ * Each step squares the seed's relative error of about 2^-21, so the second
+ * leaves the rounding of the last operations.  Arguments outside the FP32
+ * range take the library functions; IEEE operations on the host. */
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ bool fp32_range(double x) {
+    /* 2^-100 <= x < 2^100, read from the exponent */
+    return unsigned(__double2hiint(x)) - 0x39B00000u < 0x0C800000u;
+}
+__device__ __forceinline__ float fp32_cut(double x) {
+    return __uint_as_float(((unsigned(__double2hiint(x)) - 0x38000000u) << 3) | (unsigned(__double2loint(x)) >> 29));
+}
+__device__ __forceinline__ double fp32_wide(float x) {
+    const unsigned u = __float_as_uint(x);
+    return __hiloint2double(int((u >> 3) + 0x38000000u), int(u << 29));
+}
+__device__ __forceinline__ double newton_sqrt(double x) {
+    if (!fp32_range(x)) return sqrt(x);
+    const float r = rsqrtf(fp32_cut(x));
+    const double y = fp32_wide(r), h = fp32_wide(0.5f * r);
+    double t = x * y;
+    t = fma(fma(-t, t, x), h, t);
+    return fma(fma(-t, t, x), h, t);
+}
+__device__ __forceinline__ double newton_rcp(double x) {
+    if (!fp32_range(x)) return 1.0 / x;
+    const double y = fp32_wide(__fdividef(1.0f, fp32_cut(x)));
+    const double z = fma(fma(-x, y, 1.0), y, y);
+    return fma(fma(-x, z, 1.0), z, z);
+}
+#endif
 template <class T> __host__ __device__ __forceinline__ T lsqrt(T x) {
 #ifdef __CUDA_ARCH__
     if constexpr (sizeof(T) == 4) return x > T(0) ? x * rsqrtf(x) : T(0);
-#endif
+    else return newton_sqrt(x);
+#else
     return sqrt(x);
+#endif
 }
 template <class T> __host__ __device__ __forceinline__ T lrcp(T x) {
 #ifdef __CUDA_ARCH__
     if constexpr (sizeof(T) == 4) return __fdividef(1.0f, x);
-#endif
+    else return newton_rcp(x);
+#else
     return T(1) / x;
+#endif
 }
 
 /* Smagorinsky relaxation (LR7:683-685): tau = tau0/2 + sqrt(tau0^2 + 18 sqrt2 CS Q)/2.
@@ -216,12 +254,14 @@ __host__ __device__ __forceinline__ void collide_mrt(T f[19], T omega, bool les,
 }
 
 /* the square root of a non-negative x for the deviation collision: on the
- * device x rsqrt(x + 1e-30), which is 0 at 0 without a branch */
+ * device in FP32 x rsqrt(x + 1e-30), which is 0 at 0 without a branch */
 template <class T> __host__ __device__ __forceinline__ T dsqrt(T x) {
 #ifdef __CUDA_ARCH__
     if constexpr (sizeof(T) == 4) return x * rsqrtf(x + 1e-30f);
-#endif
+    else return newton_sqrt(x);
+#else
     return sqrt(x);
+#endif
 }
 
 /* the deviation collision's opposite-pair sums and final rebuild in packed
@@ -236,6 +276,7 @@ template <class T> __host__ __device__ __forceinline__ T dsqrt(T x) {
 #endif
 #if LBM_F2_ON
 __device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 psub(float2 a, float2 b) {
     unsigned long long ra = *reinterpret_cast<unsigned long long*>(&a);
     unsigned long long rb = *reinterpret_cast<unsigned long long*>(&b), rd;
@@ -263,173 +304,235 @@ __device__ __forceinline__ float2 psub(float2 a, float2 b) {
  * jy^2 - jz^2, meq11 = jy^2 - jz^2, meq13,14,15 = jx jy, jy jz, jx jz,
  * meq10 = meq12 = meq16,17,18 = 0.
  * tau0 = 1 / omega and smag_k = 18 sqrt(2) CS are the Smagorinsky constants
- * (LR7:683-685), worked out once per launch. */
+ * (LR7:683-685), worked out once per launch.
+ *
+ * About 60 operations for the moments, 25 for the eddy viscosity and 55 for
+ * the rebuild, against some 325 in collide_mrt, which relaxes all 19 moments:
+ * in FP64, where the operations are the bound, 1.05 M nodes took 0.54 ms
+ * through collide_mrt. */
 /* the moments of collide_mrt_dev that the populations give: density and
- * momentum deviations, j^2 - U^2, the stress equilibria and the
- * non-equilibrium stress moments n1, n9, n11, n13, n14, n15 */
+ * momentum deviations, j^2 - U^2, the stress equilibria, the non-equilibrium
+ * stress moments n9, n11, n13, n14, n15 and the trace tr = n1 / 19 of Pi_neq */
 template <class T> struct MrtDev {
-    T rho, jx, jy, jz, q2, U2, m9eq, m11eq, jxy, jyz, jxz, n1, n9, n11, n13, n14, n15;
+    T rho, jx, jy, jz, q2, U2, m9eq, m11eq, jxy, jyz, jxz, tr, n9, n11, n13, n14, n15;
 };
+
+/* the products of the moments from rho and j */
+template <class T> __host__ __device__ __forceinline__ void mrt_dev_complete(MrtDev<T>& m, T U) {
+    const T Jx = m.jx + U; /* the momentum */
+    const T jxx = Jx * Jx, jyy = m.jy * m.jy, yz = m.jz * m.jz + jyy;
+    m.U2 = U * U;
+    m.q2 = (jxx - m.U2) + yz;
+    m.m9eq = T(2) * jxx - yz;
+    m.m11eq = jyy - m.jz * m.jz;
+    m.jxy = Jx * m.jy, m.jyz = m.jy * m.jz, m.jxz = Jx * m.jz;
+}
 
 /* The projected collision is linear in the deviation from any equilibrium of
  * the model at rest, so it also takes full populations with U = 0 (the
  * rest equilibrium, alpha_q rho, then cancels exactly): collide_mrt_dev(f,
  * ..., 0) is collide_mrt<MRT> up to rounding. */
-template <class T> __host__ __device__ __forceinline__ MrtDev<T> mrt_dev_moments(const T f[19], T U) {
+/* the linear parts alone (n9 .. tr without their equilibria) */
+template <class T> __host__ __device__ __forceinline__ MrtDev<T> mrt_dev_sums(const T f[19]) {
+    T sx, sy, sz, dx, dy, dz, a5, a6, a10, a11, a12, b5, b6, b10, b11, b12;
+    /* even and odd parts of the opposite pairs; in FP32 on the device two
+     * pairs per instruction */
 #if LBM_F2_ON
-    /* even and odd parts of the opposite pairs, two pairs per instruction */
-    const float2 S1 = padd(make_float2(f[1], f[2]), make_float2(f[3], f[4]));
-    const float2 D1 = psub(make_float2(f[1], f[2]), make_float2(f[3], f[4]));
-    const float2 S2 = padd(make_float2(f[9], f[5]), make_float2(f[14], f[7]));
-    const float2 D2 = psub(make_float2(f[9], f[5]), make_float2(f[14], f[7]));
-    const float2 S3 = padd(make_float2(f[6], f[10]), make_float2(f[8], f[17]));
-    const float2 D3 = psub(make_float2(f[6], f[10]), make_float2(f[8], f[17]));
-    const float2 S4 = padd(make_float2(f[12], f[11]), make_float2(f[15], f[18]));
-    const float2 D4 = psub(make_float2(f[12], f[11]), make_float2(f[15], f[18]));
-    const T sx = S1.x, sy = S1.y, dx = D1.x, dy = D1.y, sz = S2.x, a5 = S2.y, dz = D2.x, b5 = D2.y;
-    const T a6 = S3.x, a10 = S3.y, b6 = D3.x, b10 = D3.y, a12 = S4.x, a11 = S4.y, b12 = D4.x, b11 = D4.y;
-#else
-    const T sx = f[1] + f[3], dx = f[1] - f[3];
-    const T sy = f[2] + f[4], dy = f[2] - f[4];
-    const T sz = f[9] + f[14], dz = f[9] - f[14];
-    const T a5 = f[5] + f[7], b5 = f[5] - f[7];
-    const T a6 = f[6] + f[8], b6 = f[6] - f[8];
-    const T a10 = f[10] + f[17], b10 = f[10] - f[17];
-    const T a12 = f[12] + f[15], b12 = f[12] - f[15];
-    const T a11 = f[11] + f[18], b11 = f[11] - f[18];
+    if constexpr (sizeof(T) == 4) {
+        const float2 S1 = padd(make_float2(f[1], f[2]), make_float2(f[3], f[4]));
+        const float2 D1 = psub(make_float2(f[1], f[2]), make_float2(f[3], f[4]));
+        const float2 S2 = padd(make_float2(f[9], f[5]), make_float2(f[14], f[7]));
+        const float2 D2 = psub(make_float2(f[9], f[5]), make_float2(f[14], f[7]));
+        const float2 S3 = padd(make_float2(f[6], f[10]), make_float2(f[8], f[17]));
+        const float2 D3 = psub(make_float2(f[6], f[10]), make_float2(f[8], f[17]));
+        const float2 S4 = padd(make_float2(f[12], f[11]), make_float2(f[15], f[18]));
+        const float2 D4 = psub(make_float2(f[12], f[11]), make_float2(f[15], f[18]));
+        sx = S1.x, sy = S1.y, dx = D1.x, dy = D1.y, sz = S2.x, a5 = S2.y, dz = D2.x, b5 = D2.y;
+        a6 = S3.x, a10 = S3.y, b6 = D3.x, b10 = D3.y, a12 = S4.x, a11 = S4.y, b12 = D4.x, b11 = D4.y;
+    } else
 #endif
+    {
+        sx = f[1] + f[3], dx = f[1] - f[3];
+        sy = f[2] + f[4], dy = f[2] - f[4];
+        sz = f[9] + f[14], dz = f[9] - f[14];
+        a5 = f[5] + f[7], b5 = f[5] - f[7];
+        a6 = f[6] + f[8], b6 = f[6] - f[8];
+        a10 = f[10] + f[17], b10 = f[10] - f[17];
+        a12 = f[12] + f[15], b12 = f[12] - f[15];
+        a11 = f[11] + f[18], b11 = f[11] - f[18];
+    }
     const T a13 = f[13] + f[16], b13 = f[13] - f[16];
     const T axy = a5 + a6, axz = a10 + a12, ayz = a11 + a13;
-    const T sdi = axy + axz + ayz;
+    const T ax = axy + axz, sdi = ax + ayz, syz = sy + sz;
+    MrtDev<T> m;
     /* on deviations: rho - 1 and jx - U; on full populations (U = 0, the
      * model's equilibrium at rest then being the offset) rho and jx */
-    const T rho = f[0] + (sx + sy + sz) + sdi;
-    const T jx = dx + (b5 - b6) + (b10 - b12);
-    const T jy = dy + (b5 + b6) + (b11 - b13);
-    const T jz = dz + (b10 + b12) + (b11 + b13);
-    const T Jx = jx + U;                                       /* the momentum */
-    const T jxx = Jx * Jx, jyy = jy * jy, jzz = jz * jz;
-    const T U2 = U * U;
-    const T q2 = (jxx - U2) + (jyy + jzz);                     /* j^2 - U^2 */
-    const T m9eq = T(2) * jxx - (jyy + jzz), m11eq = jyy - jzz;
-    const T jxy = Jx * jy, jyz = jy * jz, jxz = Jx * jz;
-    /* stress non-equilibrium moments (the linear parts of the deviations
-     * plus those of the equilibrium at (1, U): 2 U^2 for m9, 0 else) */
-    MrtDev<T> m;
-    const T n9 = (T(2) * sx - sy - sz + axy + axz - T(2) * ayz) + (T(2) * U2 - m9eq);
-    const T n11 = (sy - sz + axy - axz) - m11eq;
-    const T n13 = (a5 - a6) - jxy, n14 = (a11 - a13) - jyz, n15 = (a10 - a12) - jxz;
-    /* n1 = 19 (sdi - f0 - j^2) with the equilibrium's 19 U^2 */
-    m.n1 = T(19) * ((sdi - f[0]) - q2);
-    m.rho = rho, m.jx = jx, m.jy = jy, m.jz = jz, m.q2 = q2, m.U2 = U2, m.m9eq = m9eq, m.m11eq = m11eq;
-    m.jxy = jxy, m.jyz = jyz, m.jxz = jxz, m.n9 = n9, m.n11 = n11, m.n13 = n13, m.n14 = n14, m.n15 = n15;
+    m.rho = f[0] + (sx + syz) + sdi;
+    m.jx = dx + (b5 - b6) + (b10 - b12);
+    m.jy = dy + (b5 + b6) + (b11 - b13);
+    m.jz = dz + (b10 + b12) + (b11 + b13);
+    m.n9 = (T(2) * sx - syz) + (ax - T(2) * ayz);
+    m.n11 = (sy - sz) + (axy - axz);
+    m.n13 = a5 - a6, m.n14 = a11 - a13, m.n15 = a10 - a12;
+    m.tr = sdi - f[0];
+    return m;
+}
+
+/* an inlet's or outlet's rebuild (extrap) of the moments' linear parts: every
+ * moment kept but the momentum, set to (u_in, 0, 0) or (0, u_in, 0), or the
+ * density, set to rho_bc; rho0 and U are the density and velocity that the
+ * populations are deviations from.  A density change d is d / 19 in every
+ * population, so m1 / 19 + 11 rho / 19 = sdi - f0 takes 11 d / 19 */
+template <class T>
+__host__ __device__ __forceinline__ void mrt_dev_extrap(MrtDev<T>& m, int type, T rho_bc, T u_in, T rho0, T U) {
+    if (type == WEST_INLET || type == SOUTH_INLET) {
+        m.jx = (type == WEST_INLET ? u_in : T(0)) - U;
+        m.jy = type == SOUTH_INLET ? u_in : T(0);
+        m.jz = T(0);
+    } else {
+        const T d = (rho_bc - rho0) - m.rho;
+        m.rho += d;
+        m.tr += d * T(11.0 / 19.0);
+    }
+}
+
+/* the products, and the non-equilibrium parts from the linear ones (plus
+ * those of the equilibrium at (1, U): 2 U^2 for m9, U^2 for tr, 0 else) */
+template <class T> __host__ __device__ __forceinline__ void mrt_dev_finish(MrtDev<T>& m, T U) {
+    mrt_dev_complete(m, U);
+    m.n9 += T(2) * m.U2 - m.m9eq;
+    m.n11 -= m.m11eq;
+    m.n13 -= m.jxy, m.n14 -= m.jyz, m.n15 -= m.jxz;
+    m.tr -= m.q2;
+}
+
+template <class T> __host__ __device__ __forceinline__ MrtDev<T> mrt_dev_moments(const T f[19], T U) {
+    MrtDev<T> m = mrt_dev_sums(f);
+    mrt_dev_finish(m, U);
     return m;
 }
 
 /* the non-equilibrium stress Pi_neq (xx, yy, zz, xy, xz, yz) from the
  * moments, as collide_mrt forms it for the Smagorinsky model: Pi_xx =
- * n1/57 + n9/3, Pi_yy + Pi_zz = n1/19 - Pi_xx, Pi_yy - Pi_zz = n11 */
+ * (tr + n9) / 3, Pi_yy + Pi_zz = tr - Pi_xx, Pi_yy - Pi_zz = n11 */
 template <class T> __host__ __device__ __forceinline__ void mrt_dev_pi(const MrtDev<T>& m, T p[6]) {
-    const T tr = m.n1 * T(1.0 / 19.0);
-    p[0] = m.n1 * T(1.0 / 57.0) + m.n9 * T(1.0 / 3.0);
-    p[1] = T(0.5) * (tr - p[0] + m.n11);
-    p[2] = T(0.5) * (tr - p[0] - m.n11);
+    p[0] = (m.tr + m.n9) * T(1.0 / 3.0);
+    p[1] = T(0.5) * ((m.tr - p[0]) + m.n11);
+    p[2] = T(0.5) * ((m.tr - p[0]) - m.n11);
     p[3] = m.n13;
     p[4] = m.n15;
     p[5] = m.n14;
 }
 
-/* the Smagorinsky relaxation rate from the moments (LR7:683-685) */
+/* the Smagorinsky relaxation rate from the moments (LR7:683-685), with
+ * Pi_yy^2 + Pi_zz^2 = ((Pi_yy + Pi_zz)^2 + (Pi_yy - Pi_zz)^2) / 2 */
 template <class T> __host__ __device__ __forceinline__ T mrt_dev_les_omega(const MrtDev<T>& m, T tau0, T smag_k) {
-    T p[6];
-    mrt_dev_pi(m, p);
-    const T qn = dsqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2] + T(2) * (p[3] * p[3] + p[4] * p[4] + p[5] * p[5]));
+    const T px = (m.tr + m.n9) * T(1.0 / 3.0), s = m.tr - px;
+    const T off = m.n13 * m.n13 + m.n14 * m.n14 + m.n15 * m.n15;
+    const T qn = dsqrt(px * px + T(0.5) * (s * s + m.n11 * m.n11) + T(2) * off);
     return lrcp(T(0.5) * tau0 + T(0.5) * dsqrt(tau0 * tau0 + smag_k * qn));
 }
 
-/* the products of the moments again from rho, j and the stresses, for a
- * caller that kept only those (fewer registers across a long wait) */
-template <class T> __host__ __device__ __forceinline__ void mrt_dev_complete(MrtDev<T>& m, T U) {
-    const T Jx = m.jx + U;
-    const T jxx = Jx * Jx, jyy = m.jy * m.jy, jzz = m.jz * m.jz;
-    m.U2 = U * U;
-    m.q2 = (jxx - m.U2) + (jyy + jzz);
-    m.m9eq = T(2) * jxx - (jyy + jzz), m.m11eq = jyy - jzz;
-    m.jxy = Jx * m.jy, m.jyz = m.jy * m.jz, m.jxz = Jx * m.jz;
-}
+/* The constants of the rebuild: rho / 19 + meq1 M1 / 2394 + meq2 M2 / 252 for
+ * the rest, axis and diagonal rows (M1 = -30, -11, 8; M2 = 12, -4, 1), a
+ * share R of rho and Q of j^2 each, and the odd parts c.j WA on the axes, c.j WD
+ * on the diagonals (j / 10 less 4 / 40, plus 1 / 40, of meq4 = -0.666666667 j
+ * as LR7 writes it).  Mass and momentum come back exactly only if
+ * R0 + 6 Ra + 12 Rd = 1, Q0 + 6 Qa + 12 Qd = 0 and 2 WA + 8 WD = 1 hold for the
+ * rounded constants too; each rounded on its own they miss by 1e-8, which a
+ * run in FP32 adds up step by step.  So the first of each sum is formed from
+ * the others, which are such that it is representable: in FP32 1 / 63 is
+ * rounded to a multiple of 2^-28 (R0 then is one of 2^-26), the others to
+ * nearest. */
+template <class T> struct DevRebuild {
+    static constexpr T WD = T(0.1 - 0.025 * 0.666666667), WA = T(0.5 - 4.0 * double(WD));
+    static constexpr T Rd = sizeof(T) == 4 ? T(4260880.0 / 268435456.0) : T(1.0 / 63.0), Ra = T(13.0 / 126.0);
+    static constexpr T R0 = T(1.0 - 6.0 * double(Ra) - 12.0 * double(Rd));
+    static constexpr T Qa = T(-209.0 / 2394.0 - 4.0 * 7.53968254 / 252.0), Qd = T(152.0 / 2394.0 + 7.53968254 / 252.0);
+    static constexpr T Q0 = T(-6.0 * double(Qa) - 12.0 * double(Qd));
+};
+static_assert(2.0 * double(DevRebuild<float>::WA) + 8.0 * double(DevRebuild<float>::WD) == 1.0, "momentum");
+static_assert(double(DevRebuild<float>::R0) + 6.0 * double(DevRebuild<float>::Ra) + 12.0 * double(DevRebuild<float>::Rd) == 1.0,
+              "mass");
+static_assert(double(DevRebuild<float>::Q0) + 6.0 * double(DevRebuild<float>::Qa) + 12.0 * double(DevRebuild<float>::Qd) == 0.0,
+              "mass, quadratic part");
 
 /* the post-collision deviations at the stress relaxation rate omega */
 template <class T> __host__ __device__ __forceinline__ void mrt_dev_relax(T f[19], const MrtDev<T>& m, T omega) {
-    const T rho = m.rho, jx = m.jx, jy = m.jy, jz = m.jz, q2 = m.q2, U2 = m.U2, m9eq = m.m9eq, m11eq = m.m11eq;
-    const T jxy = m.jxy, jyz = m.jyz, jxz = m.jxz, n9 = m.n9, n11 = m.n11, n13 = m.n13, n14 = m.n14, n15 = m.n15;
+    const T rho = m.rho, jx = m.jx, jy = m.jy, jz = m.jz, q2 = m.q2;
     const T c1 = T(1) - omega;
-    /* post-collision stresses less their value at (1, U), over the row norms */
-    const T t9 = ((m9eq - T(2) * U2) + c1 * n9) * T(1.0 / 36.0);
-    const T t11 = (m11eq + c1 * n11) * T(1.0 / 12.0);
-    const T t13 = (jxy + c1 * n13) * T(0.25), t14 = (jyz + c1 * n14) * T(0.25), t15 = (jxz + c1 * n15) * T(0.25);
-    /* rho / 19 + meq1 M1 / 2394 + meq2 M2 / 252 for the rest, axis and
-     * diagonal rows (M1 = -30, -11, 8; M2 = 12, -4, 1) */
-    const T A0 = T(1.0 / 19.0 + 330.0 / 2394.0) * rho + T(-570.0 / 2394.0 + 12.0 * 7.53968254 / 252.0) * q2;
-    const T Aa = T(1.0 / 19.0 + 121.0 / 2394.0) * rho + T(-209.0 / 2394.0 - 4.0 * 7.53968254 / 252.0) * q2;
-    const T Ad = T(1.0 / 19.0 - 88.0 / 2394.0) * rho + T(152.0 / 2394.0 + 7.53968254 / 252.0) * q2;
-    /* odd parts: c.j / 6 on the axes, c.j / 12 on the diagonals */
-    const T ox = jx * T(1.0 / 6.0), oy = jy * T(1.0 / 6.0), oz = jz * T(1.0 / 6.0);
-    const T hx = jx * T(1.0 / 12.0), hy = jy * T(1.0 / 12.0), hz = jz * T(1.0 / 12.0);
+    /* post-collision stresses less their value at (1, U), over the row norms
+     * (the shear stresses still times 4) */
+    const T t9 = ((m.m9eq - T(2) * m.U2) + c1 * m.n9) * T(1.0 / 36.0);
+    const T t11 = (m.m11eq + c1 * m.n11) * T(1.0 / 12.0);
+    const T t13 = m.jxy + c1 * m.n13, t14 = m.jyz + c1 * m.n14, t15 = m.jxz + c1 * m.n15;
+    using K = DevRebuild<T>;
+    const T A0 = K::R0 * rho + K::Q0 * q2, Aa = K::Ra * rho + K::Qa * q2, Ad = K::Rd * rho + K::Qd * q2;
+    constexpr T WA = K::WA, WD = K::WD, Q = T(0.25);
     f[0] = A0;
     const T ayz9 = Aa - t9, d9 = Ad + t9;
     const T ex = Aa + T(2) * t9, ey = ayz9 + t11, ez = ayz9 - t11;
     const T bxy = d9 + t11, bxz = d9 - t11, byz = Ad - T(2) * t9;
-    const T e5 = bxy + t13, e6 = bxy - t13, o5 = hx + hy, o6 = hy - hx;      /* xy: (5,7), (6,8) */
-    const T e10 = bxz + t15, e12 = bxz - t15, o10 = hx + hz, o12 = hz - hx;  /* xz: (10,17), (12,15) */
-    const T e11 = byz + t14, e13 = byz - t14, o11 = hy + hz, o13 = hz - hy;  /* yz: (11,18), (13,16) */
 #if LBM_F2_ON
-    {
-        const float2 E = make_float2(ex, ey), O = make_float2(ox, oy);
-        const float2 P = padd(E, O), M = psub(E, O);
-        f[1] = P.x, f[2] = P.y, f[3] = M.x, f[4] = M.y;
+    if constexpr (sizeof(T) == 4) {
+        const float2 wa = make_float2(WA, WA), na = make_float2(-WA, -WA), wd = make_float2(WD, WD),
+                     nd = make_float2(-WD, -WD), qq = make_float2(Q, -Q);
+        {
+            const float2 E = make_float2(ex, ey), O = make_float2(jx, jy);
+            const float2 P = pfma(O, wa, E), M = pfma(O, na, E);
+            f[1] = P.x, f[2] = P.y, f[3] = M.x, f[4] = M.y;
+        }
+        f[9] = ez + WA * jz;
+        f[14] = ez - WA * jz;
+        {   /* xy: (5,7), (6,8) */
+            const float2 E = pfma(make_float2(t13, t13), qq, make_float2(bxy, bxy)), O = make_float2(jx + jy, jy - jx);
+            const float2 P = pfma(O, wd, E), M = pfma(O, nd, E);
+            f[5] = P.x, f[6] = P.y, f[7] = M.x, f[8] = M.y;
+        }
+        {   /* xz: (10,17), (12,15) */
+            const float2 E = pfma(make_float2(t15, t15), qq, make_float2(bxz, bxz)), O = make_float2(jx + jz, jz - jx);
+            const float2 P = pfma(O, wd, E), M = pfma(O, nd, E);
+            f[10] = P.x, f[12] = P.y, f[17] = M.x, f[15] = M.y;
+        }
+        {   /* yz: (11,18), (13,16) */
+            const float2 E = pfma(make_float2(t14, t14), qq, make_float2(byz, byz)), O = make_float2(jy + jz, jz - jy);
+            const float2 P = pfma(O, wd, E), M = pfma(O, nd, E);
+            f[11] = P.x, f[13] = P.y, f[18] = M.x, f[16] = M.y;
+        }
+        return;
     }
-    f[9] = ez + oz;
-    f[14] = ez - oz;
-    {
-        const float2 E = make_float2(e5, e6), O = make_float2(o5, o6);
-        const float2 P = padd(E, O), M = psub(E, O);
-        f[5] = P.x, f[6] = P.y, f[7] = M.x, f[8] = M.y;
-    }
-    {
-        const float2 E = make_float2(e10, e12), O = make_float2(o10, o12);
-        const float2 P = padd(E, O), M = psub(E, O);
-        f[10] = P.x, f[12] = P.y, f[17] = M.x, f[15] = M.y;
-    }
-    {
-        const float2 E = make_float2(e11, e13), O = make_float2(o11, o13);
-        const float2 P = padd(E, O), M = psub(E, O);
-        f[11] = P.x, f[13] = P.y, f[18] = M.x, f[16] = M.y;
-    }
-#else
-    f[1] = ex + ox;
-    f[3] = ex - ox;
-    f[2] = ey + oy;
-    f[4] = ey - oy;
-    f[9] = ez + oz;
-    f[14] = ez - oz;
-    f[5] = e5 + o5;
-    f[7] = e5 - o5;
-    f[6] = e6 + o6;
-    f[8] = e6 - o6;
-    f[10] = e10 + o10;
-    f[17] = e10 - o10;
-    f[12] = e12 + o12;
-    f[15] = e12 - o12;
-    f[11] = e11 + o11;
-    f[18] = e11 - o11;
-    f[13] = e13 + o13;
-    f[16] = e13 - o13;
 #endif
+    f[1] = ex + WA * jx;
+    f[3] = ex - WA * jx;
+    f[2] = ey + WA * jy;
+    f[4] = ey - WA * jy;
+    f[9] = ez + WA * jz;
+    f[14] = ez - WA * jz;
+    const T e5 = bxy + Q * t13, e6 = bxy - Q * t13, o5 = jx + jy, o6 = jy - jx;
+    f[5] = e5 + WD * o5;
+    f[7] = e5 - WD * o5;
+    f[6] = e6 + WD * o6;
+    f[8] = e6 - WD * o6;
+    const T e10 = bxz + Q * t15, e12 = bxz - Q * t15, o10 = jx + jz, o12 = jz - jx;
+    f[10] = e10 + WD * o10;
+    f[17] = e10 - WD * o10;
+    f[12] = e12 + WD * o12;
+    f[15] = e12 - WD * o12;
+    const T e11 = byz + Q * t14, e13 = byz - Q * t14, o11 = jy + jz, o13 = jz - jy;
+    f[11] = e11 + WD * o11;
+    f[18] = e11 - WD * o11;
+    f[13] = e13 + WD * o13;
+    f[16] = e13 - WD * o13;
 }
 
+/* type: an inlet or outlet whose neighbour's populations f are (mrt_dev_extrap
+ * before the collision), or FLUID */
 template <class T>
-__host__ __device__ __forceinline__ void collide_mrt_dev(T f[19], T omega, bool les, T tau0, T smag_k, T U) {
-    const MrtDev<T> m = mrt_dev_moments(f, U);
+__host__ __device__ __forceinline__ void collide_mrt_dev(T f[19], T omega, bool les, T tau0, T smag_k, T U,
+                                                         int type = FLUID, T rho_bc = T(0), T u_in = T(0), T rho0 = T(0)) {
+    MrtDev<T> m = mrt_dev_sums(f);
+    if (type != FLUID) mrt_dev_extrap(m, type, rho_bc, u_in, rho0, U);
+    mrt_dev_finish(m, U);
     if (les) omega = mrt_dev_les_omega(m, tau0, smag_k);
     mrt_dev_relax(f, m, omega);
 }
@@ -524,14 +627,20 @@ template <class T> __host__ __device__ __forceinline__ void pi_neq(const T f[19]
     p[5] = yz - jy * jz;
 }
 
+/* the models beside LR7's MRT */
 template <class T>
-__host__ __device__ __forceinline__ void collide(int model, T f[19], T omega, bool les, T cs, T dpdy) {
+__host__ __device__ __forceinline__ void collide_other(int model, T f[19], T omega, bool les, T cs, T dpdy) {
     switch (model) {
-        case MRT: collide_mrt<MRT>(f, omega, les, cs, dpdy); break;
         case MRT_DI3: collide_mrt<MRT_DI3>(f, omega, les, cs, dpdy); break;
         case MRT_CPU3D: collide_mrt<MRT_CPU3D>(f, omega, les, cs, dpdy); break;
         default: collide_bgk(f, omega, les, cs, dpdy); break;
     }
+}
+
+template <class T>
+__host__ __device__ __forceinline__ void collide(int model, T f[19], T omega, bool les, T cs, T dpdy) {
+    if (model == MRT) collide_mrt<MRT>(f, omega, les, cs, dpdy);
+    else collide_other(model, f, omega, les, cs, dpdy);
 }
 
 /* *_Extrap rebuild (LR7:713-897): keep every moment of the neighbour's

@@ -1,9 +1,9 @@
 /*
  * lbm_kernels.cu -- CUDA kernels of the D3Q19 stream-collide path for sm_103a:
- * the structure-of-arrays instances of the stream-collide kernels
- * (sc_kernels.cuh), and every other kernel of a level in either population
- * layout (pidx): the body-force sums, init, field and population read-outs,
- * the FP64 audit, DI3's inlet control and the refinement exchange.
+ * every kernel of a level beside the stream-collide itself (sc_kernels.cuh), in
+ * either population layout (pidx): the body-force sums, init, field and
+ * population read-outs, the FP64 audit, DI3's inlet control and the refinement
+ * exchange; and the dispatch of the stream-collide over its instances.
  */
 #include <algorithm>
 #include <mutex>
@@ -608,14 +608,23 @@ TmemLane::~TmemLane() {
     g_lane_mu[dev_].unlock();
 }
 
+constexpr int storage_code_f32 = STORE_F32, storage_code_f16 = STORE_F16, storage_code_bf16 = STORE_BF16,
+              storage_code_f64 = STORE_F64;
+
 cudaError_t launch_stream_collide(const Level& L, const StepParams& p, const void* fA, void* fB, const uint8_t* mask,
                                   float* stats, float* mom_export, cudaStream_t s, const uint32_t* links) {
     if (p.halfway && !links) return cudaErrorInvalidValue;
     StepParams q = p;
     q.tau0 = 1.f / p.omega;
     q.smag_k = 18.f * 1.41421356f * p.cs;
-    if (L.blocked) return launch_sc_blocked(L, q, fA, fB, mask, stats, mom_export, s, links);
-    return launch_sc_layout<0>(L, q, fA, fB, mask, stats, mom_export, s, links);
+    q.tau0_d = 1.0 / double(p.omega);
+    q.smag_k_d = 18.0 * 1.4142135623730951 * double(p.cs);
+    const int code = L.storage + (L.blocked ? 8 : 0);
+#define LBM_SC_GO(NAME, LAY) \
+    if (code == storage_code_##NAME + 8 * LAY) return launch_sc_##NAME##_##LAY(L, q, fA, fB, mask, stats, mom_export, s, links);
+    LBM_SC_INSTANCES(LBM_SC_GO)
+#undef LBM_SC_GO
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_stream_collide_mlp(const Level& L, const StepParams& p, const void* fA, void* fB,
@@ -625,8 +634,13 @@ cudaError_t launch_stream_collide_mlp(const Level& L, const StepParams& p, const
         return cudaErrorInvalidValue;
     TmemLane lane(s);
     if (lane.status() != cudaSuccess) return lane.status();
-    if (L.blocked) return launch_sc_mlp_blocked(L, p, fA, fB, mask, stats, links, blob, err, lane.stream());
-    return launch_sc_mlp_layout<0>(L, p, fA, fB, mask, stats, links, blob, err, lane.stream());
+    const int code = L.storage + (L.blocked ? 8 : 0);
+#define LBM_SC_GO(NAME, LAY)                    \
+    if (code == storage_code_##NAME + 8 * LAY) \
+        return launch_sc_mlp_##NAME##_##LAY(L, p, fA, fB, mask, stats, links, blob, err, lane.stream());
+    LBM_SC_INSTANCES(LBM_SC_GO)
+#undef LBM_SC_GO
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_dyn_control(const Level& L, const void* f, int y1, float umax, float kp, float dpdy0_abs,

@@ -120,6 +120,7 @@ struct StepParams {
     /* derived by launch_stream_collide: 1 / omega and 18 sqrt(2) cs, the
      * constants of the Smagorinsky relaxation (LR7:683-685) */
     float tau0, smag_k;
+    double tau0_d, smag_k_d; /* the same for FP64 storage */
     /* dynamic inlet (DI3): when dpdy_dev is set the body force is read from
      * the device (the P-control updates it there); nodes with y > dyn_y1 get
      * no body force (DI3:1358) */

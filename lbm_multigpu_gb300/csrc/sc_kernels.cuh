@@ -1,9 +1,8 @@
 /*
  * sc_kernels.cuh -- the stream-collide kernels, templated on the storage
  * format S and on the population layout LAY (Level::blocked: structure of
- * arrays, or blocks of 32 nodes).  lbm_kernels.cu instantiates the
- * structure-of-arrays kernels and lbm_blocked.cu the blocked ones, so that
- * the two sets compile in parallel.
+ * arrays, or blocks of 32 nodes).  sc_instance.cu is compiled once per format
+ * and layout, so that the sets build in parallel.
  *
  * k_stream_collide is the hot kernel: one thread per lattice node, a warp
  * spans 32 consecutive x of one row, so every population load and store of a
@@ -171,9 +170,13 @@ __device__ __forceinline__ void store19(const Level& L, S* __restrict__ f, const
  * the node types present, so a channel kernel carries no lid code (whose
  * 19-entry temporaries would otherwise set every variant's register count) */
 constexpr int FEAT_HALFWAY = 1, FEAT_LID = 2, FEAT_CLAMP = 4, FEAT_XBC = 8;
-/* FP16 / BF16 with LR7's MRT and no body force: the deviation collision
- * only (other models convert to populations and back) */
+/* LR7's MRT model (which takes no body force): the projected collision
+ * collide_mrt_dev only, on the stored deviations of FP16 / BF16 (the other
+ * models convert those to populations and back) and on the populations of
+ * FP64, whose bound is the FP64 pipe (1.05 M nodes: 0.54 ms through
+ * collide_mrt, 0.30 ms so).  Not FP32, whose kernels are bound by memory */
 constexpr int FEAT_DEVMRT = 16;
+template <class S> __host__ __device__ constexpr bool sc_has_devmrt() { return sizeof(S) != 4; }
 /* the relaxation time of each node from the learned closure's last refresh
  * (StepParams::nu) instead of the LES setting */
 constexpr int FEAT_NUBUF = 32;
@@ -192,12 +195,16 @@ constexpr int FEAT_NUBUF = 32;
 #endif
 
 /* the collision, statistics, store and moment export of a non-solid node;
- * f holds populations, or for DEV their stored deviations */
+ * f holds populations, or for DEV their stored deviations.  With DEVMRT an
+ * inlet's or outlet's rebuild (bc, uin; FLUID otherwise) is part of the
+ * collision: it only replaces the density or the momentum, which the
+ * projected collision has by then, and f is its neighbour's as stored */
 template <class S, int LAY, bool DEVMRT, bool NUBUF>
 __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParams& p, S* __restrict__ fB,
                                                  float* __restrict__ stats, float* __restrict__ mom_export,
                                                  const NodeIdx<LAY>& n, typename Fmt<S>::T f[19], unsigned c,
-                                                 const int x, const int y, const int z) {
+                                                 const int x, const int y, const int z, const int bc,
+                                                 const typename Fmt<S>::T uin) {
     using T = typename Fmt<S>::T;
     constexpr bool DEV = LBM_SC_DEV && sizeof(S) == 2;
     const unsigned qs = unsigned(L.qstride);
@@ -205,8 +212,11 @@ __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParam
      * refresh, or the configured relaxation */
     const float om = NUBUF ? 1.f / (p.tau0 + 3.f * p.nu[c]) : p.omega;
     const bool les = !NUBUF && p.les != 0;
-    if constexpr (DEV && DEVMRT) {
-        collide_mrt_dev<T>(f, T(om), les, T(p.tau0), T(p.smag_k), T(L.u_ref));
+    if constexpr (DEVMRT) {
+        if constexpr (sizeof(T) == 8)
+            collide_mrt_dev<T>(f, T(om), les, p.tau0_d, p.smag_k_d, T(0), bc, T(p.rho_out), uin, T(0));
+        else
+            collide_mrt_dev<T>(f, T(om), les, T(p.tau0), T(p.smag_k), T(L.u_ref), bc, T(p.rho_out), uin, T(1));
     } else {
         T dp = T(p.dpdy_dev ? *p.dpdy_dev : p.dpdy);
         if (y > p.dyn_y1) dp = T(0);
@@ -214,7 +224,8 @@ __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParam
 #pragma unroll
             for (int q = 0; q < 19; ++q) f[q] += L.off[q];
         }
-        collide<T>(p.model, f, T(om), les, T(p.cs), dp);
+        if constexpr (sc_has_devmrt<S>()) collide_other<T>(p.model, f, T(om), les, T(p.cs), dp);
+        else collide<T>(p.model, f, T(om), les, T(p.cs), dp);
         if (DEV) {
 #pragma unroll
             for (int q = 0; q < 19; ++q) f[q] -= L.off[q];
@@ -355,22 +366,29 @@ __device__ __forceinline__ void sc_finish(const Level& L, const StepParams& p, c
         if (p.exp_nx > 0) sc_export<S>(L, p, mom_export, f, x, y, z);
         return;
     } else {
+        int bc = FLUID;
+        T uin = T(p.u_in);
         if (type >= WEST_INLET && type <= NORTH_OUTLET) {
             /* rebuild from the neighbour's stored post-collision state */
             const unsigned cn = type == WEST_INLET ? c - x + xp : type == EAST_OUTLET ? c - x + xm
                               : type == SOUTH_INLET ? c + (yp - y) * pitch : c + (ym - y) * pitch;
+            constexpr bool RAW = DEV && (FEAT & FEAT_DEVMRT);
 #pragma unroll
-            for (int q = 0; q < 19; ++q) f[q] = F::ld(n.at(fA, q, cn), L.off[q]);
-            T uin = T(p.u_in);
+            for (int q = 0; q < 19; ++q)
+                f[q] = RAW ? T(F::ldr(n.at(fA, q, cn))) : F::ld(n.at(fA, q, cn), L.off[q]);
             if (p.noise_amp != 0.f) {
                 const uint32_t cell = uint32_t((z * L.ny + y) * L.nx + x);
                 const float xi = philox_uniform(p.noise_seed, cell, uint32_t(p.t));
                 uin = uin + T(p.u_in) * T(p.noise_amp) * (T(2) * T(xi) - T(1));
             }
-            extrap<T>(type, f, T(p.rho_out), uin);
-            if (DEV) {
+            if constexpr ((FEAT & FEAT_DEVMRT) != 0) {
+                bc = type;
+            } else {
+                extrap<T>(type, f, T(p.rho_out), uin);
+                if (DEV) {
 #pragma unroll
-                for (int q = 0; q < 19; ++q) f[q] -= L.off[q];
+                    for (int q = 0; q < 19; ++q) f[q] -= L.off[q];
+                }
             }
         } else if (((FEAT & FEAT_LID) && type == LID) || ((FEAT & FEAT_XBC) && type >= DIR_WEST)) {
             if (DEV) {
@@ -388,7 +406,7 @@ __device__ __forceinline__ void sc_finish(const Level& L, const StepParams& p, c
             }
         }
         sc_collide_store<S, LAY, (FEAT & FEAT_DEVMRT) != 0, (FEAT & FEAT_NUBUF) != 0>(L, p, fB, stats, mom_export, n,
-                                                                                      f, c, x, y, z);
+                                                                                      f, c, x, y, z, bc, uin);
     }
     if (p.exp_nx > 0) sc_export<S>(L, p, mom_export, f, x, y, z);
 }
@@ -406,12 +424,12 @@ __device__ __forceinline__ void sc_node(const Level& L, const StepParams& p, con
     sc_finish<S, FEAT, LAY>(L, p, fA, fB, stats, mom_export, links, nd, f);
 }
 
-template <int FEAT> __host__ __device__ constexpr int sc_min_blocks() {
-    return (FEAT & FEAT_DEVMRT) && !(FEAT & (FEAT_LID | FEAT_XBC)) ? LBM_SC_MINB : 0;
+template <class S, int FEAT> __host__ __device__ constexpr int sc_min_blocks() {
+    return sizeof(S) == 2 && (FEAT & FEAT_DEVMRT) && !(FEAT & (FEAT_LID | FEAT_XBC)) ? LBM_SC_MINB : 0;
 }
 
 template <class S, int FEAT, int LAY>
-__global__ void __launch_bounds__(SC_BX* SC_BY, sc_min_blocks<FEAT>()) k_stream_collide(const Level L, const StepParams p,
+__global__ void __launch_bounds__(SC_BX* SC_BY, sc_min_blocks<S, FEAT>()) k_stream_collide(const Level L, const StepParams p,
                                                                   const S* __restrict__ fA, S* __restrict__ fB,
                                                                   const uint8_t* __restrict__ mask,
                                                                   float* __restrict__ stats,
@@ -539,7 +557,7 @@ __global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_
         if (p.nu) p.nu[c] = nu;
         MrtDev<float> mr;
         mr.rho = keep[0], mr.jx = keep[1], mr.jy = keep[2], mr.jz = keep[3], mr.n9 = keep[4], mr.n11 = keep[5];
-        mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8], mr.n1 = 0.f;
+        mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8];
         mrt_dev_complete(mr, 0.f);
         mrt_dev_relax(f, mr, 1.f / (tau0 + 3.f * nu));
         if (p.stats_on && p.t >= p.start_av) {
@@ -570,94 +588,48 @@ __global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_
 #endif
 }
 
-#define LBM_DISPATCH3(storage, KERNEL_CALL)                                  \
-    switch (storage) {                                                       \
-        case STORE_F32: { using S = float; KERNEL_CALL; } break;             \
-        case STORE_F16: { using S = __half; KERNEL_CALL; } break;            \
-        case STORE_BF16: { using S = __nv_bfloat16; KERNEL_CALL; } break;    \
-        default: return cudaErrorInvalidValue;                               \
-    }
+/* whether launch_sc_t has a kernel of these features */
+template <class S> inline bool sc_feat_built(int feat) {
+    if (!sc_has_devmrt<S>() && (feat & FEAT_DEVMRT)) return false;
+    if (feat & FEAT_NUBUF) return sizeof(S) <= 4 && !(feat & (FEAT_LID | FEAT_CLAMP | FEAT_XBC));
+    return feat >= 0 && feat < 32;
+}
 
-/* the stream-collide launch of one layout; FP64 storage only in the
- * structure-of-arrays layout */
-template <int LAY>
-inline cudaError_t launch_sc_layout(const Level& L, const StepParams& p, const void* fA, void* fB,
-                                    const uint8_t* mask, float* stats, float* mom_export, cudaStream_t s,
-                                    const uint32_t* links) {
+/* the stream-collide launch of one storage format and layout */
+template <class S, int LAY>
+inline cudaError_t launch_sc_t(const Level& L, const StepParams& p, const void* fA, void* fB, const uint8_t* mask,
+                               float* stats, float* mom_export, cudaStream_t s, const uint32_t* links) {
     const dim3 block(SC_BX, SC_BY), grid(L.pitch / SC_BX, (L.ny + SC_BY - 1) / SC_BY, L.nz);
-    const bool reduced = L.storage == STORE_F16 || L.storage == STORE_BF16;
     const int feat = (p.halfway ? FEAT_HALFWAY : 0) | (p.has_lid ? FEAT_LID : 0) | (p.pull_clamp ? FEAT_CLAMP : 0) |
-                     (p.has_xbc ? FEAT_XBC : 0) |
-                     (reduced && p.model == MRT && p.dpdy == 0.f && !p.dpdy_dev ? FEAT_DEVMRT : 0) |
-                     (p.nu_reuse ? FEAT_NUBUF : 0);
-#define LBM_SC_CALL(FT)                                                                                          \
-    (k_stream_collide<S, FT, LAY><<<grid, block, 0, s>>>(L, p, (const S*)fA, (S*)fB, mask, stats, mom_export, \
-                                                          links))
-#define LBM_SC(FT)                                                                   \
-    if constexpr (LAY != 0) {                                                        \
-        LBM_DISPATCH3(L.storage, LBM_SC_CALL(FT))                                    \
-    } else {                                                                         \
-        if (L.storage == STORE_F64) {                                                \
-            using S = double;                                                        \
-            LBM_SC_CALL(FT);                                                         \
-        } else {                                                                     \
-            LBM_DISPATCH3(L.storage, LBM_SC_CALL(FT))                                \
-        }                                                                            \
-    }
-#define LBM_SC_DEV(FT)                                                               \
-    if (L.storage == STORE_F16) {                                                    \
-        using S = __half;                                                            \
-        LBM_SC_CALL(FT);                                                             \
-    } else {                                                                         \
-        using S = __nv_bfloat16;                                                     \
-        LBM_SC_CALL(FT);                                                             \
-    }
+                     (p.has_xbc ? FEAT_XBC : 0) | (sc_has_devmrt<S>() && p.model == MRT ? FEAT_DEVMRT : 0) | (p.nu_reuse ? FEAT_NUBUF : 0);
+    if (!sc_feat_built<S>(feat)) return cudaErrorInvalidValue;
+#define LBM_SC(FT)                                                                                                \
+    case FT:                                                                                                      \
+        k_stream_collide<S, FT, LAY><<<grid, block, 0, s>>>(L, p, (const S*)fA, (S*)fB, mask, stats, mom_export, \
+                                                            links);                                              \
+        break;
     switch (feat) {
-        case 0: LBM_SC(0); break;
-        case 1: LBM_SC(1); break;
-        case 2: LBM_SC(2); break;
-        case 3: LBM_SC(3); break;
-        case 4: LBM_SC(4); break;
-        case 5: LBM_SC(5); break;
-        case 6: LBM_SC(6); break;
-        case 7: LBM_SC(7); break;
-        /* alternate boundaries, with every combination of the others */
-        case 8: LBM_SC(8); break;
-        case 9: LBM_SC(9); break;
-        case 10: LBM_SC(10); break;
-        case 11: LBM_SC(11); break;
-        case 12: LBM_SC(12); break;
-        case 13: LBM_SC(13); break;
-        case 14: LBM_SC(14); break;
-        case 15: LBM_SC(15); break;
-        /* FP16 / BF16 with the deviation MRT collision */
-        case 16: LBM_SC_DEV(16); break;
-        case 17: LBM_SC_DEV(17); break;
-        case 18: LBM_SC_DEV(18); break;
-        case 19: LBM_SC_DEV(19); break;
-        case 20: LBM_SC_DEV(20); break;
-        case 21: LBM_SC_DEV(21); break;
-        case 22: LBM_SC_DEV(22); break;
-        case 23: LBM_SC_DEV(23); break;
-        case 24: LBM_SC_DEV(24); break;
-        case 25: LBM_SC_DEV(25); break;
-        case 26: LBM_SC_DEV(26); break;
-        case 27: LBM_SC_DEV(27); break;
-        case 28: LBM_SC_DEV(28); break;
-        case 29: LBM_SC_DEV(29); break;
-        case 30: LBM_SC_DEV(30); break;
-        case 31: LBM_SC_DEV(31); break;
-        /* the steps between refreshes of the learned closure (channels:
-         * no lid, no alternate boundaries, no clamped pulls) */
-        case 32: LBM_SC(32); break;
-        case 33: LBM_SC(33); break;
-        case 48: LBM_SC_DEV(48); break;
-        case 49: LBM_SC_DEV(49); break;
-        default: return cudaErrorInvalidValue;
+        /* every combination of half-way, lid, clamp and alternate boundaries,
+         * without and with the projected MRT */
+        LBM_SC(0) LBM_SC(1) LBM_SC(2) LBM_SC(3) LBM_SC(4) LBM_SC(5) LBM_SC(6) LBM_SC(7)
+        LBM_SC(8) LBM_SC(9) LBM_SC(10) LBM_SC(11) LBM_SC(12) LBM_SC(13) LBM_SC(14) LBM_SC(15)
+        default:
+            if constexpr (sc_has_devmrt<S>()) {
+                switch (feat) {
+                    LBM_SC(16) LBM_SC(17) LBM_SC(18) LBM_SC(19) LBM_SC(20) LBM_SC(21) LBM_SC(22) LBM_SC(23)
+                    LBM_SC(24) LBM_SC(25) LBM_SC(26) LBM_SC(27) LBM_SC(28) LBM_SC(29) LBM_SC(30) LBM_SC(31)
+                    default: break;
+                }
+            }
+            /* the steps between refreshes of the learned closure (channels:
+             * no lid, no alternate boundaries, no clamped pulls; not FP64) */
+            if constexpr (sizeof(S) == 4) {
+                switch (feat) { LBM_SC(32) LBM_SC(33) default: break; }
+            } else if constexpr (sizeof(S) == 2) {
+                switch (feat) { LBM_SC(32) LBM_SC(33) LBM_SC(48) LBM_SC(49) default: break; }
+            }
     }
 #undef LBM_SC
-#undef LBM_SC_DEV
-#undef LBM_SC_CALL
     return cudaGetLastError();
 }
 
@@ -700,30 +672,25 @@ static cudaError_t sc_mlp_t(const Level& L, const StepParams& p, const void* fA,
     return cudaGetLastError();
 }
 
-/* the closure's stream-collide launch of one layout (FP32, FP16, BF16) */
-template <int LAY>
-inline cudaError_t launch_sc_mlp_layout(const Level& L, const StepParams& p, const void* fA, void* fB,
-                                        const uint8_t* mask, float* stats, const uint32_t* links, const void* blob,
-                                        int* err, cudaStream_t s) {
-    switch (L.storage) {
-        case STORE_F32:
-            return p.halfway ? sc_mlp_t<float, true, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s)
-                             : sc_mlp_t<float, false, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s);
-        case STORE_F16:
-            return p.halfway ? sc_mlp_t<__half, true, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s)
-                             : sc_mlp_t<__half, false, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s);
-        case STORE_BF16:
-            return p.halfway ? sc_mlp_t<__nv_bfloat16, true, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s)
-                             : sc_mlp_t<__nv_bfloat16, false, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s);
-        default: return cudaErrorInvalidValue;
-    }
+/* the closure's stream-collide launch of one storage format and layout */
+template <class S, int LAY>
+inline cudaError_t launch_sc_mlp_t(const Level& L, const StepParams& p, const void* fA, void* fB, const uint8_t* mask,
+                                   float* stats, const uint32_t* links, const void* blob, int* err, cudaStream_t s) {
+    return p.halfway ? sc_mlp_t<S, true, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s)
+                     : sc_mlp_t<S, false, LAY>(L, p, fA, fB, mask, stats, links, blob, err, s);
 }
 
-/* the blocked-layout launches (lbm_blocked.cu) */
-cudaError_t launch_sc_blocked(const Level& L, const StepParams& p, const void* fA, void* fB, const uint8_t* mask,
-                              float* stats, float* mom_export, cudaStream_t s, const uint32_t* links);
-cudaError_t launch_sc_mlp_blocked(const Level& L, const StepParams& p, const void* fA, void* fB,
-                                  const uint8_t* mask, float* stats, const uint32_t* links, const void* blob, int* err,
-                                  cudaStream_t s);
+/* the instances, one storage format and layout per translation unit
+ * (sc_instance.cu, compiled once for each), so that they build in parallel */
+#define LBM_SC_INSTANCES(X) X(f32, 0) X(f16, 0) X(bf16, 0) X(f64, 0) X(f32, 1) X(f16, 1) X(bf16, 1)
+#define LBM_SC_DECLARE(NAME, LAY)                                                                                  \
+    cudaError_t launch_sc_##NAME##_##LAY(const Level& L, const StepParams& p, const void* fA, void* fB,           \
+                                         const uint8_t* mask, float* stats, float* mom_export, cudaStream_t s,    \
+                                         const uint32_t* links);                                                  \
+    cudaError_t launch_sc_mlp_##NAME##_##LAY(const Level& L, const StepParams& p, const void* fA, void* fB,       \
+                                             const uint8_t* mask, float* stats, const uint32_t* links,            \
+                                             const void* blob, int* err, cudaStream_t s);
+LBM_SC_INSTANCES(LBM_SC_DECLARE)
+#undef LBM_SC_DECLARE
 
 }  // namespace lbm

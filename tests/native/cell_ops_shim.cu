@@ -43,6 +43,23 @@ void cell_collide_mrt_dev(int les, float omega, float cs, float u, float* h, int
 void cell_pi_neq_d(const double* f, double* rho, double* p6, int n) {
     for (int i = 0; i < n; ++i) pi_neq<double>(f + 19L * i, rho[i], p6 + 6L * i);
 }
+/* an inlet / outlet rebuild of h + off and the projected collision of it: as part
+ * of the collision (fused) or extrap first; U = u */
+void cell_collide_mrt_dev_bc_d(int fused, int type, double omega, double cs, double u, double rho_bc, double u_in,
+                               const double* off, double* h, int n) {
+    const double k = 18.0 * 1.4142135623730951 * cs;
+    for (int i = 0; i < n; ++i) {
+        double* f = h + 19L * i;
+        if (fused) {
+            collide_mrt_dev<double>(f, omega, true, 1.0 / omega, k, u, type, rho_bc, u_in, 1.0);
+        } else {
+            for (int q = 0; q < 19; ++q) f[q] += off[q];
+            extrap<double>(type, f, rho_bc, u_in);
+            for (int q = 0; q < 19; ++q) f[q] -= off[q];
+            collide_mrt_dev<double>(f, omega, true, 1.0 / omega, k, u);
+        }
+    }
+}
 void cell_mrt_dev_pi_d(const double* f, double* rho, double* p6, int n) {
     for (int i = 0; i < n; ++i) {
         const MrtDev<double> m = mrt_dev_moments<double>(f + 19L * i, 0.0);

@@ -101,6 +101,20 @@ def test_projected_collision_on_full_populations(cellops, les):
     np.testing.assert_allclose(g, f, rtol=0, atol=1e-11)
 
 
+@pytest.mark.parametrize("type_", [3, 4, 5, 6])  # west inlet, east outlet, south inlet, north outlet
+@pytest.mark.parametrize("u", [0.0, 0.05])
+def test_rebuild_within_the_projected_collision(cellops, type_, u):
+    """the inlet / outlet rebuild as a change of the collision's moments
+    equals the rebuild of the populations before the collision"""
+    off = _model_eq(cellops, u)
+    _, h = _states(off, 200, 20 + type_, 0.01)
+    g = h.copy()
+    args = [ctypes.c_double(v) for v in (1 / 0.52, 0.01, u, 1.003, 0.047)]
+    for fused, a in ((0, h), (1, g)):
+        cellops.cell_collide_mrt_dev_bc_d(fused, type_, *args, _ptr(off), _ptr(a), len(a))
+    np.testing.assert_allclose(g, h, rtol=0, atol=1e-14)  # FP64 rounding of sums of 19 terms below 1
+
+
 def test_moment_stress_equals_pi_neq(cellops):
     """Pi_neq taken from the collision's moments (the closure's features)
     equals sum c c f - rho/3 I - j j of the populations (pi_neq)"""
