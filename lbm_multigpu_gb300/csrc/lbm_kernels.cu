@@ -60,8 +60,10 @@ __global__ void __launch_bounds__(256) k_dyn_control(const Level L, const S* __r
  * of inside the stream-collide kernel, so the hot kernel carries no FP64 and no
  * block barrier.  Per node the sum is FP32 (as in the reference); across nodes
  * it is FP64: per-block partials, and the last block to finish adds them in
- * block order, so the result does not depend on scheduling. */
-constexpr int FORCE_BLOCKS = 152, FORCE_THREADS = 256;
+ * block order, so the result does not depend on scheduling.  Latency-bound
+ * (a few thousand nodes): only as many blocks as the list fills, since every
+ * block's FP64 tree costs 60 operations of a pipe that does 2 per clock. */
+constexpr int FORCE_BLOCKS = 608, FORCE_THREADS = 128;
 template <class S>
 __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, const S* __restrict__ fA,
                                                               const unsigned* __restrict__ body, int nbody,
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
     using T = typename F::T;
     double s[3] = {0.0, 0.0, 0.0};
     const unsigned plane = unsigned(L.plane), pitch = unsigned(L.pitch);
-    for (int i = blockIdx.x * FORCE_THREADS + threadIdx.x; i < nbody; i += FORCE_BLOCKS * FORCE_THREADS) {
+    for (int i = blockIdx.x * FORCE_THREADS + threadIdx.x; i < nbody; i += int(gridDim.x) * FORCE_THREADS) {
         const unsigned c = body[i];
         const unsigned z = c / plane, r = c - z * plane;
         const unsigned y = r / pitch, x = r - y * pitch;
@@ -120,8 +122,10 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
         double v = 0.0;
 #pragma unroll
         for (int w = 0; w < FORCE_THREADS / 32; ++w) v += red[threadIdx.x][w];
-        part[3 * blockIdx.x + threadIdx.x] = v;
+        if (gridDim.x == 1) out3[threadIdx.x] += v;
+        else part[3 * blockIdx.x + threadIdx.x] = v;
     }
+    if (gridDim.x == 1) return;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(done, 1u) == gridDim.x - 1);
@@ -140,27 +144,16 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
     }
 }
 
-/* sum n block partials (3 doubles each) in a fixed order; one block */
-__global__ void k_reduce3(const double* __restrict__ part, int n, double* __restrict__ out) {
-    __shared__ double red[3][32];
-    double s[3] = {0.0, 0.0, 0.0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        s[0] += part[3LL * i];
-        s[1] += part[3LL * i + 1];
-        s[2] += part[3LL * i + 2];
-    }
-    for (int k = 0; k < 3; ++k) {
-        double v = s[k];
+/* add n block partials (3 doubles each) to out, in a fixed order: warp k sums
+ * component k, lane-strided, then a fixed shuffle tree */
+__global__ void __launch_bounds__(96) k_reduce3(const double* __restrict__ part, int n, double* __restrict__ out) {
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v = 0.0;
+#pragma unroll 8
+    for (int i = lane; i < n; i += 32) v += part[3LL * i + k];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double v = 0.0;
-        for (int w = 0; w < int(blockDim.x >> 5); ++w) v += red[threadIdx.x][w];
-        out[threadIdx.x] += v;
-    }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) out[k] += v;
 }
 
 /* initialize / initializeLR (LR7:1060-1125): rest state at rho = 1 with the
@@ -656,38 +649,80 @@ int force_partials() { return FORCE_BLOCKS; }
 cudaError_t launch_force(const Level& L, const void* fA, const unsigned* body, int nbody, double* partials,
                          unsigned* done, double* out3, cudaStream_t s, const uint8_t* mask, int halfway) {
     if (nbody <= 0) return cudaSuccess;
-    LBM_DISPATCH(L.storage, (k_force_list<S><<<FORCE_BLOCKS, FORCE_THREADS, 0, s>>>(L, (const S*)fA, body, nbody,
-                                                                                    partials, done, out3, mask,
-                                                                                    halfway)));
+    const int blocks = std::min(FORCE_BLOCKS, (nbody + FORCE_THREADS - 1) / FORCE_THREADS);
+    LBM_DISPATCH(L.storage, (k_force_list<S><<<blocks, FORCE_THREADS, 0, s>>>(L, (const S*)fA, body, nbody, partials,
+                                                                              done, out3, mask, halfway)));
     return cudaGetLastError();
 }
 
 /* momentum exchange by scanning the mask (the kernel-level API has no body
- * list): grid-stride over rows, FP64 per-block partials, fixed-order sum */
+ * list).  A warp takes SCAN_NODES consecutive bytes of the pitched mask, 16
+ * per lane, compacts the BODY nodes among them in order (a prefix sum over the
+ * lanes) and shares them out one per lane: a body is a dense block of the
+ * mask, which one lane per run of bytes would walk alone.  The FP64 tree runs
+ * only in blocks that found a body (it is 120 operations of a pipe that does 2
+ * per clock).  As many blocks as the mask fills, up to SCAN_BLOCKS; the order
+ * of the sums depends on the sizes alone.  At 96 x 48 x 33 this and its
+ * reduction took 13.9 + 9.7 us with a lane per byte and a tree in all of 1216
+ * blocks. */
 constexpr int SCAN_BLOCKS = 1216; /* 8 blocks per SM on a 152-SM GB300 */
-template <class S>
-__global__ void __launch_bounds__(256) k_force_scan(const Level L, const S* __restrict__ fA,
-                                                    const uint8_t* __restrict__ mask, double* __restrict__ part) {
-    using F = Fmt<S>;
+constexpr int SCAN_WARPS = 8, SCAN_NODES = 512;
+__global__ void __launch_bounds__(32 * SCAN_WARPS) k_force_scan(const Level L, const float* __restrict__ fA,
+                                                                const uint8_t* __restrict__ mask,
+                                                                double* __restrict__ part, int vec) {
+    __shared__ uint16_t list[SCAN_WARPS][SCAN_NODES];
+    __shared__ double red[3][SCAN_WARPS];
     double s[3] = {0.0, 0.0, 0.0};
-    const long long rows = (long long)L.ny * L.nz;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (long long r = (long long)blockIdx.x * 8 + warp; r < rows; r += (long long)gridDim.x * 8) {
-        const int y = int(r % L.ny), z = int(r / L.ny);
-        for (int x = lane; x < L.nx; x += 32) {
-            if ((mask[z * L.plane + (long long)y * L.pitch + x] & TYPE_MASK) != BODY) continue;
-            const int xm = (x == 0) ? L.nx - 1 : x - 1, xp = (x == L.nx - 1) ? 0 : x + 1;
-            const int ym = (y == 0) ? L.ny - 1 : y - 1, yp = (y == L.ny - 1) ? 0 : y + 1;
-            const int zm = (z == 0) ? L.nz - 1 : z - 1, zp = (z == L.nz - 1) ? 0 : z + 1;
-            const long long zb[3] = {zm * L.plane, z * L.plane, zp * L.plane};
-            const long long yb[3] = {(long long)ym * L.pitch, (long long)y * L.pitch, (long long)yp * L.pitch};
-            const int xs[3] = {xm, x, xp};
-            /* per node in the storage's arithmetic (as k_force_list), across nodes FP64 */
-            typename F::T a[3] = {0, 0, 0};
+    const unsigned total = unsigned(L.qstride), plane = unsigned(L.plane), pitch = unsigned(L.pitch);
+    const unsigned chunks = (total + SCAN_NODES - 1) / SCAN_NODES;
+    bool any = false;
+    for (unsigned ch = blockIdx.x * SCAN_WARPS + warp; ch < chunks; ch += gridDim.x * SCAN_WARPS) {
+        const unsigned c0 = ch * SCAN_NODES + 16 * lane; /* total is a multiple of 32: 16 bytes are in or out together */
+        unsigned w[4] = {0, 0, 0, 0};
+        if (c0 < total) {
+            if (vec) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(mask + c0));
+                w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) w[i >> 2] |= unsigned(mask[c0 + i]) << (8 * (i & 3));
+            }
+        }
+        /* bit i: byte i is a BODY node of the domain (not of the row padding) */
+        unsigned bits = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) bits |= unsigned(((w[i >> 2] >> (8 * (i & 3))) & TYPE_MASK) == BODY) << i;
+        const unsigned x0 = c0 % pitch;
+        const int in = L.nx - int(x0);
+        if (in < 16) bits &= in > 0 ? (1u << in) - 1u : 0u;
+        if (!__any_sync(0xffffffffu, bits)) continue;
+        any = true;
+        const int n = __popc(bits);
+        int at = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += v;
+        }
+        const int found = __shfl_sync(0xffffffffu, at, 31);
+        at -= n;
+        for (unsigned b = bits; b; b &= b - 1) list[warp][at++] = uint16_t(16 * lane + __ffs(b) - 1);
+        __syncwarp();
+        for (int i = lane; i < found; i += 32) {
+            const unsigned c = ch * SCAN_NODES + list[warp][i];
+            const unsigned z = c / plane, r = c - z * plane, y = r / pitch, x = r - y * pitch;
+            const unsigned xm = (x == 0) ? L.nx - 1 : x - 1, xp = (x == unsigned(L.nx) - 1) ? 0 : x + 1;
+            const unsigned ym = (y == 0) ? L.ny - 1 : y - 1, yp = (y == unsigned(L.ny) - 1) ? 0 : y + 1;
+            const unsigned zm = (z == 0) ? L.nz - 1 : z - 1, zp = (z == unsigned(L.nz) - 1) ? 0 : z + 1;
+            const unsigned zb[3] = {zm * plane, z * plane, zp * plane};
+            const unsigned yb[3] = {ym * pitch, y * pitch, yp * pitch};
+            const unsigned xs[3] = {xm, x, xp};
+            /* per node in FP32 (as k_force_list), across nodes FP64 */
+            float a[3] = {0, 0, 0};
 #pragma unroll
             for (int q = 1; q < 19; ++q) {
-                const typename F::T v = typename F::T(2) *
-                    F::ld(fA + pidx(L, q, unsigned(zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)])), L.off[q]);
+                const float v = 2.f * __ldg(fA + (unsigned(q) * total + zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]));
                 if (cx(q)) a[0] += cx(q) * v;
                 if (cy(q)) a[1] += cy(q) * v;
                 if (cz(q)) a[2] += cz(q) * v;
@@ -695,29 +730,36 @@ __global__ void __launch_bounds__(256) k_force_scan(const Level L, const S* __re
 #pragma unroll
             for (int k = 0; k < 3; ++k) s[k] += double(a[k]);
         }
+        __syncwarp(); /* the list is rewritten for the next chunk */
     }
-    __shared__ double red[3][8];
-    for (int k = 0; k < 3; ++k) {
-        double v = s[k];
+    if (__syncthreads_or(any)) {
+        for (int k = 0; k < 3; ++k) {
+            double v = s[k];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[k][warp] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double v = 0.0;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) red[k][warp] = v;
+        }
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            double v = 0.0;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) v += red[threadIdx.x][w];
-        part[3 * blockIdx.x + threadIdx.x] = v;
+            for (int w = 0; w < SCAN_WARPS; ++w) v += red[threadIdx.x][w];
+            part[3 * blockIdx.x + threadIdx.x] = v;
+        }
+    } else if (threadIdx.x < 3) {
+        part[3 * blockIdx.x + threadIdx.x] = 0.0;
     }
 }
 
 int force_scan_partials() { return SCAN_BLOCKS; }
 
-cudaError_t launch_force_scan(const Level& L, const void* fA, const uint8_t* mask, double* partials, double* out3,
+cudaError_t launch_force_scan(const Level& L, const float* fA, const uint8_t* mask, double* partials, double* out3,
                               cudaStream_t s) {
-    LBM_DISPATCH(L.storage, (k_force_scan<S><<<SCAN_BLOCKS, 256, 0, s>>>(L, (const S*)fA, mask, partials)));
-    k_reduce3<<<1, 1024, 0, s>>>(partials, SCAN_BLOCKS, out3);
+    if (L.storage != STORE_F32 || L.blocked) return cudaErrorInvalidValue;
+    const long long chunks = (L.qstride + SCAN_NODES - 1) / SCAN_NODES;
+    const int blocks = int(std::min<long long>(SCAN_BLOCKS, (chunks + SCAN_WARPS - 1) / SCAN_WARPS));
+    k_force_scan<<<blocks, 32 * SCAN_WARPS, 0, s>>>(L, fA, mask, partials, (reinterpret_cast<uintptr_t>(mask) & 15) == 0);
+    k_reduce3<<<1, 96, 0, s>>>(partials, blocks, out3);
     return cudaGetLastError();
 }
 

@@ -179,8 +179,9 @@ cudaError_t launch_force(const Level& L, const void* fA, const unsigned* body, i
                          unsigned* done, double* out3, cudaStream_t s, const uint8_t* mask = nullptr,
                          int halfway = 0);
 int force_partials();
-/* the same sum found by scanning the mask; partials holds force_scan_partials()*3 doubles */
-cudaError_t launch_force_scan(const Level& L, const void* fA, const uint8_t* mask, double* partials, double* out3,
+/* the same sum found by scanning the mask, of an FP32 structure-of-arrays
+ * level; partials holds force_scan_partials()*3 doubles */
+cudaError_t launch_force_scan(const Level& L, const float* fA, const uint8_t* mask, double* partials, double* out3,
                               cudaStream_t s);
 int force_scan_partials();
 

@@ -12,7 +12,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from oracle_bindings import REF_CODE, OracleRun, Refine, moments, rel_l2
+from oracle_bindings import CX, CY, CZ, REF_CODE, OracleRun, Refine, moments, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -492,6 +492,40 @@ def test_kernel_level_api_matches_handle(product):
     np.testing.assert_array_equal(fa[..., :NX].cpu().numpy(), f_ref)
     # same per-node sums, FP64 sums over nodes grouped differently
     assert abs(force[0].item() - F_ref[1, 0]) <= 1e-12 * abs(F_ref[1, 0])
+
+
+@pytest.mark.parametrize("nx,ny,nz,pitch,shift", [(20, 12, 5, 32, 0), (33, 7, 3, 64, 5), (96, 48, 33, 96, 0),
+                                                  (257, 40, 31, 288, 16)])
+def test_body_force_scan_against_numpy(product, nx, ny, nz, pitch, shift):
+    """the mask scan over scattered and dense bodies, mask buffers off a
+    16-byte boundary, domains that end inside a warp's 512 bytes, and BODY
+    bytes in the row padding (not part of the domain)"""
+    torch = pytest.importorskip("torch")
+    lib = product.library()
+    rng = np.random.default_rng(nx)
+    m = np.zeros((nz, ny, pitch), np.uint8)
+    m[rng.random(m.shape) < 0.02] = 2
+    m[:, ny // 3:ny // 2, nx // 4:nx // 2] = 2
+    m[:, :, nx:] = 2
+    f = np.zeros((19, nz, ny, pitch), np.float32)
+    f[..., :nx] = rng.random((19, nz, ny, nx), np.float32)
+    room = torch.zeros(m.size + shift, dtype=torch.uint8, device="cuda")
+    dm = room[shift:].copy_(torch.from_numpy(m.reshape(-1)).cuda())
+    df = torch.from_numpy(f).cuda()
+    force = torch.zeros(3, dtype=torch.float64, device="cuda")
+    scratch = torch.full((int(lib.lbm_body_force_scratch_doubles()),), float("nan"), dtype=torch.float64, device="cuda")
+    at = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert lib.lbm_body_force_f32(at(df), at(dm), nx, ny, nz, pitch, at(force), at(scratch), None) == 0
+    torch.cuda.synchronize()
+    g = f[..., :nx].astype(np.float64)
+    body = m[..., :nx] == 2
+    want, size = np.zeros(3), 0.0
+    for q in range(19):
+        v = 2 * np.roll(g[q], (CZ[q], CY[q], CX[q]), (0, 1, 2))[body].sum()
+        want += np.array([CX[q], CY[q], CZ[q]]) * v
+        size += v
+    # per node an FP32 sum of 18 terms (18 roundings of 2^-24 each at most), across nodes FP64
+    np.testing.assert_allclose(force.cpu().numpy(), want, rtol=0, atol=18 * 2.0 ** -24 * size)
 
 
 def test_c2_size_properties(product):
