@@ -559,6 +559,21 @@ int lbm::set_error(int code, const char* what, cudaError_t e) {
     return fail(code, "%s", what);
 }
 
+/* an executable graph of k steps and what its launches were captured with:
+ * it can be launched again as it is while all of that still holds and every
+ * parameter that changes from step to step is read from the device's step
+ * counter (steady) */
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    bool steady = false;
+    long long epoch = -1;
+    int cur1 = 0;           /* the refinement level's current buffer at the start */
+    bool force = false;     /* every step records a force (else none does) */
+    int phase = 0;          /* t modulo the closure's refresh interval at the start */
+    const float* mom = nullptr;
+    long long launches = 0; /* kernels of one replay */
+};
+
 struct lbm_handle {
     Config cfg;
     int storage = STORE_F32;
@@ -583,11 +598,16 @@ struct lbm_handle {
      * stream: forked after the previous step, joined before the next */
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    /* refinement steps are launch-bound (a dozen small launches and events
-     * each): lbm_step captures batches of steps into one CUDA graph, updated
-     * in place from batch to batch (uniform runs too: it removes the gaps
-     * between their launches) */
-    cudaGraphExec_t gexec[17] = {}; /* by batch length (GRAPH_STEPS = 16) */
+    /* lbm_step runs batches of 2, 4, 8 or 16 steps as CUDA graphs, which
+     * removes the gaps between their launches.  The step number lives on the
+     * device (step_dev, which a graph advances by its length), so that a
+     * batch is captured once and then launched again with one host call; a
+     * capture costs the host 1 to 10 us per step, more than a step of a small
+     * domain takes.  By log2 of the length and the buffer it starts from */
+    StepGraph graphs[5][2];
+    int* step_dev = nullptr;        /* behind audit_out's four sums */
+    int step_dev_val = -1;          /* its value once everything queued so far has run */
+    long long epoch = 0;            /* bumped when anything that captured launches carry changes */
     long long launches = 0;         /* kernels this handle has launched */
     /* FP32 staging of the populations of a level for lbm_get/set_populations
      * (the stored layout or precision is not the caller's), allocated on
@@ -678,6 +698,7 @@ int alloc_level(LevelState& s, int nx, int ny, int nz, int storage, int blocked,
  * full-way bounce-back, the fluid nodes next to BODY nodes for half-way. */
 int upload_mask(lbm_handle* h, int level) {
     LevelState& s = h->lv[level];
+    ++h->epoch;
     const Level& L = s.L;
     const bool clamp = h->cfg.pull_clamp, halfway = h->cfg.halfway;
     std::vector<uint8_t> pitched(size_t(L.qstride), WALL);
@@ -743,6 +764,7 @@ int ensure_force_cap(lbm_handle* h, int n) {
     }
     h->force_hist = nh;
     h->force_cap = cap;
+    ++h->epoch;
     return LBM_OK;
 }
 
@@ -809,26 +831,31 @@ int do_init(lbm_handle* h) {
  * side stream, after everything queued so far on the main stream; the caller
  * joins (waits for ev_join) once the step's stream-collide is queued.  The
  * force kernel adds into `out` (3 doubles), which is zero or holds the other
- * level's sum of the same step. */
-cudaError_t fork_force(lbm_handle* h, LevelState& s, double* out) {
+ * level's sum of the same step; with step_dev, out is the history's entry of
+ * device step 0. */
+cudaError_t fork_force(lbm_handle* h, LevelState& s, double* out, const int* step_dev) {
     cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
     if (e == cudaSuccess)
-        e = launch_force(s.L, s.f[s.cur], s.body, s.nbody, s.fpart, s.done, out, h->side, s.mask, h->cfg.halfway);
+        e = launch_force(s.L, s.f[s.cur], s.body, s.nbody, s.fpart, s.done, out, h->side, s.mask, h->cfg.halfway,
+                         step_dev);
     if (e == cudaSuccess) e = cudaEventRecord(h->ev_join, h->side);
     ++h->launches;
     return e;
 }
 
 /* one base step and, with refinement, the patch sub-steps and the two
- * interpolations; the order of LR7:2849-2950 */
-int one_step(lbm_handle* h) {
+ * interpolations; the order of LR7:2849-2950.  rel >= 0: the launches carry
+ * the step as rel steps past the device's counter instead of h->t */
+int one_step(lbm_handle* h, int rel = -1) {
     const Config& c = h->cfg;
     const int t = h->t;
+    const int* step_dev = rel >= 0 ? h->step_dev : nullptr;
     LevelState& C = h->lv[0];
     StepParams p = base_params(h, 0);
-    p.t = t;
-    p.force_on = (!c.refinement && t > c.startf) ? 1 : 0;
+    p.t = rel >= 0 ? rel : t;
+    p.step_dev = step_dev;
+    const bool force = !c.refinement && t > c.startf;
     if (c.refinement) {
         p.exp_x0 = int(c.lrx0);
         p.exp_y0 = int(c.lry0);
@@ -836,10 +863,11 @@ int one_step(lbm_handle* h) {
         p.exp_ny = h->eny;
     }
     const int fidx = t - c.startf;
-    if (p.force_on) {
-        int rc = ensure_force_cap(h, fidx + 1);
-        if (rc) return rc;
-    }
+    if (t > c.startf)
+        if (int rc = ensure_force_cap(h, fidx + 1)) return rc;
+    /* the history's entry of this step, or with the counter of its step 0 */
+    double* const fout = h->force_hist + 3LL * ((rel >= 0 ? rel : t) - c.startf);
+    const bool force0 = force && C.nbody > 0;
     if (h->trip_in_mask && t >= c.trip_end) {
         /* the trip blocks vanish (DI3's ImageFcn is false from TRIP end on) */
         CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -850,7 +878,7 @@ int one_step(lbm_handle* h) {
     }
     if (c.sgs_mlp && !h->mlp_ready)
         return fail(LBM_ERR_STATE, "SGS mlp: no weights (SGS weights record line or lbm_set_sgs_mlp)");
-    if (p.force_on) CUDA_TRY(fork_force(h, C, h->force_hist + 3LL * fidx));
+    if (force0) CUDA_TRY(fork_force(h, C, fout, step_dev));
     /* CF TIME linear: this step's export goes to the other buffer, the last
      * one is kept for the interpolation in time */
     bool blend = false;
@@ -879,7 +907,7 @@ int one_step(lbm_handle* h) {
         CUDA_TRY(launch_stream_collide(C.L, p, C.f[C.cur], C.f[1 - C.cur], C.mask, C.stats, h->mom, h->stream,
                                        C.links));
     ++h->launches;
-    if (p.force_on) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
+    if (force0) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
     C.cur = 1 - C.cur;
     if (h->dpdy_dev && c.dyny1 >= 0 && c.dyn_every > 0 && t % c.dyn_every == 0 && t > c.dyn_start &&
         h->dyn_n < h->dyn_cap) {
@@ -900,17 +928,14 @@ int one_step(lbm_handle* h) {
                 ++h->launches;
             }
             StepParams pf = base_params(h, 1);
-            pf.t = t;
-            pf.force_on = (t > c.startf && i == 0) ? 1 : 0;
-            if (pf.force_on) {
-                int rc = ensure_force_cap(h, fidx + 1);
-                if (rc) return rc;
-            }
-            if (pf.force_on) CUDA_TRY(fork_force(h, Fn, h->force_hist + 3LL * fidx));
+            pf.t = p.t;
+            pf.step_dev = step_dev;
+            const bool force1 = t > c.startf && i == 0 && Fn.nbody > 0;
+            if (force1) CUDA_TRY(fork_force(h, Fn, fout, step_dev));
             CUDA_TRY(launch_stream_collide(Fn.L, pf, Fn.f[Fn.cur], Fn.f[1 - Fn.cur], Fn.mask, Fn.stats, nullptr,
                                            h->stream, Fn.links));
             ++h->launches;
-            if (pf.force_on) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
+            if (force1) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
             Fn.cur = 1 - Fn.cur;
         }
         /* the band fill at the end of the coarse step and the restriction
@@ -923,7 +948,7 @@ int one_step(lbm_handle* h) {
     return LBM_OK;
 }
 
-constexpr int GRAPH_STEPS = 16; /* steps per captured graph */
+constexpr int GRAPH_LG = 4; /* graphs of up to 2^GRAPH_LG = 16 steps */
 
 /* k steps from h->t on can be captured: their steps call nothing that
  * synchronises (the trip leaving the mask does) or sets kernel attributes
@@ -936,13 +961,85 @@ bool graph_ok(const lbm_handle* h, int k) {
     return true;
 }
 
-/* k steps captured from the main stream into one graph (the force and
- * band-fill stream forks from it and joins it again inside every step), then
- * launched.  The executable graph of the previous batch is updated in place
- * when the topology is the same (an update leaves launches already queued as
- * they were), else instantiated anew. */
-int run_graph(lbm_handle* h, int k) {
+/* whether the k steps from h->t on can be captured with the device's step
+ * counter in place of every parameter that changes from step to step: not the
+ * dynamic inlet's control (its host-side schedule and history position), and
+ * not a batch in which the recording of the force, the time blending or the
+ * closure's first evaluation begins */
+bool steady_batch(const lbm_handle* h, int k) {
     const Config& c = h->cfg;
+    if (h->dpdy_dev) return false;
+    if (h->t <= c.startf && h->t + k - 1 > c.startf) return false;
+    if (c.refinement && c.cf_time && !h->have_mom) return false;
+    if (c.sgs_mlp && h->lv[0].nu && !h->nu_valid) return false;
+    return true;
+}
+
+/* whether any launch of a steady batch reads the counter */
+bool uses_counter(const lbm_handle* h, bool force) {
+    return force || h->cfg.noise != 0.f || h->cfg.velav || h->lv[0].has_xbc || h->lv[1].has_xbc;
+}
+
+/* the executable graph of k = 2^lg steps from h->t on, when the one at hand
+ * can be launched as it is */
+StepGraph* ready_graph(lbm_handle* h, int lg) {
+    StepGraph& g = h->graphs[lg][h->lv[0].cur];
+    const Config& c = h->cfg;
+    if (lg == 0 || !graph_ok(h, 1 << lg)) return nullptr;
+    if (!g.exec || !g.steady || g.epoch != h->epoch || !steady_batch(h, 1 << lg)) return nullptr;
+    if (g.cur1 != h->lv[1].cur || g.mom != h->mom || g.force != (h->t > c.startf)) return nullptr;
+    if (c.sgs_mlp && g.phase != h->t % c.sgs_every) return nullptr;
+    if (g.force && h->t + (1 << lg) - c.startf > h->force_cap) return nullptr;
+    return &g;
+}
+
+/* queue the graph g of k steps from h->t0 on (the step counter first, when
+ * the device's is not there yet) */
+int launch_graph(lbm_handle* h, StepGraph& g, int t0, int k) {
+    if (g.steady && uses_counter(h, g.force)) {
+        if (h->step_dev_val != t0) {
+            CUDA_TRY(launch_set_step(h->step_dev, t0, h->stream));
+            ++h->launches;
+        }
+        h->step_dev_val = t0 + k;
+    }
+    const cudaError_t e = cudaGraphLaunch(g.exec, h->stream);
+    if (e != cudaSuccess) {
+        h->step_dev_val = -1;
+        return fail(LBM_ERR_CUDA, "step graph: %s", cudaGetErrorString(e));
+    }
+    return LBM_OK;
+}
+
+/* the graph's side-stream nodes replay on the main stream: later work queued
+ * on the side stream (lbm_get_last_force_async) waits for it */
+int join_side(lbm_handle* h) {
+    cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
+    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "step graph: %s", cudaGetErrorString(e));
+    return LBM_OK;
+}
+
+/* the graph g, ready for the steps from h->t on, launched once more */
+int replay_graph(lbm_handle* h, StepGraph& g, int k) {
+    const long long launches0 = h->launches;
+    if (int rc = launch_graph(h, g, h->t, k)) {
+        h->launches = launches0;
+        return rc;
+    }
+    h->launches += g.launches;
+    h->t += k;
+    return join_side(h);
+}
+
+/* k = 2^lg steps captured from the main stream into one graph (the force
+ * stream forks from it and joins it again inside every step), then launched.
+ * The executable graph at hand is updated in place when the topology is the
+ * same (an update leaves launches already queued as they were), else
+ * instantiated anew. */
+int run_graph(lbm_handle* h, int lg) {
+    const Config& c = h->cfg;
+    const int k = 1 << lg;
     /* what could allocate or synchronise happens before the capture */
     const int last_fidx = h->t + k - 1 - c.startf;
     if (last_fidx >= 0)
@@ -960,40 +1057,49 @@ int run_graph(lbm_handle* h, int k) {
         h->mom = mom0, h->mom_prev = mom_prev0, h->have_mom = have_mom0, h->launches = launches0;
         h->nu_valid = nu_valid0;
     };
+    StepGraph& sg = h->graphs[lg][cur0];
+    sg.steady = steady_batch(h, k);
+    sg.epoch = h->epoch;
+    sg.cur1 = cur1;
+    sg.force = t0 > c.startf;
+    sg.phase = c.sgs_mlp ? t0 % c.sgs_every : 0;
+    sg.mom = mom0;
     CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LBM_OK;
-    for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h);
+    for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h, sg.steady ? j : -1);
+    if (rc == LBM_OK && sg.steady && uses_counter(h, sg.force)) {
+        const cudaError_t e = launch_advance_step(h->step_dev, k, h->stream);
+        if (e != cudaSuccess) rc = fail(LBM_ERR_CUDA, "step counter: %s", cudaGetErrorString(e));
+        ++h->launches;
+    }
+    sg.launches = h->launches - launches0;
     cudaGraph_t g = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(h->stream, &g);
     if (rc != LBM_OK || ec != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         cudaGetLastError();
         restore();
+        sg.steady = false;
         return rc != LBM_OK ? rc : fail(LBM_ERR_CUDA, "step capture: %s", cudaGetErrorString(ec));
     }
     cudaError_t e = cudaSuccess;
-    cudaGraphExec_t& gx = h->gexec[k];
-    if (gx) {
+    if (sg.exec) {
         cudaGraphExecUpdateResultInfo info{};
-        if (cudaGraphExecUpdate(gx, g, &info) != cudaSuccess) {
+        if (cudaGraphExecUpdate(sg.exec, g, &info) != cudaSuccess) {
             cudaGetLastError();
-            cudaGraphExecDestroy(gx);
-            gx = nullptr;
+            cudaGraphExecDestroy(sg.exec);
+            sg.exec = nullptr;
         }
     }
-    if (!gx) e = cudaGraphInstantiate(&gx, g, 0);
+    if (!sg.exec) e = cudaGraphInstantiate(&sg.exec, g, 0);
     cudaGraphDestroy(g);
-    if (e == cudaSuccess) e = cudaGraphLaunch(gx, h->stream);
-    if (e != cudaSuccess) {
+    rc = e == cudaSuccess ? launch_graph(h, sg, t0, k) : fail(LBM_ERR_CUDA, "step graph: %s", cudaGetErrorString(e));
+    if (rc) {
         restore();
-        return fail(LBM_ERR_CUDA, "step graph: %s", cudaGetErrorString(e));
+        sg.steady = false;
+        return rc;
     }
-    /* the graph's side-stream nodes replay on the main stream: later work
-     * queued on the side stream (lbm_get_last_force_async) waits for it */
-    e = cudaEventRecord(h->ev_fork, h->stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
-    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "step graph: %s", cudaGetErrorString(e));
-    return LBM_OK;
+    return join_side(h);
 }
 
 int check_level(const lbm_handle* h, int level) {
@@ -1221,8 +1327,9 @@ int lbm_create(const char* inputs_text, lbm_handle** out) {
         r.eny = h->eny;
     }
     if (cudaMalloc(&h->audit_part, size_t(audit_partials(h->lv[0].L)) * 4 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&h->audit_out, 4 * sizeof(double)) != cudaSuccess)
+        cudaMalloc(&h->audit_out, 5 * sizeof(double)) != cudaSuccess)
         return bail(fail(LBM_ERR_NOMEM, "cannot allocate audit scratch"));
+    h->step_dev = reinterpret_cast<int*>(h->audit_out + 4);
     if ((rc = ensure_force_cap(h, std::max(1, c.tmax - c.startf)))) return bail(rc);
     if (c.sgs_mlp && c.sgs_every > 1) {
         const size_t nb = size_t(h->lv[0].L.qstride) * sizeof(float);
@@ -1252,8 +1359,9 @@ int lbm_destroy(lbm_handle* h) {
     cudaFree(h->dyn_hist);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
-    for (cudaGraphExec_t& g : h->gexec)
-        if (g) cudaGraphExecDestroy(g);
+    for (auto& row : h->graphs)
+        for (StepGraph& g : row)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
     cudaFree(h->stage);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -1427,22 +1535,21 @@ int lbm_set_populations(lbm_handle* h, int level, const float* f) {
 int lbm_step(lbm_handle* h, int nsteps) {
     if (!h) return fail(LBM_ERR_ARG, "null handle");
     if (nsteps < 0) return fail(LBM_ERR_ARG, "nsteps %d < 0", nsteps);
-    /* the first step is launched directly and the batches grow 2, 4, 8, 16,
-     * so that the host captures each batch while the GPU runs the one
-     * before (one executable graph per batch length, updated in place) */
-    int kb = 1;
-    for (int i = 0; i < nsteps;) {
-        const int k = std::min(kb, nsteps - i);
-        kb = std::min(2 * kb, GRAPH_STEPS);
-        int rc;
-        if (k >= 2 && graph_ok(h, k)) {
-            rc = run_graph(h, k);
-            i += k;
-        } else {
-            rc = one_step(h);
-            ++i;
-        }
+    /* the longest batch that fits, when its graph is at hand; else batches
+     * that grow 2, 4, 8, 16, so that the host captures each while the GPU
+     * runs the one before (after one direct step where graphs need it) */
+    int ramp = graph_ok(h, 2) ? 1 : 0;
+    for (int left = nsteps; left > 0;) {
+        int lg = GRAPH_LG, rc;
+        while ((1 << lg) > left) --lg;
+        StepGraph* g = ready_graph(h, lg);
+        if (!g && lg > ramp) g = ready_graph(h, lg = ramp);
+        if (!g) ramp = std::min(ramp + 1, GRAPH_LG);
+        if (g) rc = replay_graph(h, *g, 1 << lg);
+        else if (lg > 0 && graph_ok(h, 1 << lg)) rc = run_graph(h, lg);
+        else rc = one_step(h), lg = 0;
         if (rc) return rc;
+        left -= 1 << lg;
     }
     return LBM_OK;
 }
@@ -1488,6 +1595,7 @@ int lbm_set_sgs_mlp(lbm_handle* h, const float* params, int n) {
     h->mlp_params.assign(params, params + n);
     h->mlp_ready = true;
     h->nu_valid = false;
+    ++h->epoch;
     return LBM_OK;
 }
 

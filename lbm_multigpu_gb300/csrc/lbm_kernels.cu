@@ -69,9 +69,11 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
                                                               const unsigned* __restrict__ body, int nbody,
                                                               double* __restrict__ part, unsigned* __restrict__ done,
                                                               double* __restrict__ out3,
-                                                              const uint8_t* __restrict__ mask, int halfway) {
+                                                              const uint8_t* __restrict__ mask, int halfway,
+                                                              const int* __restrict__ step_dev) {
     using F = Fmt<S>;
     using T = typename F::T;
+    if (step_dev) out3 += 3LL * *step_dev;
     double s[3] = {0.0, 0.0, 0.0};
     const unsigned plane = unsigned(L.plane), pitch = unsigned(L.pitch);
     for (int i = blockIdx.x * FORCE_THREADS + threadIdx.x; i < nbody; i += int(gridDim.x) * FORCE_THREADS) {
@@ -644,14 +646,28 @@ cudaError_t launch_dyn_control(const Level& L, const void* f, int y1, float umax
     return cudaGetLastError();
 }
 
+__global__ void k_set_step(int* step, int t) { *step = t; }
+__global__ void k_advance_step(int* step, int k) { *step += k; }
+
+cudaError_t launch_set_step(int* step_dev, int t, cudaStream_t s) {
+    k_set_step<<<1, 1, 0, s>>>(step_dev, t);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_advance_step(int* step_dev, int k, cudaStream_t s) {
+    k_advance_step<<<1, 1, 0, s>>>(step_dev, k);
+    return cudaGetLastError();
+}
+
 int force_partials() { return FORCE_BLOCKS; }
 
 cudaError_t launch_force(const Level& L, const void* fA, const unsigned* body, int nbody, double* partials,
-                         unsigned* done, double* out3, cudaStream_t s, const uint8_t* mask, int halfway) {
+                         unsigned* done, double* out3, cudaStream_t s, const uint8_t* mask, int halfway,
+                         const int* step_dev) {
     if (nbody <= 0) return cudaSuccess;
     const int blocks = std::min(FORCE_BLOCKS, (nbody + FORCE_THREADS - 1) / FORCE_THREADS);
     LBM_DISPATCH(L.storage, (k_force_list<S><<<blocks, FORCE_THREADS, 0, s>>>(L, (const S*)fA, body, nbody, partials,
-                                                                              done, out3, mask, halfway)));
+                                                                              done, out3, mask, halfway, step_dev)));
     return cudaGetLastError();
 }
 

@@ -135,8 +135,8 @@ struct StepParams {
     int halfway;           /* half-way bounce-back: a pull from a solid node returns the node's own
                             * opposite post-collision population; solids are not updated */
     int has_lid;           /* the level's mask contains LID nodes */
-    int force_on;          /* accumulate momentum exchange at BODY nodes */
     int t;                 /* time step index (stats, noise) */
+    const int* step_dev;   /* when non-null, t counts from the device's step counter */
     int stats_on, start_av, start_fluc;
     float stats_weight;
     float noise_amp;
@@ -174,10 +174,14 @@ cudaError_t launch_stream_collide(const Level& L, const StepParams& p, const voi
 cudaError_t launch_stream_collide_mlp(const Level& L, const StepParams& p, const void* fA, void* fB,
                                       const uint8_t* mask, float* stats, const uint32_t* links, const void* blob,
                                       int* err, cudaStream_t s);
-/* FP64 momentum exchange over a list of BODY nodes (pitched indices), ADDED to out3 */
+/* FP64 momentum exchange over a list of BODY nodes (pitched indices), ADDED to
+ * out3 (with step_dev, to out3 + 3 *step_dev) */
 cudaError_t launch_force(const Level& L, const void* fA, const unsigned* body, int nbody, double* partials,
                          unsigned* done, double* out3, cudaStream_t s, const uint8_t* mask = nullptr,
-                         int halfway = 0);
+                         int halfway = 0, const int* step_dev = nullptr);
+/* the device's step counter: set, and advanced by k */
+cudaError_t launch_set_step(int* step_dev, int t, cudaStream_t s);
+cudaError_t launch_advance_step(int* step_dev, int k, cudaStream_t s);
 int force_partials();
 /* the same sum found by scanning the mask, of an FP32 structure-of-arrays
  * level; partials holds force_scan_partials()*3 doubles */

@@ -194,6 +194,34 @@ constexpr int FEAT_NUBUF = 32;
 #define LBM_SC_MINB 10
 #endif
 
+/* the step index of the launch; a load for launches replayed from a graph,
+ * so it is read only where it is needed */
+__device__ __forceinline__ int sc_time(const StepParams& p) { return p.t + (p.step_dev ? *p.step_dev : 0); }
+
+/* vel_av / vel_fluc (LR7:1018-1058) of node c with the velocity (u, v) after
+ * the collision: running mean, then variance about it */
+__device__ __forceinline__ void sc_stats(const StepParams& p, float* __restrict__ stats, unsigned qs, unsigned c,
+                                         float u, float v) {
+    const int t = sc_time(p);
+    if (t < p.start_av) return;
+    float* au = stats;
+    float* av = stats + qs;
+    const float w = p.stats_weight;
+    if (t < p.start_fluc) {
+        const float nn = float(t - p.start_av);
+        au[c] = (au[c] * nn + u * w) / (nn + w);
+        av[c] = (av[c] * nn + v * w) / (nn + w);
+    } else {
+        float* fu = stats + 2 * (size_t)qs;
+        float* fv = stats + 3 * (size_t)qs;
+        const float nn = float(t - p.start_fluc);
+        const float du = (u - au[c]) * (u - au[c]);
+        const float dv = (v - av[c]) * (v - av[c]);
+        fu[c] = (fu[c] * nn + du * w) / (nn + w);
+        fv[c] = (fv[c] * nn + dv * w) / (nn + w);
+    }
+}
+
 /* the collision, statistics, store and moment export of a non-solid node;
  * f holds populations, or for DEV their stored deviations.  With DEVMRT an
  * inlet's or outlet's rebuild (bc, uin; FLUID otherwise) is part of the
@@ -231,8 +259,7 @@ __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParam
             for (int q = 0; q < 19; ++q) f[q] -= L.off[q];
         }
     }
-    if (p.stats_on && p.t >= p.start_av) {
-        /* vel_av / vel_fluc (LR7:1018-1058): running mean, then variance */
+    if (p.stats_on) {
         T u = 0, v = 0;
 #pragma unroll
         for (int q = 0; q < 19; ++q) {
@@ -240,22 +267,7 @@ __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParam
             if (cx(q)) u += T(cx(q)) * g;
             if (cy(q)) v += T(cy(q)) * g;
         }
-        float* au = stats;
-        float* av = stats + qs;
-        const float w = p.stats_weight;
-        if (p.t < p.start_fluc) {
-            const float nn = float(p.t - p.start_av);
-            au[c] = (au[c] * nn + float(u) * w) / (nn + w);
-            av[c] = (av[c] * nn + float(v) * w) / (nn + w);
-        } else {
-            float* fu = stats + 2 * (size_t)qs;
-            float* fv = stats + 3 * (size_t)qs;
-            const float nn = float(p.t - p.start_fluc);
-            const float du = (float(u) - au[c]) * (float(u) - au[c]);
-            const float dv = (float(v) - av[c]) * (float(v) - av[c]);
-            fu[c] = (fu[c] * nn + du * w) / (nn + w);
-            fv[c] = (fv[c] * nn + dv * w) / (nn + w);
-        }
+        sc_stats(p, stats, qs, c, float(u), float(v));
     }
     store19<S, LAY, DEV>(L, fB, n, f);
 }
@@ -378,7 +390,7 @@ __device__ __forceinline__ void sc_finish(const Level& L, const StepParams& p, c
                 f[q] = RAW ? T(F::ldr(n.at(fA, q, cn))) : F::ld(n.at(fA, q, cn), L.off[q]);
             if (p.noise_amp != 0.f) {
                 const uint32_t cell = uint32_t((z * L.ny + y) * L.nx + x);
-                const float xi = philox_uniform(p.noise_seed, cell, uint32_t(p.t));
+                const float xi = philox_uniform(p.noise_seed, cell, uint32_t(sc_time(p)));
                 uin = uin + T(p.u_in) * T(p.noise_amp) * (T(2) * T(xi) - T(1));
             }
             if constexpr ((FEAT & FEAT_DEVMRT) != 0) {
@@ -398,7 +410,7 @@ __device__ __forceinline__ void sc_finish(const Level& L, const StepParams& p, c
             if ((FEAT & FEAT_LID) && type == LID) {
                 lid<T>(f, p.lid_face, T(p.lid_u[0]), T(p.lid_u[1]), T(p.lid_u[2]), p.lid_quirk != 0);
             } else if (FEAT & FEAT_XBC) {
-                alt_boundary<T>(type, f, x, y, z, L.nx, L.ny, L.nz, T(p.u_in), p.t);
+                alt_boundary<T>(type, f, x, y, z, L.nx, L.ny, L.nz, T(p.u_in), sc_time(p));
             }
             if (DEV) {
 #pragma unroll
@@ -517,7 +529,7 @@ __global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_
                 float uin = p.u_in;
                 if (p.noise_amp != 0.f) {
                     const uint32_t cell = uint32_t((z * L.ny + y) * L.nx + x);
-                    const float xi = philox_uniform(p.noise_seed, cell, uint32_t(p.t));
+                    const float xi = philox_uniform(p.noise_seed, cell, uint32_t(sc_time(p)));
                     uin = uin + p.u_in * p.noise_amp * (2.f * xi - 1.f);
                 }
                 extrap<float>(type, f, p.rho_out, uin);
@@ -560,27 +572,14 @@ __global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_
         mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8];
         mrt_dev_complete(mr, 0.f);
         mrt_dev_relax(f, mr, 1.f / (tau0 + 3.f * nu));
-        if (p.stats_on && p.t >= p.start_av) {
+        if (p.stats_on) {
             float u = 0, v = 0;
 #pragma unroll
             for (int q = 0; q < 19; ++q) {
                 if (cx(q)) u += float(cx(q)) * f[q];
                 if (cy(q)) v += float(cy(q)) * f[q];
             }
-            float* au = stats;
-            float* av = stats + qs;
-            const float w = p.stats_weight;
-            if (p.t < p.start_fluc) {
-                const float nn = float(p.t - p.start_av);
-                au[c] = (au[c] * nn + u * w) / (nn + w);
-                av[c] = (av[c] * nn + v * w) / (nn + w);
-            } else {
-                float* fu = stats + 2 * (size_t)qs;
-                float* fv = stats + 3 * (size_t)qs;
-                const float nn = float(p.t - p.start_fluc);
-                fu[c] = (fu[c] * nn + (u - au[c]) * (u - au[c]) * w) / (nn + w);
-                fv[c] = (fv[c] * nn + (v - av[c]) * (v - av[c]) * w) / (nn + w);
-            }
+            sc_stats(p, stats, qs, c, u, v);
         }
         store19<S, LAY, false>(L, fB, n, f);
     }

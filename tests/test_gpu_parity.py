@@ -227,6 +227,44 @@ def test_uniform_step_graphs_are_bit_exact(product, precision):
         np.testing.assert_array_equal(x, y)
 
 
+@pytest.mark.parametrize("kind", ["stats_noise", "no_body", "fp16_late_force", "refined", "new_mask"])
+def test_replayed_step_graphs_are_bit_exact(product, kind):
+    """graphs launched again without a new capture (the step number on the
+    device): calls of several lengths equal single steps in populations,
+    statistics and the recorded forces, with statistics and inlet noise, with
+    no body, with the force recorded from a later step on, with refinement,
+    and with the mask changed in between"""
+    lbm = product
+    kw = dict(obst1=(18.5, 11.5, 0.0), r1=4.0, re=60.0, umax=0.05, tmax=400, les=1, cs=0.01, bounceback="halfway",
+              inlet_noise=0.01, seed=5)
+    if kind == "stats_noise":
+        kw.update(velav=1, start_velav=20, start_velfluc=70)
+    elif kind == "no_body":
+        kw.update(geometry="channel")
+    elif kind == "fp16_late_force":
+        kw.update(precision="fp16", startf=37)
+    elif kind == "refined":
+        kw.update(refinement=1, lr_dims=(32, 32, 12), lr_factor=0.5, lr_origin=(12.25, 4.25, 2.25), cf_time="linear",
+                  bounceback="fullway")
+    text = lbm.make_inputs(64, 24, 12, **kw)
+    res = []
+    for calls in ([16, 16, 5, 33, 16, 1, 48], [1] * 135):
+        with lbm.Solver(text) as s:
+            t = 0
+            for n in calls:
+                s.step(n)
+                t += n
+                if kind == "new_mask" and t == 70:
+                    m = s.mask()
+                    m[3:6, 15:18, 40:44] = lbm.NODE["BODY"]
+                    s.set_mask(m)
+            got = [s.populations(k) for k in range(s.nlevels)] + [s.forces()]
+            res.append(got + ([s.stats()] if kind == "stats_noise" else []))
+    for a, b in zip(*res):
+        np.testing.assert_array_equal(a, b)
+    assert np.isfinite(res[0][0]).all()
+
+
 def test_async_force_read_after_graph_steps(product):
     """lbm_get_last_force_async after a graph-replayed lbm_step(n): the copy
     on the force stream waits for the replayed steps, so it reads the same
