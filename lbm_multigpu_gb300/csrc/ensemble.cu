@@ -3,7 +3,7 @@
  *
  * Every member is a compact SoA level f[q][z][y][pitch] (pitch = n rounded up
  * to 32) inside one A and one B buffer; a block of 32 x TY threads updates a
- * 32 x TY tile of one z plane of one member.  The launch is persistent: a
+ * 32 x TY tile of one z plane of one member (TY 4 or 8, 4 with the closure).  The launch is persistent: a
  * grid sized by the autotuner walks the global tile list, so the per-member
  * work is balanced across the SMs whatever the mix of sizes, and a CUDA graph
  * of several steps replays the whole sequence with one host call.
@@ -18,8 +18,6 @@
  * samples for the closure.
  */
 #include <cuda_runtime.h>
-
-#include <type_traits>
 
 #include "d3q19.cuh"
 #include "ensemble.cuh"
@@ -36,16 +34,7 @@ __device__ __forceinline__ int find_member(const Table& T, int g) {
 
 template <int TY, int SGS>
 __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float* __restrict__ fA,
-                                                      float* __restrict__ fB, const unsigned char* __restrict__ blob,
-                                                      float cs, int* __restrict__ err) {
-    constexpr int ROWS = 32 * TY;
-    /* the MLP variant's operands live in dynamic shared memory (over 48 KB
-     * for 256 rows), aligned up to 1 KB inside the allocation */
-    extern __shared__ unsigned char dsm[];
-    sgs::InferSmem<ROWS>& smem = *reinterpret_cast<sgs::InferSmem<ROWS>*>(
-        (reinterpret_cast<uintptr_t>(dsm) + 1023) & ~uintptr_t(1023));
-#if defined(__CUDA_ARCH__)
-    if constexpr (SGS == SGS_MLP) sgs::infer_setup<ROWS>(smem, blob);
+                                                      float* __restrict__ fB, float cs) {
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int g = blockIdx.x; g < T.ntiles; g += gridDim.x) {
         const int mi = find_member(T, g);
@@ -55,43 +44,85 @@ __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float
         const int z = local / per_z, r = local - z * per_z;
         const int y = (r / M.tiles_x) * TY + ty, x = (r % M.tiles_x) * 32 + tx;
         const int n = M.n;
-        const bool live = x < n && y < n;
+        if (x >= n || y >= n) continue;
         const unsigned pitch = unsigned(M.pitch), plane = unsigned(n) * pitch, qs = plane * unsigned(n);
         const float* a = fA + M.off;
         float* b = fB + M.off;
         float f[19];
-        unsigned c = 0;
+        const unsigned c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
+        const unsigned xs[3] = {unsigned(x == 0 ? n - 1 : x - 1), unsigned(x), unsigned(x == n - 1 ? 0 : x + 1)};
+        const unsigned yb[3] = {(y == 0 ? n - 1 : y - 1) * pitch, y * pitch, (y == n - 1 ? 0 : y + 1) * pitch};
+        const unsigned zb[3] = {(z == 0 ? n - 1 : z - 1) * plane, z * plane, (z == n - 1 ? 0 : z + 1) * plane};
+#pragma unroll
+        for (int q = 0; q < 19; ++q) f[q] = __ldg(a + q * qs + zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]);
+        collide_mrt<MRT>(f, M.omega, SGS == SGS_SMAG, cs, 0.f);
+#pragma unroll
+        for (int q = 0; q < 19; ++q) b[q * qs + c] = f[q];
+    }
+}
+
+/* The step with the learned closure, as k_stream_collide_mlp: tiles of 32 x 4
+ * (one M = 128 MMA per layer), persistent blocks, and the projected MRT
+ * collision, of which only rho, j and the five stresses stay live across the
+ * tensor-core round trips.  Eight boxes of sides 32 to 80 (1.8 M nodes): 87 us
+ * with 7 blocks per SM and just their shared memory taken from L1 (4, 5, 6, 8
+ * blocks: 102, 93, 90, 100 us; one block of 256 rows per SM, what the
+ * occupancy API made of kernels with TMEM: 188 us). */
+constexpr int MLP_TY = 4, MLP_ROWS = 32 * MLP_TY, MLP_BLOCKS = 7;
+__global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS) k_ens_step_mlp(const Table T, const float* __restrict__ fA,
+                                                                       float* __restrict__ fB,
+                                                                       const unsigned char* __restrict__ blob,
+                                                                       int* __restrict__ err) {
+    extern __shared__ __align__(128) unsigned char dsm[];
+#if defined(__CUDA_ARCH__)
+    sgs::InferSmem<MLP_ROWS>& sm = *reinterpret_cast<sgs::InferSmem<MLP_ROWS>*>(dsm);
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    sgs::infer_setup<MLP_ROWS>(sm, blob);
+    for (int g = blockIdx.x; g < T.ntiles; g += gridDim.x) {
+        const Member& M = T.m[find_member(T, g)];
+        const int local = g - M.tile0, per_z = M.tiles_x * M.tiles_y;
+        const int z = local / per_z, r = local - z * per_z;
+        const int y = (r / M.tiles_x) * MLP_TY + ty, x = (r % M.tiles_x) * 32 + tx;
+        const int n = M.n;
+        const bool live = x < n && y < n;
+        const unsigned pitch = unsigned(M.pitch), plane = unsigned(n) * pitch, qs = plane * unsigned(n);
+        const unsigned c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
+        float f[19];
         if (live) {
-            c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
+            const float* a = fA + M.off;
             const unsigned xs[3] = {unsigned(x == 0 ? n - 1 : x - 1), unsigned(x), unsigned(x == n - 1 ? 0 : x + 1)};
             const unsigned yb[3] = {(y == 0 ? n - 1 : y - 1) * pitch, y * pitch, (y == n - 1 ? 0 : y + 1) * pitch};
             const unsigned zb[3] = {(z == 0 ? n - 1 : z - 1) * plane, z * plane, (z == n - 1 ? 0 : z + 1) * plane};
 #pragma unroll
-            for (int q = 0; q < 19; ++q)
-                f[q] = __ldg(a + q * qs + zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]);
+            for (int q = 0; q < 19; ++q) f[q] = __ldg(a + q * qs + zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]);
         } else {
 #pragma unroll
             for (int q = 0; q < 19; ++q) f[q] = wq(q);
         }
-        float omega = M.omega;
-        if constexpr (SGS == SGS_MLP) {
-            float rho, p6[6], xf[sgs::NIN];
-            pi_neq<float>(f, rho, p6);
-            const float s = -1.5f / rho;
+        const MrtDev<float> mo = mrt_dev_moments<float>(f, 0.f);
+        float p6[6], xf[sgs::NIN];
+        mrt_dev_pi(mo, p6);
+        const float sc = -1.5f / mo.rho;
 #pragma unroll
-            for (int k = 0; k < 6; ++k) p6[k] *= s;
-            sgs::features_fast(p6, M.tau0, M.omega, xf); /* omega = 1 / tau0 */
-            const float o = sgs::infer_nu<ROWS>(smem, xf, err);
-            if (o < 0.f) break; /* a tensor-core wait ran out (block-uniform) */
-            omega = 1.f / (M.tau0 + 3.f * o * sgs::strain_gain(xf, M.omega));
-        }
-        collide_mrt<MRT>(f, omega, SGS == SGS_SMAG, cs, 0.f);
-        if (live) {
+        for (int k = 0; k < 6; ++k) p6[k] *= sc;
+        sgs::features_fast(p6, M.tau0, M.omega, xf); /* omega = 1 / tau0 */
+        float keep[10] = {mo.rho, mo.jx, mo.jy, mo.jz, mo.n9, mo.n11, mo.n13, mo.n14, mo.n15,
+                          sgs::strain_gain(xf, M.omega)};
+        const float o = sgs::infer_nu<MLP_ROWS>(sm, xf, err);
+        if (o < 0.f) break; /* a tensor-core wait ran out (block-uniform) */
+        if (!live) continue;
 #pragma unroll
-            for (int q = 0; q < 19; ++q) b[q * qs + c] = f[q];
-        }
+        for (int k = 0; k < 10; ++k) asm volatile("" : "+f"(keep[k]));
+        MrtDev<float> mr;
+        mr.rho = keep[0], mr.jx = keep[1], mr.jy = keep[2], mr.jz = keep[3], mr.n9 = keep[4], mr.n11 = keep[5];
+        mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8];
+        mrt_dev_complete(mr, 0.f);
+        mrt_dev_relax(f, mr, 1.f / (M.tau0 + 3.f * o * keep[9]));
+        float* b = fB + M.off + c;
+#pragma unroll
+        for (int q = 0; q < 19; ++q) b[q * qs] = f[q];
     }
-    if constexpr (SGS == SGS_MLP) sgs::infer_teardown<ROWS>(smem);
+    sgs::infer_teardown<MLP_ROWS>(sm);
 #endif
 }
 
@@ -375,70 +406,49 @@ __global__ void k_d2f(const double* __restrict__ a, float* __restrict__ b, size_
 }  // namespace ens
 
 /* ---- launchers */
-template <int TY, int SGS> static size_t step_smem() {
-    return SGS == ens::SGS_MLP ? sgs::infer_dyn_smem<32 * TY>() : 0;
-}
+static size_t mlp_step_smem() { return sgs::infer_dyn_smem<ens::MLP_ROWS>(); }
 
-template <int TY, int SGS> static cudaError_t step_attr() {
-    static cudaError_t done = cudaErrorNotReady;
-    if (done == cudaErrorNotReady)
-        done = cudaFuncSetAttribute(ens::k_ens_step<TY, SGS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(step_smem<TY, SGS>()));
-    return done;
-}
-
-template <int TY, int SGS> static cudaError_t step_t(const ens::Table& T, const float* fA, float* fB,
-                                                    const void* blob, float cs, int* err, int grid, cudaStream_t s) {
-    if (cudaError_t e = step_attr<TY, SGS>()) return e;
-    if (SGS == ens::SGS_MLP) {
+cudaError_t launch_ens_step(const ens::Table& T, const float* fA, float* fB, int model, const void* blob, float cs,
+                            int* err, int grid, cudaStream_t s) {
+    if (model == ens::SGS_MLP) {
+        if (T.ty != ens::MLP_TY) return cudaErrorInvalidValue;
+        const size_t smem = mlp_step_smem();
+        cudaError_t e = cudaFuncSetAttribute(ens::k_ens_step_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e != cudaSuccess) return e;
         TmemLane lane(s);
         if (lane.status() != cudaSuccess) return lane.status();
-        ens::k_ens_step<TY, SGS><<<grid, 32 * TY, step_smem<TY, SGS>(), lane.stream()>>>(
-            T, fA, fB, (const unsigned char*)blob, cs, err);
+        ens::k_ens_step_mlp<<<grid, ens::MLP_ROWS, smem, lane.stream()>>>(T, fA, fB, (const unsigned char*)blob, err);
         return cudaGetLastError();
     }
-    ens::k_ens_step<TY, SGS><<<grid, 32 * TY, step_smem<TY, SGS>(), s>>>(T, fA, fB, (const unsigned char*)blob, cs,
-                                                                         err);
+    if (T.ty == 4 && model == ens::SGS_NONE) ens::k_ens_step<4, ens::SGS_NONE><<<grid, 128, 0, s>>>(T, fA, fB, cs);
+    else if (T.ty == 4) ens::k_ens_step<4, ens::SGS_SMAG><<<grid, 128, 0, s>>>(T, fA, fB, cs);
+    else if (T.ty == 8 && model == ens::SGS_NONE) ens::k_ens_step<8, ens::SGS_NONE><<<grid, 256, 0, s>>>(T, fA, fB, cs);
+    else if (T.ty == 8) ens::k_ens_step<8, ens::SGS_SMAG><<<grid, 256, 0, s>>>(T, fA, fB, cs);
+    else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 
-cudaError_t launch_ens_step(const ens::Table& T, const float* fA, float* fB, int sgs, const void* blob, float cs,
-                            int* err, int grid, cudaStream_t s) {
-    if (T.ty == 4) {
-        if (sgs == ens::SGS_NONE) return step_t<4, ens::SGS_NONE>(T, fA, fB, blob, cs, err, grid, s);
-        if (sgs == ens::SGS_SMAG) return step_t<4, ens::SGS_SMAG>(T, fA, fB, blob, cs, err, grid, s);
-        return step_t<4, ens::SGS_MLP>(T, fA, fB, blob, cs, err, grid, s);
-    }
-    if (T.ty == 8) {
-        if (sgs == ens::SGS_NONE) return step_t<8, ens::SGS_NONE>(T, fA, fB, blob, cs, err, grid, s);
-        if (sgs == ens::SGS_SMAG) return step_t<8, ens::SGS_SMAG>(T, fA, fB, blob, cs, err, grid, s);
-        return step_t<8, ens::SGS_MLP>(T, fA, fB, blob, cs, err, grid, s);
-    }
-    return cudaErrorInvalidValue;
-}
-
-int ens_step_occupancy(int ty, int sgs) {
-    int nb = 0;
+int ens_step_resident(int ty, int model) {
+    int nb = 0, dev = 0, sms = 0;
     cudaError_t e = cudaSuccess;
-    if (ty == 4) {
-        if (sgs == ens::SGS_NONE)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<4, ens::SGS_NONE>, 128, 0);
-        else if (sgs == ens::SGS_SMAG)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<4, ens::SGS_SMAG>, 128, 0);
-        else if ((e = step_attr<4, ens::SGS_MLP>()) == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<4, ens::SGS_MLP>, 128,
-                                                              step_smem<4, ens::SGS_MLP>());
+    if (model == ens::SGS_MLP) {
+        e = sgs::infer_resident(ens::k_ens_step_mlp, ens::MLP_ROWS, mlp_step_smem(), sgs::tmem_cols<ens::MLP_ROWS>(),
+                                ens::MLP_BLOCKS, &nb);
+        if (e == cudaSuccess) return nb;
+        nb = 0;
+    } else if (ty == 4 && model == ens::SGS_NONE) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<4, ens::SGS_NONE>, 128, 0);
+    } else if (ty == 4) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<4, ens::SGS_SMAG>, 128, 0);
+    } else if (model == ens::SGS_NONE) {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<8, ens::SGS_NONE>, 256, 0);
     } else {
-        if (sgs == ens::SGS_NONE)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<8, ens::SGS_NONE>, 256, 0);
-        else if (sgs == ens::SGS_SMAG)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<8, ens::SGS_SMAG>, 256, 0);
-        else if ((e = step_attr<8, ens::SGS_MLP>()) == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<8, ens::SGS_MLP>, 256,
-                                                              step_smem<8, ens::SGS_MLP>());
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ens::k_ens_step<8, ens::SGS_SMAG>, 256, 0);
     }
-    if (e != cudaSuccess) return 1;
-    return nb < 1 ? 1 : nb;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        sms = 152;
+    return sms * (e != cudaSuccess || nb < 1 ? 1 : nb);
 }
 
 cudaError_t launch_ens_init(const ens::Table& T, const ens::KMode* modes, float* fA, cudaStream_t s) {

@@ -10,6 +10,8 @@ namespace ens {
 
 constexpr int MAXM = 32;
 constexpr int SGS_NONE = 0, SGS_SMAG = 1, SGS_MLP = 2;
+/* whether the step of a subgrid model has a kernel for tiles of this height */
+constexpr bool tile_height_ok(int ty, int model) { return ty == 4 || (ty == 8 && model != SGS_MLP); }
 
 struct Member {
     int n;                  /* cube side */
@@ -51,9 +53,10 @@ constexpr int ENERGY_BLOCKS = 256;
 
 }  // namespace ens
 
-cudaError_t launch_ens_step(const ens::Table& T, const float* fA, float* fB, int sgs, const void* blob, float cs,
+cudaError_t launch_ens_step(const ens::Table& T, const float* fA, float* fB, int model, const void* blob, float cs,
                             int* err, int grid, cudaStream_t s);
-int ens_step_occupancy(int ty, int sgs);
+/* blocks of the step kernel that the current device holds at a time */
+int ens_step_resident(int ty, int model);
 cudaError_t launch_ens_init(const ens::Table& T, const ens::KMode* modes, float* fA, cudaStream_t s);
 cudaError_t launch_ens_init_from(const ens::Table& T, const float* u, float* fA, float* fB, cudaStream_t s);
 cudaError_t launch_ens_velocity(const ens::Table& T, const float* f, float* u, cudaStream_t s);

@@ -241,7 +241,7 @@ int lbm_ensemble_create(int count, const int* sizes, const float* tau0, int sgs,
     }
     e->nelem = off;
     e->nu = uoff;
-    layout(e, 8);
+    layout(e, ens::tile_height_ok(8, sgs) ? 8 : 4);
     if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(set_error(LBM_ERR_CUDA, "ensemble: stream", cudaSuccess));
     cudaEventCreate(&e->e0);
@@ -262,7 +262,7 @@ int lbm_ensemble_create(int count, const int* sizes, const float* tau0, int sgs,
     cudaMemset(e->u, 0, e->nu * sizeof(float));
     if (launch_ens_init_from(e->T, e->u, e->f[0], e->f[1], e->stream) != cudaSuccess)
         return bail(set_error(LBM_ERR_CUDA, "ensemble: init", cudaGetLastError()));
-    e->grid = std::min(e->T.ntiles, sm_count() * ens_step_occupancy(e->T.ty, sgs));
+    e->grid = std::min(e->T.ntiles, ens_step_resident(e->T.ty, sgs));
     if (int rc = sync_check(e)) return bail(rc);
     *out = e;
     return LBM_OK;
@@ -407,8 +407,9 @@ int lbm_ensemble_autotune(lbm_ensemble* e, int* ty_out, int* grid_out, float* ms
         const int sms = sm_count();
         cudaError_t r = cudaSuccess;
         for (int ty : {4, 8}) {
+            if (!ens::tile_height_ok(ty, e->sgs)) continue;
             layout(e, ty);
-            const int occ = ens_step_occupancy(ty, e->sgs);
+            const int occ = ens_step_resident(ty, e->sgs) / sms;
             std::vector<int> grids;
             for (int b = 1; b <= occ; ++b) grids.push_back(std::min(e->T.ntiles, sms * b));
             grids.push_back(e->T.ntiles); /* one tile per block */

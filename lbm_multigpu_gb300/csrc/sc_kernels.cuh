@@ -146,8 +146,8 @@ template <> struct NodeIdx<1> {
 /* the 19 values g of this node into buffer f: raw stored values (RAW) or
  * populations with the format's offsets removed; the blocked layout writes
  * each opposite pair with one store */
-template <class S, int LAY, bool RAW>
-__device__ __forceinline__ void store19(const Level& L, S* __restrict__ f, const NodeIdx<LAY>& n,
+template <class S, int LAY, bool RAW, class IDX>
+__device__ __forceinline__ void store19(const Level& L, S* __restrict__ f, const IDX& n,
                                         const typename Fmt<S>::T g[19]) {
     using F = Fmt<S>;
     if constexpr (LAY == 1) {
@@ -460,79 +460,106 @@ __global__ void __launch_bounds__(SC_BX* SC_BY, sc_min_blocks<S, FEAT>()) k_stre
  * eddy viscosity of every node from the MLP evaluated on the tensor cores
  * for the whole 32 x 4 tile at once.  Persistent blocks walk the tiles so
  * that each block stages the weights and allocates its TMEM once per launch.
- * MRT collision (LR7:583-711) at tau_eff = tau0 + 3 nu_t; FP32 arithmetic. */
+ * MRT collision (LR7:583-711) at tau_eff = tau0 + 3 nu_t; FP32 arithmetic.
+ *
+ * What bounds it is the L1 cache: the pair-interleaved layout brings every
+ * sector of a row twice to an SM (q and its opposite are pulled by different
+ * rows) unless L1 still holds it, and a block's operands take 27 KB of the
+ * array that L1 shares with shared memory.  So the launch asks for exactly the
+ * shared memory of its resident blocks (7: 196 of 228 KB).  512 x 128 x 128,
+ * FP32: 316 us; with all of the array as shared memory 433 us, and 376 us with
+ * the network left out altogether; 4, 5, 6, 8 blocks per SM 370, 314, 362,
+ * 478 us (FP16 408, 322, 353, 402 and with 7 313 us).  Copying the next
+ * tile's pulls into shared memory with cp.async cost more L1 than it hid
+ * (462 us). */
 constexpr int MLP_BY = 4; /* tile 32 x 4: one M = 128 MMA per layer */
-/* resident blocks per SM the closure kernel is compiled for */
-#ifndef LBM_MLP_MINB
-#define LBM_MLP_MINB 7
-#endif
+constexpr int MLP_ROWS = SC_BX * MLP_BY;
+constexpr int MLP_BLOCKS = 7;
+
+/* the 19 values g of node c into buffer f, as store19 */
+template <int LAY> struct CellIdx {
+    unsigned c, qs;
+    template <class P> __device__ __forceinline__ P* own(P* f, int q) const {
+        if (LAY == 0) return f + (unsigned(q) * qs + c);
+        return q == 0 ? f + ((c >> 5) * BLOCK_ELEMS + (c & 31u))
+                      : (f + ((c >> 5) * BLOCK_ELEMS + 2u * (c & 31u))) + pair_qoff(q);
+    }
+};
+
 template <class S, bool HALFWAY, int LAY>
-__global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_mlp(const Level L, const StepParams p,
-                                                                      const S* __restrict__ fA, S* __restrict__ fB,
-                                                                      const uint8_t* __restrict__ mask,
-                                                                      float* __restrict__ stats,
-                                                                      const uint32_t* __restrict__ links,
-                                                                      const unsigned char* __restrict__ blob,
-                                                                      int* __restrict__ err) {
+__global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS)
+    k_stream_collide_mlp(const Level L, const StepParams p, const S* __restrict__ fA, S* __restrict__ fB,
+                         const uint8_t* __restrict__ mask, float* __restrict__ stats,
+                         const uint32_t* __restrict__ links, const unsigned char* __restrict__ blob,
+                         int* __restrict__ err) {
     using F = Fmt<S>;
-    constexpr int ROWS = SC_BX * MLP_BY;
-    extern __shared__ unsigned char dsm[];
-    sgs::InferSmem<ROWS>& sm = *reinterpret_cast<sgs::InferSmem<ROWS>*>(
-        (reinterpret_cast<uintptr_t>(dsm) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(128) unsigned char dsm[];
 #if defined(__CUDA_ARCH__)
-    sgs::infer_setup<ROWS>(sm, blob);
+    sgs::InferSmem<MLP_ROWS>& sm = *reinterpret_cast<sgs::InferSmem<MLP_ROWS>*>(dsm);
+    sgs::infer_setup<MLP_ROWS>(sm, blob);
     const unsigned qs = unsigned(L.qstride);
     const unsigned plane = unsigned(L.plane), pitch = unsigned(L.pitch);
     const int tiles_x = L.pitch / SC_BX, tiles_y = (L.ny + MLP_BY - 1) / MLP_BY;
     const int ntiles = tiles_x * tiles_y * L.nz;
     const float tau0 = 1.f / p.omega, inv_t0 = p.omega;
-    /* the node of this thread in tile g */
-    auto node_of = [&](int g, int& x, int& y, int& z) {
-        z = g / (tiles_x * tiles_y);
-        const int r = g - z * tiles_x * tiles_y;
-        x = (r % tiles_x) * SC_BX + int(threadIdx.x);
-        y = (r / tiles_x) * MLP_BY + int(threadIdx.y);
-    };
-    auto node_idx = [&](int x, int y, int z) {
-        const unsigned xm = (x == 0) ? L.nx - 1 : x - 1, xp = (x == L.nx - 1) ? 0 : x + 1;
-        const unsigned ym = (y == 0) ? L.ny - 1 : y - 1, yp = (y == L.ny - 1) ? 0 : y + 1;
-        const unsigned zm = (z == 0) ? L.nz - 1 : z - 1, zp = (z == L.nz - 1) ? 0 : z + 1;
-        return NodeIdx<LAY>(L, xm, unsigned(x), xp, ym, unsigned(y), yp, zm, unsigned(z), zp);
-    };
-    for (int g = blockIdx.x; g < ntiles; g += gridDim.x) {
+    /* tile g = (tz tiles_y + ty) tiles_x + tx, advanced by the grid without
+     * dividing again */
+    struct Tile {
         int x, y, z;
-        node_of(g, x, y, z);
-        const bool live = x < L.nx && y < L.ny;
+    };
+    auto tile_of = [&](int g) {
+        const int r = g / tiles_x;
+        return Tile{g - r * tiles_x, r % tiles_y, r / tiles_y};
+    };
+    const Tile hop = tile_of(int(gridDim.x));
+    auto next_of = [&](Tile t) {
+        t.x += hop.x, t.y += hop.y, t.z += hop.z;
+        if (t.x >= tiles_x) t.x -= tiles_x, ++t.y;
+        if (t.y >= tiles_y) t.y -= tiles_y, ++t.z;
+        return t;
+    };
+    /* this thread's node in a tile; its mask byte, or -1 outside the domain */
+    auto cell_of = [&](const Tile& t, int& x, int& y) {
+        x = t.x * SC_BX + int(threadIdx.x), y = t.y * MLP_BY + int(threadIdx.y);
+        return unsigned(t.z) * plane + unsigned(y) * pitch + unsigned(x);
+    };
+    auto mask_of = [&](const Tile& t) {
+        int x, y;
+        const unsigned c = cell_of(t, x, y);
+        return x < L.nx && y < L.ny ? int(mask[c]) : -1;
+    };
+    Tile t = tile_of(int(blockIdx.x));
+    int mbyte = int(blockIdx.x) < ntiles ? mask_of(t) : -1;
+    for (int g = blockIdx.x; g < ntiles; g += gridDim.x) {
+        /* the next tile's mask is on its way during this tile's work */
+        const Tile tn = next_of(t);
+        const int mnext = g + int(gridDim.x) < ntiles ? mask_of(tn) : -1;
+        const bool live = mbyte >= 0;
+        const int type = live ? mbyte & TYPE_MASK : int(FLUID);
+        int x, y;
+        const CellIdx<LAY> n{cell_of(t, x, y), qs};
         float f[19];
-        int type = FLUID;
-        unsigned c = 0;
-        const unsigned xm = (x == 0) ? L.nx - 1 : x - 1, xp = (x == L.nx - 1) ? 0 : x + 1;
-        const unsigned ym = (y == 0) ? L.ny - 1 : y - 1, yp = (y == L.ny - 1) ? 0 : y + 1;
-        const NodeIdx<LAY> n = node_idx(x, y, z);
         if (live) {
-            c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
-            const int mbyte = mask[c];
-            type = mbyte & TYPE_MASK;
-#pragma unroll
-            for (int q = 0; q < 19; ++q) f[q] = F::ld(n.pull(fA, q), L.off[q]);
-            if (HALFWAY && (mbyte & NEAR_SOLID)) {
-                const uint32_t lk = links[c];
-#pragma unroll
-                for (int q = 1; q < 19; ++q)
-                    if (lk & (1u << q)) f[q] = F::ld(n.own(fA, opp(q)), L.off[opp(q)]);
-            }
+            const int z = t.z;
+            const unsigned xm = (x == 0) ? L.nx - 1 : x - 1, xp = (x == L.nx - 1) ? 0 : x + 1;
+            const unsigned ym = (y == 0) ? L.ny - 1 : y - 1, yp = (y == L.ny - 1) ? 0 : y + 1;
+            const unsigned zm = (z == 0) ? L.nz - 1 : z - 1, zp = (z == L.nz - 1) ? 0 : z + 1;
+            const NodeIdx<LAY> ni(L, xm, unsigned(x), xp, ym, unsigned(y), yp, zm, unsigned(z), zp);
             if (type >= WEST_INLET && type <= NORTH_OUTLET) {
-                const unsigned cn = type == WEST_INLET ? c - x + xp : type == EAST_OUTLET ? c - x + xm
-                                  : type == SOUTH_INLET ? c + (yp - y) * pitch : c + (ym - y) * pitch;
+                /* the neighbour's stored state; the rebuild is below */
+                const unsigned cn = type == WEST_INLET ? n.c - x + xp : type == EAST_OUTLET ? n.c - x + xm
+                                  : type == SOUTH_INLET ? n.c + (yp - y) * pitch : n.c + (ym - y) * pitch;
 #pragma unroll
-                for (int q = 0; q < 19; ++q) f[q] = F::ld(n.at(fA, q, cn), L.off[q]);
-                float uin = p.u_in;
-                if (p.noise_amp != 0.f) {
-                    const uint32_t cell = uint32_t((z * L.ny + y) * L.nx + x);
-                    const float xi = philox_uniform(p.noise_seed, cell, uint32_t(sc_time(p)));
-                    uin = uin + p.u_in * p.noise_amp * (2.f * xi - 1.f);
+                for (int q = 0; q < 19; ++q) f[q] = F::ld(ni.at(fA, q, cn), L.off[q]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 19; ++q) f[q] = F::ld(ni.pull(fA, q), L.off[q]);
+                if (HALFWAY && (mbyte & NEAR_SOLID)) {
+                    const uint32_t lk = links[n.c];
+#pragma unroll
+                    for (int q = 1; q < 19; ++q)
+                        if (lk & (1u << q)) f[q] = F::ld(ni.own(fA, opp(q)), L.off[opp(q)]);
                 }
-                extrap<float>(type, f, p.rho_out, uin);
             }
         } else {
 #pragma unroll
@@ -548,8 +575,19 @@ __global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_
             store19<S, LAY, false>(L, fB, n, gb);
         }
         /* the closure for the whole tile; the collision's moments give
-         * Pi_neq (the projected MRT collision on full populations) */
-        const MrtDev<float> mo = mrt_dev_moments<float>(f, 0.f);
+         * Pi_neq (the projected MRT collision on full populations), and an
+         * inlet's or outlet's rebuild is a change of them */
+        MrtDev<float> mo = mrt_dev_sums<float>(f);
+        if (type >= WEST_INLET && type <= NORTH_OUTLET) {
+            float uin = p.u_in;
+            if (p.noise_amp != 0.f) {
+                const uint32_t cell = uint32_t((t.z * L.ny + y) * L.nx + x);
+                const float xi = philox_uniform(p.noise_seed, cell, uint32_t(sc_time(p)));
+                uin = uin + p.u_in * p.noise_amp * (2.f * xi - 1.f);
+            }
+            mrt_dev_extrap(mo, type, p.rho_out, uin, 0.f, 0.f);
+        }
+        mrt_dev_finish(mo, 0.f);
         float p6[6], xf[sgs::NIN];
         mrt_dev_pi(mo, p6);
         const float sc = -1.5f / mo.rho;
@@ -560,13 +598,15 @@ __global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_
          * stresses stay live; the products are formed again afterwards */
         float keep[10] = {mo.rho, mo.jx, mo.jy, mo.jz, mo.n9, mo.n11, mo.n13, mo.n14, mo.n15,
                           sgs::strain_gain(xf, inv_t0)};
-        const float o = sgs::infer_nu<ROWS>(sm, xf, err);
+        const float o = sgs::infer_nu<MLP_ROWS>(sm, xf, err);
         if (o < 0.f) break; /* a tensor-core wait ran out (block-uniform) */
+        t = tn;
+        mbyte = mnext;
         if (!live || solid) continue;
 #pragma unroll
         for (int k = 0; k < 10; ++k) asm volatile("" : "+f"(keep[k]));
         const float nu = o * keep[9];
-        if (p.nu) p.nu[c] = nu;
+        if (p.nu) p.nu[n.c] = nu;
         MrtDev<float> mr;
         mr.rho = keep[0], mr.jx = keep[1], mr.jy = keep[2], mr.jz = keep[3], mr.n9 = keep[4], mr.n11 = keep[5];
         mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8];
@@ -579,11 +619,11 @@ __global__ void __launch_bounds__(SC_BX* MLP_BY, LBM_MLP_MINB) k_stream_collide_
                 if (cx(q)) u += float(cx(q)) * f[q];
                 if (cy(q)) v += float(cy(q)) * f[q];
             }
-            sc_stats(p, stats, qs, c, u, v);
+            sc_stats(p, stats, qs, n.c, u, v);
         }
         store19<S, LAY, false>(L, fB, n, f);
     }
-    sgs::infer_teardown<ROWS>(sm);
+    sgs::infer_teardown<MLP_ROWS>(sm);
 #endif
 }
 
@@ -635,35 +675,12 @@ inline cudaError_t launch_sc_t(const Level& L, const StepParams& p, const void* 
 template <class S, bool HW, int LAY>
 static cudaError_t sc_mlp_t(const Level& L, const StepParams& p, const void* fA, void* fB, const uint8_t* mask,
                             float* stats, const uint32_t* links, const void* blob, int* err, cudaStream_t s) {
-    const size_t smem = sgs::infer_dyn_smem<SC_BX * MLP_BY>();
+    const size_t smem = sgs::infer_dyn_smem<MLP_ROWS>();
     static cudaError_t attr = cudaErrorNotReady;
     static int grid = 0;
-    if (attr == cudaErrorNotReady) {
-        attr = cudaFuncSetAttribute(k_stream_collide_mlp<S, HW, LAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(smem));
-        /* all of the unified L1 / shared array as shared memory, so that the
-         * register limit (6 blocks of 128 threads at 80 registers) decides */
-        if (attr == cudaSuccess)
-            attr = cudaFuncSetAttribute(k_stream_collide_mlp<S, HW, LAY>,
-                                        cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        /* resident blocks per SM from the kernel's own limits: registers,
-         * shared memory, threads, and TMEM (64 columns of 512 per block) */
-        cudaFuncAttributes fa{};
-        int dev = 0, sms = 0, regs_sm = 0, smem_sm = 0;
-        if (attr == cudaSuccess) attr = cudaFuncGetAttributes(&fa, k_stream_collide_mlp<S, HW, LAY>);
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
-        cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-        const int threads = SC_BX * MLP_BY;
-        const int regs_block = ((fa.numRegs > 0 ? fa.numRegs : 255) * 32 + 255) / 256 * 256 * (threads / 32);
-        int nb = regs_sm / (regs_block > 0 ? regs_block : 1);
-        nb = std::min(nb, int(smem_sm / (smem + fa.sharedSizeBytes + 1024)));
-        nb = std::min(nb, 2048 / threads);
-        nb = std::min(nb, 512 / sgs::tmem_cols<SC_BX * MLP_BY>());
-        nb = nb < 1 ? 1 : nb;
-        grid = (sms > 0 ? sms : 152) * nb;
-    }
+    if (attr == cudaErrorNotReady)
+        attr = sgs::infer_resident(k_stream_collide_mlp<S, HW, LAY>, MLP_ROWS, smem, sgs::tmem_cols<MLP_ROWS>(),
+                                   MLP_BLOCKS, &grid);
     if (attr != cudaSuccess) return attr;
     const int ntiles = (L.pitch / SC_BX) * ((L.ny + MLP_BY - 1) / MLP_BY) * L.nz;
     k_stream_collide_mlp<S, HW, LAY><<<grid < ntiles ? grid : ntiles, dim3(SC_BX, MLP_BY), smem, s>>>(

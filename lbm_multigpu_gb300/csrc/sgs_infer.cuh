@@ -44,17 +44,19 @@ constexpr int SM_SMEM_BYTES = 228 * 1024; /* shared memory per SM */
 
 template <int ROWS> struct InferSmem;
 
-/* dynamic shared memory for a block of ROWS rows that holds InferSmem (plus
- * 1 KB of alignment slack) and is large enough that no more blocks than TMEM
- * can serve (512 columns) fit on one SM */
+/* dynamic shared memory for a block of ROWS rows that holds InferSmem and is
+ * large enough that no more blocks than TMEM can
+ * serve (512 columns) fit on one SM */
 template <int ROWS> inline size_t infer_dyn_smem();
 
 template <int ROWS> struct InferSmem {
-    alignas(1024) unsigned char w1[W1_BYTES];
-    alignas(1024) unsigned char w2[W2_BYTES];
+    /* operands without swizzle: the matrix descriptors count 16-byte units
+     * (the three lie on 128-byte boundaries, as the block's array does) */
+    alignas(16) unsigned char w1[W1_BYTES];
+    alignas(16) unsigned char w2[W2_BYTES];
     /* the layer-1 A operand (features, ROWS x 16 bf16) at the start, then
      * h1 over it (written only after the layer-1 MMA has read x) */
-    alignas(1024) unsigned char a2[ROWS * NH * 2];
+    alignas(16) unsigned char a2[ROWS * NH * 2];
     alignas(16) float w3f[NH];
     float b3;
     alignas(8) uint64_t mbar;
@@ -69,19 +71,43 @@ template <int ROWS> struct InferSmem {
 template <int ROWS> __host__ __device__ constexpr int tmem_cols() { return ROWS / 2 < 32 ? 32 : ROWS / 2; }
 
 template <int ROWS> inline size_t infer_dyn_smem() {
-    static size_t v = 0;
-    if (!v) {
-        int dev = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
-            per_sm <= 0)
-            per_sm = SM_SMEM_BYTES;
-        const int max_blocks = 512 / tmem_cols<ROWS>();
-        const size_t need = sizeof(InferSmem<ROWS>) + 1024;
-        const size_t floor = size_t(per_sm) / size_t(max_blocks + 1) + 1;
-        v = need > floor ? need : floor;
+    int dev = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess || per_sm <= 0)
+        per_sm = SM_SMEM_BYTES;
+    const int max_blocks = 512 / tmem_cols<ROWS>();
+    const size_t need = sizeof(InferSmem<ROWS>);
+    const size_t floor = size_t(per_sm) / size_t(max_blocks + 1) + 1;
+    return need > floor ? need : floor;
+}
+
+/* Prepares a kernel of `threads` threads, `smem` bytes of dynamic shared
+ * memory and `cols` TMEM columns to run with up to `most` blocks per SM; *grid
+ * = the blocks that the current device then holds at a time, by the kernel's
+ * own limits: registers, shared memory, threads, and TMEM (the occupancy API
+ * answers 1 for kernels that allocate it).  Only that much of the unified L1 /
+ * shared array is asked for as shared memory: the rest caches the pulls */
+template <class K> inline cudaError_t infer_resident(K kernel, int threads, size_t smem, int cols, int most, int* grid) {
+    cudaFuncAttributes fa{};
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess) return e;
+    int dev = 0, sms = 0, regs_sm = 0, smem_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
+    cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    const int regs_block = ((fa.numRegs > 0 ? fa.numRegs : 255) * 32 + 255) / 256 * 256 * (threads / 32);
+    const int smem_block = int(smem + fa.sharedSizeBytes + 1024);
+    int nb = most;
+    for (int limit : {regs_sm / regs_block, smem_sm / smem_block, 2048 / threads, 512 / cols}) nb = nb < limit ? nb : limit;
+    if (nb < 1) nb = 1;
+    if (smem_sm > 0) {
+        const int share = (nb * smem_block * 100 + smem_sm - 1) / smem_sm;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, share < 100 ? share : 100);
     }
-    return v;
+    *grid = (sms > 0 ? sms : 152) * nb;
+    return e;
 }
 
 #if defined(__CUDA_ARCH__)
@@ -242,7 +268,7 @@ template <int ROWS> __device__ __forceinline__ float infer_nu(InferSmem<ROWS>& s
     ok = infer_mma_wait(s, ph ^ 1u) && ok;
     /* output layer: y = b3 + w3 . relu(z2) in FP32, from the layer-2
      * accumulators (two completions per call: parities ph, ph ^ 1) */
-    float y = s.b3;
+    float2 y2 = make_float2(s.b3, 0.f);
     const uint32_t w3 = tc::smem_u32(s.w3f);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -253,12 +279,13 @@ template <int ROWS> __device__ __forceinline__ float infer_nu(InferSmem<ROWS>& s
 #pragma unroll
         for (int j = 0; j < 16; j += 4) {
             const float4 w = tc::lds128f(w3 + 4 * (16 * c + j));
-            y = fmaf(w.x, fmaxf(__uint_as_float(r[j]), 0.f), y);
-            y = fmaf(w.y, fmaxf(__uint_as_float(r[j + 1]), 0.f), y);
-            y = fmaf(w.z, fmaxf(__uint_as_float(r[j + 2]), 0.f), y);
-            y = fmaf(w.w, fmaxf(__uint_as_float(r[j + 3]), 0.f), y);
+            y2 = __ffma2_rn(make_float2(w.x, w.y), make_float2(fmaxf(__uint_as_float(r[j]), 0.f),
+                                                               fmaxf(__uint_as_float(r[j + 1]), 0.f)), y2);
+            y2 = __ffma2_rn(make_float2(w.z, w.w), make_float2(fmaxf(__uint_as_float(r[j + 2]), 0.f),
+                                                               fmaxf(__uint_as_float(r[j + 3]), 0.f)), y2);
         }
     }
+    const float y = y2.x + y2.y;
     /* two completions per call leave the parity of the next one at ph */
     if (!ok) {
         if ((t & 31) == 0) atomicExch(err, 2);

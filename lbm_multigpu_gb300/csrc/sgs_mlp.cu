@@ -404,10 +404,9 @@ __global__ void __launch_bounds__(128) k_tc_selftest(const __nv_bfloat16* __rest
 __global__ void __launch_bounds__(128) k_mlp_predict_tc(const unsigned char* __restrict__ blob,
                                                         const float* __restrict__ X, int n, float* __restrict__ nu,
                                                         int* __restrict__ err) {
-    extern __shared__ unsigned char dsm[];
-    InferSmem<128>& s =
-        *reinterpret_cast<InferSmem<128>*>((reinterpret_cast<uintptr_t>(dsm) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(128) unsigned char dsm[];
 #if defined(__CUDA_ARCH__)
+    InferSmem<128>& s = *reinterpret_cast<InferSmem<128>*>(dsm);
     infer_setup<128>(s, blob);
     for (int base = blockIdx.x * 128; base < n; base += gridDim.x * 128) {
         const int i = base + threadIdx.x;
