@@ -21,6 +21,7 @@
 
 #include "d3q19.cuh"
 #include "ensemble.cuh"
+#include "lbm_kernels.cuh"
 #include "sgs_infer.cuh"
 
 namespace lbm {
@@ -35,6 +36,7 @@ __device__ __forceinline__ int find_member(const Table& T, int g) {
 template <int TY, int SGS>
 __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float* __restrict__ fA,
                                                       float* __restrict__ fB, float cs) {
+    pdl_wait();
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int g = blockIdx.x; g < T.ntiles; g += gridDim.x) {
         const int mi = find_member(T, g);
@@ -420,12 +422,11 @@ cudaError_t launch_ens_step(const ens::Table& T, const float* fA, float* fB, int
         ens::k_ens_step_mlp<<<grid, ens::MLP_ROWS, smem, lane.stream()>>>(T, fA, fB, (const unsigned char*)blob, err);
         return cudaGetLastError();
     }
-    if (T.ty == 4 && model == ens::SGS_NONE) ens::k_ens_step<4, ens::SGS_NONE><<<grid, 128, 0, s>>>(T, fA, fB, cs);
-    else if (T.ty == 4) ens::k_ens_step<4, ens::SGS_SMAG><<<grid, 128, 0, s>>>(T, fA, fB, cs);
-    else if (T.ty == 8 && model == ens::SGS_NONE) ens::k_ens_step<8, ens::SGS_NONE><<<grid, 256, 0, s>>>(T, fA, fB, cs);
-    else if (T.ty == 8) ens::k_ens_step<8, ens::SGS_SMAG><<<grid, 256, 0, s>>>(T, fA, fB, cs);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    if (T.ty == 4 && model == ens::SGS_NONE) return launch_pdl(ens::k_ens_step<4, ens::SGS_NONE>, grid, 128, s, T, fA, fB, cs);
+    if (T.ty == 4) return launch_pdl(ens::k_ens_step<4, ens::SGS_SMAG>, grid, 128, s, T, fA, fB, cs);
+    if (T.ty == 8 && model == ens::SGS_NONE) return launch_pdl(ens::k_ens_step<8, ens::SGS_NONE>, grid, 256, s, T, fA, fB, cs);
+    if (T.ty == 8) return launch_pdl(ens::k_ens_step<8, ens::SGS_SMAG>, grid, 256, s, T, fA, fB, cs);
+    return cudaErrorInvalidValue;
 }
 
 int ens_step_resident(int ty, int model) {

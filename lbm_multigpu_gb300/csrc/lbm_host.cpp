@@ -868,6 +868,7 @@ int one_step(lbm_handle* h, int rel = -1) {
     /* the history's entry of this step, or with the counter of its step 0 */
     double* const fout = h->force_hist + 3LL * ((rel >= 0 ? rel : t) - c.startf);
     const bool force0 = force && C.nbody > 0;
+    p.early = !force0;
     if (h->trip_in_mask && t >= c.trip_end) {
         /* the trip blocks vanish (DI3's ImageFcn is false from TRIP end on) */
         CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -931,6 +932,7 @@ int one_step(lbm_handle* h, int rel = -1) {
             pf.t = p.t;
             pf.step_dev = step_dev;
             const bool force1 = t > c.startf && i == 0 && Fn.nbody > 0;
+            pf.early = !force1;
             if (force1) CUDA_TRY(fork_force(h, Fn, fout, step_dev));
             CUDA_TRY(launch_stream_collide(Fn.L, pf, Fn.f[Fn.cur], Fn.f[1 - Fn.cur], Fn.mask, Fn.stats, nullptr,
                                            h->stream, Fn.links));
@@ -2063,6 +2065,7 @@ int lbm_stream_collide_f32(const float* fA, float* fB, const uint8_t* mask, int 
     p.t = t;
     p.stats_weight = 1.f;
     p.dyn_y1 = 1 << 30;
+    p.early = 1;
     p.has_lid = 1; /* the caller's mask may hold any node type */
     p.has_xbc = 1;
     CUDA_TRY(launch_stream_collide(L, p, fA, fB, mask, nullptr, nullptr, (cudaStream_t)cuda_stream));

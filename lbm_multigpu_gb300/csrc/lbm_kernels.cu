@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
 /* add n block partials (3 doubles each) to out, in a fixed order: warp k sums
  * component k, lane-strided, then a fixed shuffle tree */
 __global__ void __launch_bounds__(96) k_reduce3(const double* __restrict__ part, int n, double* __restrict__ out) {
+    pdl_wait();
     const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double v = 0.0;
 #pragma unroll 8
@@ -445,6 +446,7 @@ template <class S>
 __global__ void k_interp_cf(const RefineParams r, const Level F, const float* __restrict__ mom_c,
                             const float* __restrict__ mom_prev, float theta, S* __restrict__ f_f,
                             const uint8_t* __restrict__ mask_f) {
+    pdl_wait();
     interp_cf_node<S>(r, F, mom_c, mom_prev, theta, f_f, mask_f, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -540,6 +542,7 @@ __global__ void __launch_bounds__(IFACE_THREADS) k_interface(const RefineParams 
                                                              const uint8_t* __restrict__ mask_f, S* __restrict__ f_c,
                                                              const uint8_t* __restrict__ mask_c, const FcBox b,
                                                              int cf_blocks) {
+    pdl_wait();
     if (int(blockIdx.x) < cf_blocks) {
         interp_cf_node<S>(r, F, mom_c, nullptr, 1.f, f_f, mask_f,
                           (long long)blockIdx.x * IFACE_THREADS + threadIdx.x);
@@ -686,6 +689,7 @@ constexpr int SCAN_WARPS = 8, SCAN_NODES = 512;
 __global__ void __launch_bounds__(32 * SCAN_WARPS) k_force_scan(const Level L, const float* __restrict__ fA,
                                                                 const uint8_t* __restrict__ mask,
                                                                 double* __restrict__ part, int vec) {
+    pdl_wait();
     __shared__ uint16_t list[SCAN_WARPS][SCAN_NODES];
     __shared__ double red[3][SCAN_WARPS];
     double s[3] = {0.0, 0.0, 0.0};
@@ -774,9 +778,9 @@ cudaError_t launch_force_scan(const Level& L, const float* fA, const uint8_t* ma
     if (L.storage != STORE_F32 || L.blocked) return cudaErrorInvalidValue;
     const long long chunks = (L.qstride + SCAN_NODES - 1) / SCAN_NODES;
     const int blocks = int(std::min<long long>(SCAN_BLOCKS, (chunks + SCAN_WARPS - 1) / SCAN_WARPS));
-    k_force_scan<<<blocks, 32 * SCAN_WARPS, 0, s>>>(L, fA, mask, partials, (reinterpret_cast<uintptr_t>(mask) & 15) == 0);
-    k_reduce3<<<1, 96, 0, s>>>(partials, blocks, out3);
-    return cudaGetLastError();
+    const cudaError_t e = launch_pdl(k_force_scan, blocks, 32 * SCAN_WARPS, s, L, fA, mask, partials,
+                                     (reinterpret_cast<uintptr_t>(mask) & 15) == 0);
+    return e != cudaSuccess ? e : launch_pdl(k_reduce3, 1, 96, s, partials, blocks, out3);
 }
 
 cudaError_t launch_init(const Level& L, const uint8_t* mask, void* f, int kind, float u0, cudaStream_t s, int axis) {
@@ -819,8 +823,8 @@ cudaError_t launch_interp_cf(const RefineParams& r, const Level& F, const float*
     const int threads = 128;
     const unsigned blocks = unsigned((n + threads - 1) / threads);
     LBM_DISPATCH(F.storage,
-                 (k_interp_cf<S><<<blocks, threads, 0, s>>>(r, F, mom_c, mom_prev, theta, (S*)f_f, mask_f)));
-    return cudaGetLastError();
+                 return launch_pdl(k_interp_cf<S>, blocks, threads, s, r, F, mom_c, mom_prev, theta, (S*)f_f, mask_f));
+    return cudaErrorInvalidValue;
 }
 
 /* the coarse nodes the restriction replaces: x with x > lrx0 + 1 and
@@ -868,9 +872,9 @@ cudaError_t launch_interface(const RefineParams& r, const Level& C, const Level&
     const int cf_blocks = int((cf_nodes(r) + IFACE_THREADS - 1) / IFACE_THREADS);
     const long long nfc = (long long)b.nxi * b.nyi * b.nzi;
     const unsigned blocks = unsigned(cf_blocks + (nfc + IFACE_THREADS - 1) / IFACE_THREADS);
-    LBM_DISPATCH(C.storage, (k_interface<S><<<blocks, IFACE_THREADS, 0, s>>>(r, C, F, mom_c, (S*)f_f, mask_f, (S*)f_c,
-                                                                             mask_c, b, cf_blocks)));
-    return cudaGetLastError();
+    LBM_DISPATCH(C.storage, return launch_pdl(k_interface<S>, blocks, IFACE_THREADS, s, r, C, F, mom_c, (S*)f_f, mask_f,
+                                              (S*)f_c, mask_c, b, cf_blocks));
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace lbm

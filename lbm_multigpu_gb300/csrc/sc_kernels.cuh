@@ -447,6 +447,7 @@ __global__ void __launch_bounds__(SC_BX* SC_BY, sc_min_blocks<S, FEAT>()) k_stre
                                                                   float* __restrict__ stats,
                                                                   float* __restrict__ mom_export,
                                                                   const uint32_t* __restrict__ links) {
+    pdl_wait();
     const int x = blockIdx.x * SC_BX + threadIdx.x;
     const int y = blockIdx.y * SC_BY + threadIdx.y;
     if (x >= L.nx || y >= L.ny) return;
@@ -642,11 +643,10 @@ inline cudaError_t launch_sc_t(const Level& L, const StepParams& p, const void* 
     const int feat = (p.halfway ? FEAT_HALFWAY : 0) | (p.has_lid ? FEAT_LID : 0) | (p.pull_clamp ? FEAT_CLAMP : 0) |
                      (p.has_xbc ? FEAT_XBC : 0) | (sc_has_devmrt<S>() && p.model == MRT ? FEAT_DEVMRT : 0) | (p.nu_reuse ? FEAT_NUBUF : 0);
     if (!sc_feat_built<S>(feat)) return cudaErrorInvalidValue;
-#define LBM_SC(FT)                                                                                                \
-    case FT:                                                                                                      \
-        k_stream_collide<S, FT, LAY><<<grid, block, 0, s>>>(L, p, (const S*)fA, (S*)fB, mask, stats, mom_export, \
-                                                            links);                                              \
-        break;
+#define LBM_SC(FT)                                                                                            \
+    case FT:                                                                                                  \
+        return launch_pdl_if(p.early, k_stream_collide<S, FT, LAY>, grid, block, s, L, p, (const S*)fA, (S*)fB, \
+                             mask, stats, mom_export, links);
     switch (feat) {
         /* every combination of half-way, lid, clamp and alternate boundaries,
          * without and with the projected MRT */
@@ -669,7 +669,7 @@ inline cudaError_t launch_sc_t(const Level& L, const StepParams& p, const void* 
             }
     }
 #undef LBM_SC
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 template <class S, bool HW, int LAY>
