@@ -544,6 +544,7 @@ struct LevelState {
     float* stats = nullptr;         /* device, 4 x qstride */
     unsigned* body = nullptr;       /* device, pitched indices of BODY nodes */
     int nbody = 0;
+    uint32_t* blinks = nullptr;     /* device, half-way: the listed nodes' links to BODY nodes */
     double* fpart = nullptr;        /* per-block force partials */
     unsigned* done = nullptr;       /* blocks finished in the force kernel (reset by its last block) */
     bool has_lid = false;           /* the mask has LID nodes */
@@ -637,6 +638,7 @@ void free_level(LevelState& s) {
     cudaFree(s.mask);
     cudaFree(s.stats);
     cudaFree(s.body);
+    cudaFree(s.blinks);
     cudaFree(s.fpart);
     cudaFree(s.done);
     cudaFree(s.links);
@@ -708,30 +710,49 @@ int upload_mask(lbm_handle* h, int level) {
     static const int CY[19] = {0, 0, 1, 0, -1, 1, 1, -1, -1, 0, 0, 1, 0, -1, 0, 0, 1, 0, -1};
     static const int CZ[19] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, -1, -1, -1, -1, -1};
     std::vector<unsigned> list;
+    std::vector<uint32_t> blist;
     std::vector<uint32_t> links(halfway ? size_t(L.qstride) : 0, 0u);
     s.has_lid = std::find(s.hmask.begin(), s.hmask.end(), uint8_t(LID)) != s.hmask.end();
     s.has_xbc = std::any_of(s.hmask.begin(), s.hmask.end(), [](uint8_t v) { return v >= DIR_WEST; });
+    /* rows that hold a solid node: away from them a row is its types alone */
+    std::vector<uint8_t> solid_row(size_t(L.ny) * L.nz);
+    for (size_t r = 0; r < solid_row.size(); ++r) {
+        const uint8_t* row = s.hmask.data() + r * L.nx;
+        solid_row[r] = std::any_of(row, row + L.nx, [](uint8_t v) { return v == WALL || v == BODY; });
+    }
     for (int z = 0; z < L.nz; ++z)
-        for (int y = 0; y < L.ny; ++y)
+        for (int y = 0; y < L.ny; ++y) {
+            bool near_row = false;
+            for (int dz = -1; dz <= 1; ++dz)
+                for (int dy = -1; dy <= 1; ++dy) near_row |= solid_row[size_t(nb(z + dz, L.nz)) * L.ny + nb(y + dy, L.ny)] != 0;
+            if (!near_row) {
+                memcpy(pitched.data() + size_t(z) * L.plane + size_t(y) * L.pitch,
+                       s.hmask.data() + (size_t(z) * L.ny + y) * L.nx, L.nx);
+                continue;
+            }
             for (int x = 0; x < L.nx; ++x) {
                 const uint8_t t = type_at(x, y, z);
                 const size_t pc = size_t(z) * L.plane + size_t(y) * L.pitch + x;
                 uint8_t m = t;
-                bool near_solid = false, near_body = false;
-                uint32_t lk = 0;
+                bool near_solid = false;
+                uint32_t lk = 0, blk = 0;
                 if (t != WALL && t != BODY) {
                     for (int q = 1; q < 19; ++q) {
                         const uint8_t u = type_at(nb(x - CX[q], L.nx), nb(y - CY[q], L.ny), nb(z - CZ[q], L.nz));
                         near_solid |= (u == WALL || u == BODY);
-                        near_body |= (u == BODY);
+                        if (u == BODY) blk |= 1u << q;
                         if (u == WALL || u == BODY) lk |= 1u << q;
                     }
                 }
                 if (halfway) links[pc] = lk;
                 if (near_solid) m |= NEAR_SOLID;
                 pitched[pc] = m;
-                if (halfway ? near_body : (t == BODY)) list.push_back(unsigned(pc));
+                if (halfway ? blk != 0 : (t == BODY)) {
+                    list.push_back(unsigned(pc));
+                    if (halfway) blist.push_back(blk);
+                }
             }
+        }
     CUDA_TRY(cudaMemcpyAsync(s.mask, pitched.data(), pitched.size(), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     cudaFree(s.links);
@@ -746,6 +767,12 @@ int upload_mask(lbm_handle* h, int level) {
     if (!list.empty()) {
         CUDA_TRY(cudaMalloc(&s.body, list.size() * sizeof(unsigned)));
         CUDA_TRY(cudaMemcpy(s.body, list.data(), list.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+    }
+    cudaFree(s.blinks);
+    s.blinks = nullptr;
+    if (!blist.empty()) {
+        CUDA_TRY(cudaMalloc(&s.blinks, blist.size() * sizeof(uint32_t)));
+        CUDA_TRY(cudaMemcpy(s.blinks, blist.data(), blist.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     }
     return LBM_OK;
 }
@@ -837,8 +864,7 @@ cudaError_t fork_force(lbm_handle* h, LevelState& s, double* out, const int* ste
     cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
     if (e == cudaSuccess)
-        e = launch_force(s.L, s.f[s.cur], s.body, s.nbody, s.fpart, s.done, out, h->side, s.mask, h->cfg.halfway,
-                         step_dev);
+        e = launch_force(s.L, s.f[s.cur], s.body, s.nbody, s.fpart, s.done, out, h->side, s.blinks, step_dev);
     if (e == cudaSuccess) e = cudaEventRecord(h->ev_join, h->side);
     ++h->launches;
     return e;

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
                                                               const unsigned* __restrict__ body, int nbody,
                                                               double* __restrict__ part, unsigned* __restrict__ done,
                                                               double* __restrict__ out3,
-                                                              const uint8_t* __restrict__ mask, int halfway,
+                                                              const uint32_t* __restrict__ blinks,
                                                               const int* __restrict__ step_dev) {
     using F = Fmt<S>;
     using T = typename F::T;
@@ -78,28 +78,29 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
     const unsigned plane = unsigned(L.plane), pitch = unsigned(L.pitch);
     for (int i = blockIdx.x * FORCE_THREADS + threadIdx.x; i < nbody; i += int(gridDim.x) * FORCE_THREADS) {
         const unsigned c = body[i];
-        const unsigned z = c / plane, r = c - z * plane;
-        const unsigned y = r / pitch, x = r - y * pitch;
-        const unsigned xm = (x == 0) ? L.nx - 1 : x - 1, xp = (x == unsigned(L.nx) - 1) ? 0 : x + 1;
-        const unsigned ym = (y == 0) ? L.ny - 1 : y - 1, yp = (y == unsigned(L.ny) - 1) ? 0 : y + 1;
-        const unsigned zm = (z == 0) ? L.nz - 1 : z - 1, zp = (z == unsigned(L.nz) - 1) ? 0 : z + 1;
-        const unsigned zb[3] = {zm * plane, z * plane, zp * plane};
-        const unsigned yb[3] = {ym * pitch, y * pitch, yp * pitch};
-        const unsigned xs[3] = {xm, x, xp};
         T a[3] = {0, 0, 0};
-        if (halfway) {
+        if (blinks) {
             /* link-wise exchange at a fluid node next to the body: each
              * population heading into a BODY node (opp(q), arriving back as q)
              * hands over 2 c_opp(q) f*_opp(q) */
+            const uint32_t lk = blinks[i];
 #pragma unroll
             for (int q = 1; q < 19; ++q) {
-                if ((mask[zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]] & TYPE_MASK) != BODY) continue;
+                if (!(lk & (1u << q))) continue;
                 const T v = T(2) * F::ld(fA + pidx(L, opp(q), c), L.off[opp(q)]);
                 if (cx(q)) a[0] -= T(cx(q)) * v;
                 if (cy(q)) a[1] -= T(cy(q)) * v;
                 if (cz(q)) a[2] -= T(cz(q)) * v;
             }
         } else {
+            const unsigned z = c / plane, r = c - z * plane;
+            const unsigned y = r / pitch, x = r - y * pitch;
+            const unsigned xm = (x == 0) ? L.nx - 1 : x - 1, xp = (x == unsigned(L.nx) - 1) ? 0 : x + 1;
+            const unsigned ym = (y == 0) ? L.ny - 1 : y - 1, yp = (y == unsigned(L.ny) - 1) ? 0 : y + 1;
+            const unsigned zm = (z == 0) ? L.nz - 1 : z - 1, zp = (z == unsigned(L.nz) - 1) ? 0 : z + 1;
+            const unsigned zb[3] = {zm * plane, z * plane, zp * plane};
+            const unsigned yb[3] = {ym * pitch, y * pitch, yp * pitch};
+            const unsigned xs[3] = {xm, x, xp};
 #pragma unroll
             for (int q = 1; q < 19; ++q) {
                 const T v = T(2) * F::ld(fA + pidx(L, q, zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]), L.off[q]);
@@ -111,21 +112,27 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
 #pragma unroll
         for (int k = 0; k < 3; ++k) s[k] += double(a[k]);
     }
-    __shared__ double red[3][FORCE_THREADS / 32];
+    /* warp k sums component k of the block: lane-strided, then a fixed shuffle
+     * tree (9 FP64 operations a warp; a tree in every warp takes 15) */
+    __shared__ double red[3][FORCE_THREADS];
     __shared__ bool last;
-    for (int k = 0; k < 3; ++k) {
-        double v = s[k];
+    for (int k = 0; k < 3; ++k) red[k][threadIdx.x] = s[k];
+    __syncthreads();
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto tree = [](double v) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
+        return v;
+    };
+    if (k < 3) {
         double v = 0.0;
 #pragma unroll
-        for (int w = 0; w < FORCE_THREADS / 32; ++w) v += red[threadIdx.x][w];
-        if (gridDim.x == 1) out3[threadIdx.x] += v;
-        else part[3 * blockIdx.x + threadIdx.x] = v;
+        for (int i = 0; i < FORCE_THREADS; i += 32) v += red[k][lane + i];
+        v = tree(v);
+        if (lane == 0) {
+            if (gridDim.x == 1) out3[k] += v;
+            else part[3 * blockIdx.x + k] = v;
+        }
     }
     if (gridDim.x == 1) return;
     __threadfence();
@@ -133,13 +140,10 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_list(const Level L, con
     if (threadIdx.x == 0) last = (atomicAdd(done, 1u) == gridDim.x - 1);
     __syncthreads();
     if (last) {
-        /* warp k sums component k: lane-strided partials, then a fixed shuffle tree */
-        const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (k < 3) {
             double v = 0.0;
             for (int b = lane; b < int(gridDim.x); b += 32) v += __ldcg(part + 3 * b + k);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            v = tree(v);
             if (lane == 0) out3[k] += v;
         }
         if (threadIdx.x == 0) *done = 0u;
@@ -665,12 +669,11 @@ cudaError_t launch_advance_step(int* step_dev, int k, cudaStream_t s) {
 int force_partials() { return FORCE_BLOCKS; }
 
 cudaError_t launch_force(const Level& L, const void* fA, const unsigned* body, int nbody, double* partials,
-                         unsigned* done, double* out3, cudaStream_t s, const uint8_t* mask, int halfway,
-                         const int* step_dev) {
+                         unsigned* done, double* out3, cudaStream_t s, const uint32_t* blinks, const int* step_dev) {
     if (nbody <= 0) return cudaSuccess;
     const int blocks = std::min(FORCE_BLOCKS, (nbody + FORCE_THREADS - 1) / FORCE_THREADS);
     LBM_DISPATCH(L.storage, (k_force_list<S><<<blocks, FORCE_THREADS, 0, s>>>(L, (const S*)fA, body, nbody, partials,
-                                                                              done, out3, mask, halfway, step_dev)));
+                                                                              done, out3, blinks, step_dev)));
     return cudaGetLastError();
 }
 

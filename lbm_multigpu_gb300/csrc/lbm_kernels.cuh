@@ -215,11 +215,12 @@ cudaError_t launch_stream_collide(const Level& L, const StepParams& p, const voi
 cudaError_t launch_stream_collide_mlp(const Level& L, const StepParams& p, const void* fA, void* fB,
                                       const uint8_t* mask, float* stats, const uint32_t* links, const void* blob,
                                       int* err, cudaStream_t s);
-/* FP64 momentum exchange over a list of BODY nodes (pitched indices), ADDED to
- * out3 (with step_dev, to out3 + 3 *step_dev) */
+/* FP64 momentum exchange over a list of BODY nodes (pitched indices), or with
+ * blinks of the fluid nodes next to them (half-way bounce-back; bit q of
+ * blinks[i]: the pull source of q is a BODY node), ADDED to out3 (with
+ * step_dev, to out3 + 3 *step_dev) */
 cudaError_t launch_force(const Level& L, const void* fA, const unsigned* body, int nbody, double* partials,
-                         unsigned* done, double* out3, cudaStream_t s, const uint8_t* mask = nullptr,
-                         int halfway = 0, const int* step_dev = nullptr);
+                         unsigned* done, double* out3, cudaStream_t s, const uint32_t* blinks, const int* step_dev);
 /* the device's step counter: set, and advanced by k */
 cudaError_t launch_set_step(int* step_dev, int t, cudaStream_t s);
 cudaError_t launch_advance_step(int* step_dev, int k, cudaStream_t s);
