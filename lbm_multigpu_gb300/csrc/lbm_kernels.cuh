@@ -312,6 +312,12 @@ cudaError_t launch_mlp_grad(const float* params, const float* X, const float* T,
 /* sums the partials; with step > 0 also one Adam step on params (m, v state) */
 cudaError_t launch_mlp_adam(const float* grad_part, int nblocks, float* params, float* m, float* v, float* grad_out,
                             float* loss_out, float lr, int step, cudaStream_t s);
+/* one epoch of the seeded mini-batch shuffle of perm[n] on the device (epoch 0
+ * starts from 0 .. n - 1): the swaps of Fisher-Yates with the n - 1 draws of
+ * splitmix64 that follow `state`; scratch: shuffle_scratch_bytes(n), kept from
+ * epoch to epoch */
+size_t shuffle_scratch_bytes(int n);
+cudaError_t launch_shuffle(int* perm, int n, unsigned long long state, int epoch, void* scratch, cudaStream_t s);
 cudaError_t launch_mlp_predict(const float* params, const float* X, int n, float* nu, cudaStream_t s);
 cudaError_t launch_tc_selftest(const void* A, const void* B, int kc, float* D, int* err, cudaStream_t s);
 /* tensor-core inference of n samples from a weight blob (sgs::BLOB_BYTES, see

@@ -41,6 +41,7 @@ struct Rng {
         z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
         return z ^ (z >> 31);
     }
+    void skip(uint64_t draws) { s += draws * 0x9E3779B97F4A7C15ull; }
     double uniform() { return double(next() >> 11) * (1.0 / 9007199254740992.0); }
 };
 
@@ -145,26 +146,25 @@ int lbm_mlp_train(const float* d_X, const float* d_T, int n, int batch, int step
     const int nb = mlp_grad_blocks(batch);
     DevBuf<float> P, M, V, part, loss;
     DevBuf<int> idx;
+    DevBuf<unsigned char> shuffle;
     SGS_TRY(P.alloc(sgs::NPARAM), "cudaMalloc");
     SGS_TRY(M.alloc(sgs::NPARAM), "cudaMalloc");
     SGS_TRY(V.alloc(sgs::NPARAM), "cudaMalloc");
     SGS_TRY(part.alloc(size_t(nb) * (sgs::NPARAM + 1)), "cudaMalloc");
     SGS_TRY(loss.alloc(size_t(steps > 0 ? steps : 1)), "cudaMalloc");
     SGS_TRY(idx.alloc(size_t(n)), "cudaMalloc");
+    SGS_TRY(shuffle.alloc(shuffle_scratch_bytes(n)), "cudaMalloc");
     SGS_TRY(cudaMemcpyAsync(P.p, params, sgs::NPARAM * sizeof(float), cudaMemcpyHostToDevice, s), "params upload");
     SGS_TRY(cudaMemsetAsync(M.p, 0, sgs::NPARAM * sizeof(float), s), "memset");
     SGS_TRY(cudaMemsetAsync(V.p, 0, sgs::NPARAM * sizeof(float), s), "memset");
-    /* epochs over a seeded permutation; one pinned-free upload per epoch */
+    /* epochs over a seeded permutation, shuffled on the device; an epoch takes
+     * n - 1 draws */
     Rng r(seed);
-    std::vector<int> perm(n);
-    for (int i = 0; i < n; ++i) perm[i] = i;
-    int pos = n;
+    int pos = n, epoch = 0;
     for (int st = 0; st < steps; ++st) {
         if (pos + batch > n) {
-            for (int i = n - 1; i > 0; --i) std::swap(perm[i], perm[int(r.next() % uint64_t(i + 1))]);
-            SGS_TRY(cudaMemcpyAsync(idx.p, perm.data(), size_t(n) * sizeof(int), cudaMemcpyHostToDevice, s),
-                    "index upload");
-            SGS_TRY(cudaStreamSynchronize(s), "index upload");
+            SGS_TRY(launch_shuffle(idx.p, n, r.s, epoch++, shuffle.p, s), "shuffle launch");
+            r.skip(uint64_t(n - 1));
             pos = 0;
         }
         SGS_TRY(launch_mlp_grad(P.p, d_X, d_T, idx.p + pos, batch, part.p, nb, s), "gradient launch");

@@ -125,6 +125,44 @@ def test_mlp_tiles_match_oracle(product, n, shift):
     np.testing.assert_allclose(nu.cpu().numpy(), want, rtol=2e-5, atol=1e-10)
 
 
+@pytest.mark.parametrize("n,epochs", [(1, 3), (2, 4), (33, 3), (1000, 2), (20011, 2)])
+def test_shuffle_is_fisher_yates(product, n, epochs):
+    """the mini-batch order is that of the sequential shuffle: with batches of
+    one and a vanishing learning rate the loss history is the loss of each
+    sample in turn"""
+    torch = pytest.importorskip("torch")
+    lib = product.library()
+    seed = 9
+    X = np.zeros((n, NIN), np.float32)
+    X[:, 15] = 1
+    T = ((1 + np.arange(n)) * np.float32(1e-4)).astype(np.float32)   # one loss per sample
+    P, hist = _params(lib, 3), np.zeros(n * epochs, np.float32)
+    dX, dT = _dev(torch, X), _dev(torch, T)
+    assert lib.lbm_mlp_train(ctypes.c_void_p(dX.data_ptr()), ctypes.c_void_p(dT.data_ptr()), n, 1, n * epochs,
+                             ctypes.c_float(1e-30), seed, ptr(P), ptr(hist), None) == 0, lib.lbm_last_error()
+    state, m64, perm, want = (seed * 0x9E3779B97F4A7C15 + 0x632BE59BD9B4E019) % 2 ** 64, 2 ** 64 - 1, list(range(n)), []
+    for _ in range(epochs):
+        for i in range(n - 1, 0, -1):
+            state = (state + 0x9E3779B97F4A7C15) & m64
+            z = ((state ^ (state >> 30)) * 0xBF58476D1CE4E5B9) & m64
+            z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & m64
+            j = (z ^ (z >> 31)) % (i + 1)
+            perm[i], perm[j] = perm[j], perm[i]
+        want += perm
+    # loss = (o / 1e-4 - (1 + index))^2 with the same o for every sample, o below 20
+    o = np.zeros(n, np.float32)
+    do = _dev(torch, o)
+    dP = _dev(torch, P)
+    assert lib.lbm_mlp_predict(ctypes.c_void_p(dP.data_ptr()), ctypes.c_void_p(dX.data_ptr()), n,
+                               ctypes.c_void_p(do.data_ptr()), None) == 0
+    torch.cuda.synchronize()
+    base = float(do[0].item()) / 1e-4
+    # the loss of index k rounds at 2^-23 (k + 1)^2 relative to steps of 2 (k + 1 - base): under half a step to 2^21
+    got = np.sqrt(hist.astype(np.float64))
+    loss = np.abs(base - (1 + np.arange(n)))
+    np.testing.assert_allclose(got, loss[want], rtol=0, atol=0.02 + 1e-6 * n)
+
+
 def test_training_reduces_loss(product):
     torch = pytest.importorskip("torch")
     lib = product.library()
