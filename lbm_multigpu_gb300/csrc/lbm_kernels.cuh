@@ -184,10 +184,12 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... P, class... A>
-inline cudaError_t launch_pdl_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
+inline cudaError_t launch_pdl_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                 A&&... args) {
     cudaLaunchConfig_t c{};
     c.gridDim = grid;
     c.blockDim = block;
+    c.dynamicSmemBytes = smem;
     c.stream = s;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -198,7 +200,7 @@ inline cudaError_t launch_pdl_if(bool early, void (*kernel)(P...), dim3 grid, di
 }
 template <class... P, class... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
-    return launch_pdl_if(true, kernel, grid, block, s, std::forward<A>(args)...);
+    return launch_pdl_if(true, kernel, grid, block, 0, s, std::forward<A>(args)...);
 }
 #endif
 

@@ -645,7 +645,7 @@ inline cudaError_t launch_sc_t(const Level& L, const StepParams& p, const void* 
     if (!sc_feat_built<S>(feat)) return cudaErrorInvalidValue;
 #define LBM_SC(FT)                                                                                            \
     case FT:                                                                                                  \
-        return launch_pdl_if(p.early, k_stream_collide<S, FT, LAY>, grid, block, s, L, p, (const S*)fA, (S*)fB, \
+        return launch_pdl_if(p.early, k_stream_collide<S, FT, LAY>, grid, block, 0, s, L, p, (const S*)fA, (S*)fB, \
                              mask, stats, mom_export, links);
     switch (feat) {
         /* every combination of half-way, lid, clamp and alternate boundaries,

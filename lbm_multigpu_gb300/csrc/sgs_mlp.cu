@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(GTH, 2) k_mlp_grad(const float* __restrict__ p
                                                      float inv_n, float* __restrict__ grad_part, int vec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     GradSmem& s = *reinterpret_cast<GradSmem*>(smem_raw);
+    pdl_wait();
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
     const int u0 = unit0(), q0 = sample0();
     fwd_weights(s, params);
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(32 * ADAM_WARPS) k_mlp_adam(const float* __res
                                                               float* __restrict__ loss_out, float lr, float b1,
                                                               float b2, float eps, int step) {
     __shared__ float part[ADAM_WARPS][32];
+    pdl_wait();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int p = blockIdx.x * 32 + lane;
     float g = 0.f;
@@ -536,16 +538,15 @@ cudaError_t launch_mlp_grad(const float* params, const float* X, const float* T,
     cudaError_t e = cudaFuncSetAttribute(sgs::k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm));
     if (e != cudaSuccess) return e;
     const float inv_n = 1.f / float(n > 0 ? n : 1);
-    sgs::k_mlp_grad<<<nblocks, sgs::GTH, sm, s>>>(params, X, T, idx, n, inv_n, grad_part, vec16(X));
-    return cudaGetLastError();
+    return launch_pdl_if(true, sgs::k_mlp_grad, nblocks, sgs::GTH, sm, s, params, X, T, idx, n, inv_n, grad_part,
+                         vec16(X));
 }
 
 cudaError_t launch_mlp_adam(const float* grad_part, int nblocks, float* params, float* m, float* v, float* grad_out,
                             float* loss_out, float lr, int step, cudaStream_t s) {
     const int n = sgs::NPARAM + 1;
-    sgs::k_mlp_adam<<<(n + 31) / 32, 32 * sgs::ADAM_WARPS, 0, s>>>(grad_part, nblocks, params, m, v, grad_out, loss_out,
-                                                                   lr, 0.9f, 0.999f, 1e-8f, step);
-    return cudaGetLastError();
+    return launch_pdl(sgs::k_mlp_adam, (n + 31) / 32, 32 * sgs::ADAM_WARPS, s, grad_part, nblocks, params, m, v,
+                      grad_out, loss_out, lr, 0.9f, 0.999f, 1e-8f, step);
 }
 
 cudaError_t launch_mlp_predict(const float* params, const float* X, int n, float* nu, cudaStream_t s) {
