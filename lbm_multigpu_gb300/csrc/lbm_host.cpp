@@ -599,6 +599,10 @@ struct lbm_handle {
      * stream: forked after the previous step, joined before the next */
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    /* refinement: a coarse step's first fine sub-step reads nothing of the
+     * coarse level, so it runs beside the coarse stream-collide on this stream */
+    cudaStream_t fine = nullptr;
+    cudaEvent_t ev_fine0 = nullptr, ev_fine1 = nullptr;
     /* lbm_step runs batches of 2, 4, 8 or 16 steps as CUDA graphs, which
      * removes the gaps between their launches.  The step number lives on the
      * device (step_dev, which a graph advances by its length), so that a
@@ -859,10 +863,10 @@ int do_init(lbm_handle* h) {
  * joins (waits for ev_join) once the step's stream-collide is queued.  The
  * force kernel adds into `out` (3 doubles), which is zero or holds the other
  * level's sum of the same step; with step_dev, out is the history's entry of
- * device step 0. */
-cudaError_t fork_force(lbm_handle* h, LevelState& s, double* out, const int* step_dev) {
-    cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
+ * device step 0.  after: the event it waits for instead of the main stream. */
+cudaError_t fork_force(lbm_handle* h, LevelState& s, double* out, const int* step_dev, cudaEvent_t after) {
+    cudaError_t e = after ? cudaSuccess : cudaEventRecord(h->ev_fork, h->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, after ? after : h->ev_fork, 0);
     if (e == cudaSuccess)
         e = launch_force(s.L, s.f[s.cur], s.body, s.nbody, s.fpart, s.done, out, h->side, s.blinks, step_dev);
     if (e == cudaSuccess) e = cudaEventRecord(h->ev_join, h->side);
@@ -872,8 +876,9 @@ cudaError_t fork_force(lbm_handle* h, LevelState& s, double* out, const int* ste
 
 /* one base step and, with refinement, the patch sub-steps and the two
  * interpolations; the order of LR7:2849-2950.  rel >= 0: the launches carry
- * the step as rel steps past the device's counter instead of h->t */
-int one_step(lbm_handle* h, int rel = -1) {
+ * the step as rel steps past the device's counter instead of h->t.  chained:
+ * nothing was queued since the step before, in the same capture */
+int one_step(lbm_handle* h, int rel = -1, bool chained = false) {
     const Config& c = h->cfg;
     const int t = h->t;
     const int* step_dev = rel >= 0 ? h->step_dev : nullptr;
@@ -894,7 +899,7 @@ int one_step(lbm_handle* h, int rel = -1) {
     /* the history's entry of this step, or with the counter of its step 0 */
     double* const fout = h->force_hist + 3LL * ((rel >= 0 ? rel : t) - c.startf);
     const bool force0 = force && C.nbody > 0;
-    p.early = !force0;
+    p.early = !force0 && !c.refinement;
     if (h->trip_in_mask && t >= c.trip_end) {
         /* the trip blocks vanish (DI3's ImageFcn is false from TRIP end on) */
         CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -905,7 +910,36 @@ int one_step(lbm_handle* h, int rel = -1) {
     }
     if (c.sgs_mlp && !h->mlp_ready)
         return fail(LBM_ERR_STATE, "SGS mlp: no weights (SGS weights record line or lbm_set_sgs_mlp)");
-    if (force0) CUDA_TRY(fork_force(h, C, fout, step_dev));
+    if (force0) CUDA_TRY(fork_force(h, C, fout, step_dev, nullptr));
+    /* the next fine sub-step */
+    auto fine_step = [&](cudaStream_t s, bool early, int band) {
+        LevelState& Fn = h->lv[1];
+        StepParams pf = base_params(h, 1);
+        pf.t = p.t;
+        pf.step_dev = step_dev;
+        pf.early = early;
+        pf.band = band;
+        pf.band_z = h->rp.zbounded;
+        const cudaError_t e = launch_stream_collide(Fn.L, pf, Fn.f[Fn.cur], Fn.f[1 - Fn.cur], Fn.mask, Fn.stats, nullptr,
+                                                    s, Fn.links);
+        ++h->launches;
+        Fn.cur = 1 - Fn.cur;
+        return e;
+    };
+    bool force1 = false;
+    if (c.refinement) {
+        /* beside the coarse stream-collide: the fine level's force reduction
+         * and its first sub-step, both of the state that the step before left
+         * there; in a chain of steps also beside that step's restriction,
+         * which only reads the fine level */
+        LevelState& Fn = h->lv[1];
+        force1 = t > c.startf && Fn.nbody > 0;
+        if (!chained) CUDA_TRY(cudaEventRecord(h->ev_fine0, h->stream));
+        if (force1) CUDA_TRY(fork_force(h, Fn, fout, step_dev, h->ev_fine0));
+        CUDA_TRY(cudaStreamWaitEvent(h->fine, h->ev_fine0, 0));
+        CUDA_TRY(fine_step(h->fine, false, 0));
+        CUDA_TRY(cudaEventRecord(h->ev_fine1, h->fine));
+    }
     /* CF TIME linear: this step's export goes to the other buffer, the last
      * one is kept for the interpolation in time */
     bool blend = false;
@@ -946,30 +980,25 @@ int one_step(lbm_handle* h, int rel = -1) {
     }
     if (c.refinement) {
         LevelState& Fn = h->lv[1];
-        const int L = int(std::lround(1.0 / c.lrfactor));
-        for (int i = 0; i < L; ++i) {
-            if (blend && i > 0) {
-                /* the band at fine time i / L of the coarse step */
-                CUDA_TRY(launch_interp_cf(h->rp, Fn.L, h->mom, Fn.f[Fn.cur], Fn.mask, h->stream, h->mom_prev,
-                                          float(i) / float(L)));
+        const int L = h->rp.lrlevel;
+        CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_fine1, 0));
+        if (force1) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
+        for (int i = 1; i < L; ++i) {
+            /* before fine sub-step i the band at fine time i / L of the coarse
+             * step, where it is blended in time; before the last one also the
+             * band at its end, into the buffer that sub-step writes (which
+             * leaves the band out): one launch for both */
+            const bool last = i == L - 1;
+            if (blend || last) {
+                CUDA_TRY(launch_interp_cf(h->rp, Fn.L, h->mom, h->mom_prev, float(i) / float(L),
+                                          last ? Fn.f[1 - Fn.cur] : nullptr, blend ? Fn.f[Fn.cur] : nullptr, Fn.mask,
+                                          h->stream));
                 ++h->launches;
             }
-            StepParams pf = base_params(h, 1);
-            pf.t = p.t;
-            pf.step_dev = step_dev;
-            const bool force1 = t > c.startf && i == 0 && Fn.nbody > 0;
-            pf.early = !force1;
-            if (force1) CUDA_TRY(fork_force(h, Fn, fout, step_dev));
-            CUDA_TRY(launch_stream_collide(Fn.L, pf, Fn.f[Fn.cur], Fn.f[1 - Fn.cur], Fn.mask, Fn.stats, nullptr,
-                                           h->stream, Fn.links));
-            ++h->launches;
-            if (force1) CUDA_TRY(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
-            Fn.cur = 1 - Fn.cur;
+            CUDA_TRY(fine_step(h->stream, true, last ? L : 0));
         }
-        /* the band fill at the end of the coarse step and the restriction
-         * touch disjoint nodes (band vs the coarse nodes over the interior
-         * with its 2-node margin): one launch */
-        CUDA_TRY(launch_interface(h->rp, C.L, Fn.L, h->mom, Fn.f[Fn.cur], Fn.mask, C.f[C.cur], C.mask, h->stream));
+        CUDA_TRY(cudaEventRecord(h->ev_fine0, h->stream));
+        CUDA_TRY(launch_interp_fc(h->rp, C.L, Fn.L, Fn.f[Fn.cur], C.f[C.cur], C.mask, h->stream));
         ++h->launches;
     }
     h->t = t + 1;
@@ -1094,7 +1123,7 @@ int run_graph(lbm_handle* h, int lg) {
     sg.mom = mom0;
     CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LBM_OK;
-    for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h, sg.steady ? j : -1);
+    for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h, sg.steady ? j : -1, j > 0);
     if (rc == LBM_OK && sg.steady && uses_counter(h, sg.force)) {
         const cudaError_t e = launch_advance_step(h->step_dev, k, h->stream);
         if (e != cudaSuccess) rc = fail(LBM_ERR_CUDA, "step counter: %s", cudaGetErrorString(e));
@@ -1307,6 +1336,10 @@ int lbm_create(const char* inputs_text, lbm_handle** out) {
             cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess)
             return bail(fail(LBM_ERR_CUDA, "cannot create the force stream"));
+        if (c.refinement && (cudaStreamCreateWithPriority(&h->fine, cudaStreamNonBlocking, hi) != cudaSuccess ||
+                             cudaEventCreateWithFlags(&h->ev_fine0, cudaEventDisableTiming) != cudaSuccess ||
+                             cudaEventCreateWithFlags(&h->ev_fine1, cudaEventDisableTiming) != cudaSuccess))
+            return bail(fail(LBM_ERR_CUDA, "cannot create the fine level's stream"));
     }
     /* reference velocity of the FP16/BF16 offsets: the inlet velocity of a channel */
     const float u_ref = c.geometry.rfind("channel", 0) == 0 || c.geometry == "duct" ? c.umax : 0.f;
@@ -1387,6 +1420,9 @@ int lbm_destroy(lbm_handle* h) {
     cudaFree(h->dyn_hist);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
+    if (h->ev_fine0) cudaEventDestroy(h->ev_fine0);
+    if (h->ev_fine1) cudaEventDestroy(h->ev_fine1);
+    if (h->fine) cudaStreamDestroy(h->fine);
     for (auto& row : h->graphs)
         for (StepGraph& g : row)
             if (g.exec) cudaGraphExecDestroy(g.exec);

@@ -332,12 +332,6 @@ __device__ __forceinline__ void second_order_scale(float a[9]) {
     for (int j = 0; j < 9; ++j) a[j] *= (j % 4 == 0) ? -0.03125f : -0.0625f;
 }
 
-/* InterpCF (LR7:1991-2170): fine nodes of the LRLEVEL-wide x/y band get the
- * coarse moments interpolated (trilinear + second-order velocity correction)
- * and rebuilt with the LES-aware non-equilibrium rescale (LR7:524-579).  One
- * thread per band node; mom_c is [9][cnz][eny][enx] (coarse footprint).
- * With mom_prev (the previous coarse step's export) the corner moments are
- * first interpolated in time, (1 - theta) prev + theta cur. */
 /* band nodes of the coarse-to-fine fill */
 inline long long cf_nodes(const RefineParams& r) {
     const int L = r.lrlevel;
@@ -345,82 +339,12 @@ inline long long cf_nodes(const RefineParams& r) {
            (r.zbounded ? 2LL * L * (r.fnx - 2 * L) * (r.fny - 2 * L) : 0LL);
 }
 
-/* the band node idx of the coarse-to-fine fill */
+/* the interpolated moments of a band node, rebuilt into its populations with
+ * the LES-aware non-equilibrium rescale (LR7:524-579): mom and a are the sums
+ * over the corners of the trilinear moments and of the second-order terms */
 template <class S>
-__device__ __forceinline__ void interp_cf_node(const RefineParams& r, const Level& F, const float* __restrict__ mom_c,
-                                               const float* __restrict__ mom_prev, float theta, S* __restrict__ f_f,
-                                               const uint8_t* __restrict__ mask_f, const long long idx) {
-    const int L = r.lrlevel;
-    const int nb_x = r.fny * 2 * L;                /* x-band nodes per plane */
-    const int nb_y = (r.fnx - 2 * L) * 2 * L;      /* y-band nodes per plane (x-band excluded) */
-    const int per_plane = nb_x + nb_y;
-    const int inner = (r.fnx - 2 * L) * (r.fny - 2 * L);  /* z-band nodes per plane (bounded patch) */
-    const long long nxy = (long long)per_plane * r.fnz;
-    if (idx >= nxy + (r.zbounded ? 2LL * L * inner : 0LL)) return;
-    int k, xf, yf;
-    if (idx < nxy) {
-        k = int(idx / per_plane);
-        int i = int(idx % per_plane);
-        if (i < nb_x) {
-            yf = i / (2 * L);
-            const int b = i % (2 * L);
-            xf = b < L ? b : r.fnx - 2 * L + b;
-        } else {
-            i -= nb_x;
-            xf = L + i / (2 * L);
-            const int b = i % (2 * L);
-            yf = b < L ? b : r.fny - 2 * L + b;
-        }
-    } else {
-        /* the L bottom and L top planes of a bounded patch, x/y band excluded */
-        const int j = int(idx - nxy), b = j / inner, rem = j % inner;
-        k = b < L ? b : r.fnz - 2 * L + b;
-        xf = L + rem % (r.fnx - 2 * L);
-        yf = L + rem / (r.fnx - 2 * L);
-    }
-    const long long cf = k * F.plane + (long long)yf * F.pitch + xf;
-    const int t = mask_f[cf] & TYPE_MASK;
-    if (t == WALL || t == BODY) return;
-    const float xr = xf * r.lrfactor + r.lrfactor * 0.5f, yr = yf * r.lrfactor + r.lrfactor * 0.5f;
-    const int xm = int(xr), ym = int(yr);
-    const float fx = xr - xm, fy = yr - ym;
-    /* z: periodic full-depth patch (fine plane k at coarse z k / L - 1 +
-     * ...), or, bounded, as x and y from the coarse plane cz0 */
-    int zb;
-    float fz;
-    if (r.zbounded) {
-        const float zr = k * r.lrfactor + r.lrfactor * 0.5f;
-        zb = r.cz0 + int(zr);
-        fz = zr - int(zr);
-    } else {
-        zb = k / L - 1;
-        fz = (k % L) * r.lrfactor + r.lrfactor * 0.5f;
-    }
-    const long long ne = (long long)r.enx * r.eny * r.cnz;
-    /* trilinear moments and the second-order terms, one corner at a time */
-    float mom[9], a[9];
-#pragma unroll
-    for (int m = 0; m < 9; ++m) mom[m] = a[m] = 0.f;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        int zc = zb + ((c >> 2) & 1);
-        zc = zc < 0 ? zc + r.cnz : (zc >= r.cnz ? zc - r.cnz : zc);
-        const long long ce = ((long long)zc * r.eny + (ym + ((c >> 1) & 1))) * r.enx + (xm + (c & 1));
-        float mc[9], Sc[6];
-#pragma unroll
-        for (int m = 0; m < 9; ++m) mc[m] = __ldg(mom_c + m * ne + ce);
-        if (mom_prev) {
-#pragma unroll
-            for (int m = 0; m < 9; ++m) mc[m] = (1.f - theta) * __ldg(mom_prev + m * ne + ce) + theta * mc[m];
-        }
-        const float wx = (c & 1) ? fx : 1.f - fx, wy = (c & 2) ? fy : 1.f - fy, wz = (c & 4) ? fz : 1.f - fz;
-#pragma unroll
-        for (int m = 0; m < 9; ++m) mom[m] += mc[m] * wx * wy * wz;
-        if (r.order == 2) {
-            strain_rate<float>(mc, Sc);
-            second_order_add(a, c, mc, Sc);
-        }
-    }
+__device__ __forceinline__ void interp_cf_store(const RefineParams& r, const Level& F, float mom[9], float a[9],
+                                                float fx, float fy, float fz, S* __restrict__ f_f, unsigned cf) {
     if (r.order == 2) {
         second_order_scale(a);
         const float wx = 1.f - (4.f * fx * fx - 4.f * fx + 1.f);
@@ -443,15 +367,127 @@ __device__ __forceinline__ void interp_cf_node(const RefineParams& r, const Leve
     float g[19];
     invert_scaled<float>(mom, SF, g);
 #pragma unroll
-    for (int q = 0; q < 19; ++q) Fmt<S>::st(f_f + pidx(F, q, unsigned(cf)), g[q], F.off[q]);
+    for (int q = 0; q < 19; ++q) Fmt<S>::st(f_f + pidx(F, q, cf), g[q], F.off[q]);
 }
 
-template <class S>
-__global__ void k_interp_cf(const RefineParams r, const Level F, const float* __restrict__ mom_c,
-                            const float* __restrict__ mom_prev, float theta, S* __restrict__ f_f,
-                            const uint8_t* __restrict__ mask_f) {
+/* InterpCF (LR7:1991-2170): fine nodes of the LRLEVEL-wide x/y band get the
+ * coarse moments interpolated (trilinear + second-order velocity correction).
+ * mom_c is [9][cnz][eny][enx] (coarse footprint), mom_prev the previous coarse
+ * step's export.  FILL_END: f_end from mom_c;
+ * FILL_MID: f_mid with the corner moments first interpolated in time, (1 -
+ * theta) mom_prev + theta mom_c; both together share their loads and one
+ * launch.
+ * Bound by latency (some 62,000 nodes, 72 or 144 loads each): two lanes per
+ * node, one for the four corners at lower x and one for the upper, which
+ * exchange their sums; with both fills one lane finishes each, else the first
+ * finishes alone.  Both fills 13.3 us (the end's beside the restriction and the
+ * middle's alone took 17.0 + 10.4 us); whole cells of moments stored together
+ * for wider loads measured the same (13.7 us). */
+constexpr int FILL_END = 1, FILL_MID = 2;
+constexpr int IFACE_THREADS = 128;
+template <class S, int FILL>
+__global__ void __launch_bounds__(IFACE_THREADS) k_interp_cf(const RefineParams r, const Level F, const float* __restrict__ mom_c,
+                                                  const float* __restrict__ mom_prev, float theta, S* __restrict__ f_end,
+                                                  S* __restrict__ f_mid, const uint8_t* __restrict__ mask_f) {
     pdl_wait();
-    interp_cf_node<S>(r, F, mom_c, mom_prev, theta, f_f, mask_f, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+    /* a level indexes below 2^31: 32-bit arithmetic (a 64-bit division is a
+     * hundred instructions) */
+    const unsigned nidx = (blockIdx.x * blockDim.x + threadIdx.x) >> 1;
+    const int half = threadIdx.x & 1;
+    const int L = r.lrlevel;
+    const unsigned nb_x = r.fny * 2 * L;                /* x-band nodes per plane */
+    const unsigned nb_y = (r.fnx - 2 * L) * 2 * L;      /* y-band nodes per plane (x-band excluded) */
+    const unsigned per_plane = nb_x + nb_y;
+    const unsigned inner = (r.fnx - 2 * L) * (r.fny - 2 * L);  /* z-band nodes per plane (bounded patch) */
+    const unsigned nxy = per_plane * r.fnz;
+    const unsigned nodes = nxy + (r.zbounded ? 2 * L * inner : 0);
+    /* lanes past the end work on the last node and store nothing */
+    const unsigned idx = nidx < nodes ? nidx : nodes - 1;
+    int k, xf, yf;
+    if (idx < nxy) {
+        k = int(idx / per_plane);
+        unsigned i = idx % per_plane;
+        if (i < nb_x) {
+            yf = int(i / (2 * L));
+            const int b = int(i % (2 * L));
+            xf = b < L ? b : r.fnx - 2 * L + b;
+        } else {
+            i -= nb_x;
+            xf = L + int(i / (2 * L));
+            const int b = int(i % (2 * L));
+            yf = b < L ? b : r.fny - 2 * L + b;
+        }
+    } else {
+        /* the L bottom and L top planes of a bounded patch, x/y band excluded */
+        const unsigned j = idx - nxy;
+        const int b = int(j / inner), rem = int(j % inner);
+        k = b < L ? b : r.fnz - 2 * L + b;
+        xf = L + rem % (r.fnx - 2 * L);
+        yf = L + rem / (r.fnx - 2 * L);
+    }
+    const unsigned cf = unsigned(k) * unsigned(F.plane) + unsigned(yf) * unsigned(F.pitch) + unsigned(xf);
+    const int t = mask_f[cf] & TYPE_MASK;
+    const bool on = nidx < nodes && t != WALL && t != BODY;
+    const float xr = xf * r.lrfactor + r.lrfactor * 0.5f, yr = yf * r.lrfactor + r.lrfactor * 0.5f;
+    const int xm = int(xr), ym = int(yr);
+    const float fx = xr - xm, fy = yr - ym;
+    /* z: periodic full-depth patch (fine plane k at coarse z k / L - 1 +
+     * ...), or, bounded, as x and y from the coarse plane cz0 */
+    int zb;
+    float fz;
+    if (r.zbounded) {
+        const float zr = k * r.lrfactor + r.lrfactor * 0.5f;
+        zb = r.cz0 + int(zr);
+        fz = zr - int(zr);
+    } else {
+        zb = k / L - 1;
+        fz = (k % L) * r.lrfactor + r.lrfactor * 0.5f;
+    }
+    const unsigned ne = unsigned(r.enx) * r.eny * r.cnz;
+    /* trilinear moments and the second-order terms, one corner at a time; the
+     * corner's x bit is this lane's */
+    constexpr int N = FILL == (FILL_END | FILL_MID) ? 2 : 1;
+    float mom[N][9], a[N][9];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int m = 0; m < 9; ++m) mom[i][m] = a[i][m] = 0.f;
+#pragma unroll
+    for (int cyz = 0; cyz < 4; ++cyz) {
+        const int c = 2 * cyz + half;
+        int zc = zb + ((c >> 2) & 1);
+        zc = zc < 0 ? zc + r.cnz : (zc >= r.cnz ? zc - r.cnz : zc);
+        const unsigned ce = (unsigned(zc) * r.eny + (ym + ((c >> 1) & 1))) * r.enx + (xm + half);
+        float mc[N][9];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) mc[0][m] = __ldg(mom_c + m * ne + ce);
+        if constexpr ((FILL & FILL_MID) != 0) {
+#pragma unroll
+            for (int m = 0; m < 9; ++m) mc[N - 1][m] = (1.f - theta) * __ldg(mom_prev + m * ne + ce) + theta * mc[0][m];
+        }
+        const float wx = half ? fx : 1.f - fx, wy = (c & 2) ? fy : 1.f - fy, wz = (c & 4) ? fz : 1.f - fz;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+#pragma unroll
+            for (int m = 0; m < 9; ++m) mom[i][m] += mc[i][m] * wx * wy * wz;
+            if (r.order == 2) {
+                float Sc[6];
+                strain_rate<float>(mc[i], Sc);
+                second_order_add(a[i], c, mc[i], Sc);
+            }
+        }
+    }
+    /* lane 0 takes fill 0 (and fill N - 1 is lane 1's) */
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+        const float gm = __shfl_xor_sync(0xffffffffu, half ? mom[0][m] : mom[N - 1][m], 1);
+        const float ga = __shfl_xor_sync(0xffffffffu, half ? a[0][m] : a[N - 1][m], 1);
+        mom[0][m] = (half ? mom[N - 1][m] : mom[0][m]) + gm;
+        a[0][m] = (half ? a[N - 1][m] : a[0][m]) + ga;
+    }
+    if (!on || (N == 1 && half)) return;
+    S* const f_f = (FILL & FILL_MID) && (N == 1 || half) ? f_mid : f_end;
+    interp_cf_store<S>(r, F, mom[0], a[0], fx, fy, fz, f_f, cf);
 }
 
 /* the coarse nodes strictly inside the patch that the restriction replaces:
@@ -461,15 +497,24 @@ struct FcBox {
 };
 
 /* InterpFC (LR7:2172-2348): coarse nodes strictly inside the patch (2-node
- * margin) are replaced by the restriction of their 8 fine children. */
+ * margin) are replaced by the restriction of their 8 fine children.  Two lanes
+ * per node, one for the four children at lower x and one for the upper
+ * (adjacent lanes then read adjacent fine nodes), which exchange their sums;
+ * the first finishes: 8.5 us for 35,000 nodes, 12.7 us with one lane each. */
 template <class S>
-__device__ __forceinline__ void interp_fc_node(const RefineParams& r, const Level& C, const Level& F,
-                                               const S* __restrict__ f_f, S* __restrict__ f_c,
-                                               const uint8_t* __restrict__ mask_c, const int x, const int y,
-                                               const int z) {
+__global__ void __launch_bounds__(IFACE_THREADS) k_interp_fc(const RefineParams r, const Level C, const Level F,
+                                                             const S* __restrict__ f_f, S* __restrict__ f_c,
+                                                             const uint8_t* __restrict__ mask_c, const FcBox b) {
+    pdl_wait();
+    const long long nidx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 1;
+    const int half = threadIdx.x & 1;
+    const int per_plane = b.nxi * b.nyi;
+    const long long nodes = (long long)per_plane * b.nzi, i = nidx < nodes ? nidx : nodes - 1;
+    const int zi = int(i / per_plane), rem = int(i - (long long)zi * per_plane);
+    const int x = b.x0 + rem % b.nxi, y = b.y0 + rem / b.nxi, z = b.z0 + zi;
     const long long cc = z * C.plane + (long long)y * C.pitch + x;
     const int t = mask_c[cc] & TYPE_MASK;
-    if (t == WALL || t == BODY) return;
+    const bool on = nidx < nodes && t != WALL && t != BODY;
     const int L = r.lrlevel;
     const int xm = int(L * (x - r.lrx0)), ym = int(L * (y - r.lry0));
     int kl = int(L * (z - r.lrz0)), kh = kl + 1;
@@ -483,14 +528,15 @@ __device__ __forceinline__ void interp_fc_node(const RefineParams& r, const Leve
         k1 = kl;
     }
     /* the children's mean moments and the second-order terms, one child at
-     * a time */
+     * a time; the child's x bit is this lane's */
     float sum[9], a[9];
 #pragma unroll
     for (int m = 0; m < 9; ++m) sum[m] = a[m] = 0.f;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
+    for (int cyz = 0; cyz < 4; ++cyz) {
+        const int c = 2 * cyz + half;
         const int kk = (c & 4) ? k1 : k0;
-        const long long cf = kk * F.plane + (long long)(ym + ((c >> 1) & 1)) * F.pitch + (xm + (c & 1));
+        const long long cf = kk * F.plane + (long long)(ym + ((c >> 1) & 1)) * F.pitch + (xm + half);
         float g[19], mc[9], Sc[6];
         load19<S>(F, f_f, cf, g);
         physical_moments<float>(g, mc);
@@ -501,6 +547,12 @@ __device__ __forceinline__ void interp_fc_node(const RefineParams& r, const Leve
             second_order_add(a, c, mc, Sc);
         }
     }
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+        sum[m] += __shfl_xor_sync(0xffffffffu, sum[m], 1);
+        a[m] += __shfl_xor_sync(0xffffffffu, a[m], 1);
+    }
+    if (!on || half) return;
     float mom[9];
 #pragma unroll
     for (int m = 0; m < 9; ++m) mom[m] = 0.125f * sum[m];
@@ -525,38 +577,6 @@ __device__ __forceinline__ void interp_fc_node(const RefineParams& r, const Leve
     invert_scaled<float>(mom, SF, g);
 #pragma unroll
     for (int q = 0; q < 19; ++q) Fmt<S>::st(f_c + pidx(C, q, unsigned(cc)), g[q], C.off[q]);
-}
-
-template <class S>
-__global__ void k_interp_fc(const RefineParams r, const Level C, const Level F, const S* __restrict__ f_f,
-                            S* __restrict__ f_c, const uint8_t* __restrict__ mask_c, const FcBox b) {
-    const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y * blockDim.y + threadIdx.y;
-    if (xi >= b.nxi || yi >= b.nyi) return;
-    interp_fc_node<S>(r, C, F, f_f, f_c, mask_c, b.x0 + xi, b.y0 + yi, b.z0 + int(blockIdx.z));
-}
-
-/* the final band fill of a coarse step and the restriction in one launch:
- * they touch disjoint nodes (the band, and the coarse nodes over the
- * patch's interior with its 2-node margin), so the first cf_blocks blocks
- * fill the band and the others restrict, one coarse node per thread */
-constexpr int IFACE_THREADS = 128;
-template <class S>
-__global__ void __launch_bounds__(IFACE_THREADS) k_interface(const RefineParams r, const Level C, const Level F,
-                                                             const float* __restrict__ mom_c, S* __restrict__ f_f,
-                                                             const uint8_t* __restrict__ mask_f, S* __restrict__ f_c,
-                                                             const uint8_t* __restrict__ mask_c, const FcBox b,
-                                                             int cf_blocks) {
-    pdl_wait();
-    if (int(blockIdx.x) < cf_blocks) {
-        interp_cf_node<S>(r, F, mom_c, nullptr, 1.f, f_f, mask_f,
-                          (long long)blockIdx.x * IFACE_THREADS + threadIdx.x);
-        return;
-    }
-    const long long i = (long long)(blockIdx.x - cf_blocks) * IFACE_THREADS + threadIdx.x;
-    const long long per_plane = (long long)b.nxi * b.nyi;
-    if (i >= per_plane * b.nzi) return;
-    const int zi = int(i / per_plane), rem = int(i - zi * per_plane);
-    interp_fc_node<S>(r, C, F, f_f, f_c, mask_c, b.x0 + rem % b.nxi, b.y0 + rem / b.nxi, b.z0 + zi);
 }
 
 /* ---- launchers ---- */
@@ -619,6 +639,7 @@ cudaError_t launch_stream_collide(const Level& L, const StepParams& p, const voi
     StepParams q = p;
     q.tau0 = 1.f / p.omega;
     q.smag_k = 18.f * 1.41421356f * p.cs;
+    q.extras = p.stats_on || p.band;
     q.tau0_d = 1.0 / double(p.omega);
     q.smag_k_d = 18.0 * 1.4142135623730951 * double(p.cs);
     const int code = L.storage + (L.blocked ? 8 : 0);
@@ -820,13 +841,16 @@ cudaError_t launch_audit(const Level& L, const void* f, const uint8_t* mask, dou
     return cudaGetLastError();
 }
 
-cudaError_t launch_interp_cf(const RefineParams& r, const Level& F, const float* mom_c, void* f_f,
-                             const uint8_t* mask_f, cudaStream_t s, const float* mom_prev, float theta) {
-    const long long n = cf_nodes(r);
-    const int threads = 128;
-    const unsigned blocks = unsigned((n + threads - 1) / threads);
-    LBM_DISPATCH(F.storage,
-                 return launch_pdl(k_interp_cf<S>, blocks, threads, s, r, F, mom_c, mom_prev, theta, (S*)f_f, mask_f));
+cudaError_t launch_interp_cf(const RefineParams& r, const Level& F, const float* mom_c, const float* mom_prev,
+                             float theta, void* f_end, void* f_mid, const uint8_t* mask_f, cudaStream_t s) {
+    const unsigned threads = IFACE_THREADS, blocks = unsigned((2 * cf_nodes(r) + threads - 1) / threads);
+#define LBM_FILL(N) \
+    LBM_DISPATCH(F.storage, return launch_pdl(k_interp_cf<S, N>, blocks, threads, s, r, F, mom_c, mom_prev, theta, \
+                                              (S*)f_end, (S*)f_mid, mask_f))
+    if (f_end && f_mid) LBM_FILL(FILL_END | FILL_MID);
+    if (f_end) LBM_FILL(FILL_END);
+    if (f_mid) LBM_FILL(FILL_MID);
+#undef LBM_FILL
     return cudaErrorInvalidValue;
 }
 
@@ -863,20 +887,8 @@ cudaError_t launch_interp_fc(const RefineParams& r, const Level& C, const Level&
                              const uint8_t* mask_c, cudaStream_t s) {
     const FcBox b = fc_box(r, C);
     if (b.nxi == 0) return cudaSuccess;
-    const dim3 block(32, 4), grid((b.nxi + 31) / 32, (b.nyi + 3) / 4, b.nzi);
-    LBM_DISPATCH(C.storage, (k_interp_fc<S><<<grid, block, 0, s>>>(r, C, F, (const S*)f_f, (S*)f_c, mask_c, b)));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_interface(const RefineParams& r, const Level& C, const Level& F, const float* mom_c, void* f_f,
-                             const uint8_t* mask_f, void* f_c, const uint8_t* mask_c, cudaStream_t s) {
-    if (C.storage != F.storage) return cudaErrorInvalidValue;
-    const FcBox b = fc_box(r, C);
-    const int cf_blocks = int((cf_nodes(r) + IFACE_THREADS - 1) / IFACE_THREADS);
-    const long long nfc = (long long)b.nxi * b.nyi * b.nzi;
-    const unsigned blocks = unsigned(cf_blocks + (nfc + IFACE_THREADS - 1) / IFACE_THREADS);
-    LBM_DISPATCH(C.storage, return launch_pdl(k_interface<S>, blocks, IFACE_THREADS, s, r, C, F, mom_c, (S*)f_f, mask_f,
-                                              (S*)f_c, mask_c, b, cf_blocks));
+    const unsigned threads = IFACE_THREADS, blocks = unsigned((2LL * b.nxi * b.nyi * b.nzi + threads - 1) / threads);
+    LBM_DISPATCH(C.storage, return launch_pdl(k_interp_fc<S>, blocks, threads, s, r, C, F, (const S*)f_f, (S*)f_c, mask_c, b));
     return cudaErrorInvalidValue;
 }
 

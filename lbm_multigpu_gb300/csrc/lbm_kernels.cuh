@@ -144,6 +144,10 @@ struct StepParams {
      * beside them (211 x 70 x 45 channel: 26 instead of 21 us a step) */
     int early;
     const int* step_dev;   /* when non-null, t counts from the device's step counter */
+    /* refinement: the outermost band layers of non-solid nodes (in x and y,
+     * with band_z in z) are not stored, the band fill writes them */
+    int band, band_z;
+    int extras; /* derived by launch_stream_collide: stats_on or band */
     int stats_on, start_av, start_fluc;
     float stats_weight;
     float noise_amp;
@@ -294,17 +298,13 @@ struct RefineParams {
     int zbounded, cz0;
 };
 
-/* mom_prev: the previous coarse export, blended in time with weight theta
- * on mom_c (linear temporal interpolation); null: mom_c alone */
-cudaError_t launch_interp_cf(const RefineParams& r, const Level& F, const float* mom_c, void* f_f,
-                             const uint8_t* mask_f, cudaStream_t s, const float* mom_prev = nullptr,
-                             float theta = 1.f);
+/* the band fill of f_end from the coarse export mom_c and / or of f_mid from
+ * the exports blended in time, (1 - theta) mom_prev + theta mom_c (a null
+ * buffer is not filled) */
+cudaError_t launch_interp_cf(const RefineParams& r, const Level& F, const float* mom_c, const float* mom_prev,
+                             float theta, void* f_end, void* f_mid, const uint8_t* mask_f, cudaStream_t s);
 cudaError_t launch_interp_fc(const RefineParams& r, const Level& C, const Level& F, const void* f_f, void* f_c,
                              const uint8_t* mask_c, cudaStream_t s);
-/* the final band fill of a coarse step (from mom_c alone) and the
- * restriction in one launch (they touch disjoint nodes) */
-cudaError_t launch_interface(const RefineParams& r, const Level& C, const Level& F, const float* mom_c, void* f_f,
-                             const uint8_t* mask_f, void* f_c, const uint8_t* mask_c, cudaStream_t s);
 
 /* learned subgrid closure (sgs_mlp.cu) */
 int mlp_grad_blocks(int n);

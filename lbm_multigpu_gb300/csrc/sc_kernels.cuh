@@ -222,6 +222,12 @@ __device__ __forceinline__ void sc_stats(const StepParams& p, float* __restrict_
     }
 }
 
+/* whether the refinement's band fill writes this node */
+__device__ __forceinline__ bool sc_in_band(const Level& L, const StepParams& p, int x, int y, int z) {
+    const int b = p.band;
+    return b && (x < b || x >= L.nx - b || y < b || y >= L.ny - b || (p.band_z && (z < b || z >= L.nz - b)));
+}
+
 /* the collision, statistics, store and moment export of a non-solid node;
  * f holds populations, or for DEV their stored deviations.  With DEVMRT an
  * inlet's or outlet's rebuild (bc, uin; FLUID otherwise) is part of the
@@ -259,15 +265,18 @@ __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParam
             for (int q = 0; q < 19; ++q) f[q] -= L.off[q];
         }
     }
-    if (p.stats_on) {
-        T u = 0, v = 0;
+    if (p.extras) {
+        if (p.stats_on) {
+            T u = 0, v = 0;
 #pragma unroll
-        for (int q = 0; q < 19; ++q) {
-            const T g = DEV ? f[q] + L.off[q] : f[q];
-            if (cx(q)) u += T(cx(q)) * g;
-            if (cy(q)) v += T(cy(q)) * g;
+            for (int q = 0; q < 19; ++q) {
+                const T g = DEV ? f[q] + L.off[q] : f[q];
+                if (cx(q)) u += T(cx(q)) * g;
+                if (cy(q)) v += T(cy(q)) * g;
+            }
+            sc_stats(p, stats, qs, c, float(u), float(v));
         }
-        sc_stats(p, stats, qs, c, float(u), float(v));
+        if (sc_in_band(L, p, x, y, z)) return;
     }
     store19<S, LAY, DEV>(L, fB, n, f);
 }

@@ -177,6 +177,31 @@ def test_z_bounded_patch_vs_oracle(product, cf_time):
 
 
 @pytest.mark.parametrize("cf_time", ["none", "linear"])
+def test_patch_of_ratio_4_vs_oracle(product, cf_time):
+    """four fine sub-steps per coarse step: the band filled before each of the
+    middle ones and, with the end of the coarse step, before the last"""
+    lbm = product
+    steps = 12
+    text = lbm.make_inputs(64, 24, 12, obst1=(20.5, 11.5, 0.0), r1=2.0, re=30.0, umax=0.05, tmax=steps, les=1,
+                           cs=0.01, refinement=1, lr_dims=(48, 40, 24), lr_factor=0.25, lr_origin=(15.125, 6.125, 2.125),
+                           geometry="channel_square", cf_time=cf_time)
+    with lbm.Solver(text) as s:
+        s.step(steps)
+        fc, ff, mc, mf, pr = s.populations(0), s.populations(1), s.mask(0), s.mask(1), s.params()
+    assert np.isfinite(ff).all()
+    r = Refine(cnx=64, cny=24, cnz=12, fnx=48, fny=40, fnz=24, lrx0=15.125, lry0=6.125, lrz0=2.125, lrfactor=0.25,
+               lrlevel=4, order=2, cs=0.01, omega_c=pr["omega"], omega_f=pr["omega_lr"], quirk_fc_top_zflip=1,
+               zbounded=1, cz0=2)
+    o = OracleRun(64, 24, 12, mc, pr["omega"], les=1, cs=0.01, refine=dict(r=r, mask=mf, omega_f=pr["omega_lr"]),
+                  cf_time=cf_time == "linear")
+    o.step(steps)
+    assert _compare(fc, o.fa, mc)[0] < RTOL
+    _, jf = moments(ff)
+    _, jo = moments(o.ffa)
+    assert rel_l2(jf[:, mf != 2], jo[:, mf != 2]) < RTOL
+
+
+@pytest.mark.parametrize("cf_time", ["none", "linear"])
 def test_refinement_step_graphs_are_bit_exact(product, cf_time):
     """lbm_step captures refinement steps in batches into CUDA graphs; one
     call of n steps (one direct step, then batches of 16, 16 and 7 replayed
