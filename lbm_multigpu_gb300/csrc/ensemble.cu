@@ -64,12 +64,13 @@ __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float
 }
 
 /* The step with the learned closure, as k_stream_collide_mlp: tiles of 32 x 4
- * (one M = 128 MMA per layer), persistent blocks, and the projected MRT
- * collision, of which only rho, j and the five stresses stay live across the
- * tensor-core round trips.  Eight boxes of sides 32 to 80 (1.8 M nodes): 87 us
- * with 7 blocks per SM and just their shared memory taken from L1 (4, 5, 6, 8
- * blocks: 102, 93, 90, 100 us; one block of 256 rows per SM, what the
- * occupancy API made of kernels with TMEM: 188 us). */
+ * (one M = 128 MMA per layer) and persistent blocks; the populations stay in
+ * registers across the tensor-core round trips.  Eight boxes of sides 32 to 80
+ * (1.8 M nodes): about 100 us with 7 blocks per SM and just their shared
+ * memory taken from L1 (one block of 256 rows per SM, what the occupancy API
+ * made of kernels with TMEM: 188 us).  The features are rounded to BF16, so
+ * the order of operations that leads to them is part of the result: the
+ * projected collision (87 us) moves the fields of 50 steps by 1e-5. */
 constexpr int MLP_TY = 4, MLP_ROWS = 32 * MLP_TY, MLP_BLOCKS = 7;
 __global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS) k_ens_step_mlp(const Table T, const float* __restrict__ fA,
                                                                        float* __restrict__ fB,
@@ -101,25 +102,17 @@ __global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS) k_ens_step_mlp(const Tab
 #pragma unroll
             for (int q = 0; q < 19; ++q) f[q] = wq(q);
         }
-        const MrtDev<float> mo = mrt_dev_moments<float>(f, 0.f);
-        float p6[6], xf[sgs::NIN];
-        mrt_dev_pi(mo, p6);
-        const float sc = -1.5f / mo.rho;
+        float rho, p6[6], xf[sgs::NIN];
+        pi_neq<float>(f, rho, p6);
+        const float sc = -1.5f / rho;
 #pragma unroll
         for (int k = 0; k < 6; ++k) p6[k] *= sc;
         sgs::features_fast(p6, M.tau0, M.omega, xf); /* omega = 1 / tau0 */
-        float keep[10] = {mo.rho, mo.jx, mo.jy, mo.jz, mo.n9, mo.n11, mo.n13, mo.n14, mo.n15,
-                          sgs::strain_gain(xf, M.omega)};
+        const float gain = sgs::strain_gain(xf, M.omega);
         const float o = sgs::infer_nu<MLP_ROWS>(sm, xf, err);
         if (o < 0.f) break; /* a tensor-core wait ran out (block-uniform) */
         if (!live) continue;
-#pragma unroll
-        for (int k = 0; k < 10; ++k) asm volatile("" : "+f"(keep[k]));
-        MrtDev<float> mr;
-        mr.rho = keep[0], mr.jx = keep[1], mr.jy = keep[2], mr.jz = keep[3], mr.n9 = keep[4], mr.n11 = keep[5];
-        mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8];
-        mrt_dev_complete(mr, 0.f);
-        mrt_dev_relax(f, mr, 1.f / (M.tau0 + 3.f * o * keep[9]));
+        collide_mrt<MRT>(f, 1.f / (M.tau0 + 3.f * o * gain), false, 0.f, 0.f);
         float* b = fB + M.off + c;
 #pragma unroll
         for (int q = 0; q < 19; ++q) b[q * qs] = f[q];

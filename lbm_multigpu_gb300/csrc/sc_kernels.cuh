@@ -170,13 +170,15 @@ __device__ __forceinline__ void store19(const Level& L, S* __restrict__ f, const
  * the node types present, so a channel kernel carries no lid code (whose
  * 19-entry temporaries would otherwise set every variant's register count) */
 constexpr int FEAT_HALFWAY = 1, FEAT_LID = 2, FEAT_CLAMP = 4, FEAT_XBC = 8;
-/* LR7's MRT model (which takes no body force): the projected collision
- * collide_mrt_dev only, on the stored deviations of FP16 / BF16 (the other
- * models convert those to populations and back) and on the populations of
- * FP64, whose bound is the FP64 pipe (1.05 M nodes: 0.54 ms through
- * collide_mrt, 0.30 ms so).  Not FP32, whose kernels are bound by memory */
+/* LR7's MRT model (which takes no body force): the projected collision only,
+ * on the stored deviations of FP16 / BF16 (collide_mrt_dev; the other models
+ * convert those to populations and back) and on populations
+ * (collide_mrt_pop): FP64, whose bound is the FP64 pipe (1.05 M nodes: 0.54 ms
+ * through collide_mrt, 0.30 ms so), and FP32 (48 registers instead of 56:
+ * level on the 512 x 128 x 128 channel, which HBM bounds, 21.88 -> 21.74 ms
+ * for 100 steps; where a step is two or three waves of blocks the latency
+ * counts: 4 % on a ragged channel of 0.7 M nodes, 2 % on a refined one) */
 constexpr int FEAT_DEVMRT = 16;
-template <class S> __host__ __device__ constexpr bool sc_has_devmrt() { return sizeof(S) != 4; }
 /* the relaxation time of each node from the learned closure's last refresh
  * (StepParams::nu) instead of the LES setting */
 constexpr int FEAT_NUBUF = 32;
@@ -229,10 +231,10 @@ __device__ __forceinline__ bool sc_in_band(const Level& L, const StepParams& p, 
 }
 
 /* the collision, statistics, store and moment export of a non-solid node;
- * f holds populations, or for DEV their stored deviations.  With DEVMRT an
- * inlet's or outlet's rebuild (bc, uin; FLUID otherwise) is part of the
- * collision: it only replaces the density or the momentum, which the
- * projected collision has by then, and f is its neighbour's as stored */
+ * f holds populations, or for DEV their stored deviations.  With DEVMRT on
+ * populations an inlet's or outlet's rebuild (bc, uin; FLUID otherwise) is
+ * part of the collision: it only replaces the density or the momentum, which
+ * the projected collision has by then, and f is its neighbour's as stored */
 template <class S, int LAY, bool DEVMRT, bool NUBUF>
 __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParams& p, S* __restrict__ fB,
                                                  float* __restrict__ stats, float* __restrict__ mom_export,
@@ -247,10 +249,12 @@ __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParam
     const float om = NUBUF ? 1.f / (p.tau0 + 3.f * p.nu[c]) : p.omega;
     const bool les = !NUBUF && p.les != 0;
     if constexpr (DEVMRT) {
-        if constexpr (sizeof(T) == 8)
-            collide_mrt_dev<T>(f, T(om), les, p.tau0_d, p.smag_k_d, T(0), bc, T(p.rho_out), uin, T(0));
+        if constexpr (DEV)
+            collide_mrt_dev<T>(f, T(om), les, T(p.tau0), T(p.smag_k), T(L.u_ref));
+        else if constexpr (sizeof(T) == 8)
+            collide_mrt_pop<T>(f, T(om), les, p.tau0_d, p.smag_k_d, bc, T(p.rho_out), uin);
         else
-            collide_mrt_dev<T>(f, T(om), les, T(p.tau0), T(p.smag_k), T(L.u_ref), bc, T(p.rho_out), uin, T(1));
+            collide_mrt_pop<T>(f, T(om), les, p.tau0, p.smag_k, bc, T(p.rho_out), uin);
     } else {
         T dp = T(p.dpdy_dev ? *p.dpdy_dev : p.dpdy);
         if (y > p.dyn_y1) dp = T(0);
@@ -258,8 +262,7 @@ __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParam
 #pragma unroll
             for (int q = 0; q < 19; ++q) f[q] += L.off[q];
         }
-        if constexpr (sc_has_devmrt<S>()) collide_other<T>(p.model, f, T(om), les, T(p.cs), dp);
-        else collide<T>(p.model, f, T(om), les, T(p.cs), dp);
+        collide_other<T>(p.model, f, T(om), les, T(p.cs), dp);
         if (DEV) {
 #pragma unroll
             for (int q = 0; q < 19; ++q) f[q] -= L.off[q];
@@ -393,16 +396,14 @@ __device__ __forceinline__ void sc_finish(const Level& L, const StepParams& p, c
             /* rebuild from the neighbour's stored post-collision state */
             const unsigned cn = type == WEST_INLET ? c - x + xp : type == EAST_OUTLET ? c - x + xm
                               : type == SOUTH_INLET ? c + (yp - y) * pitch : c + (ym - y) * pitch;
-            constexpr bool RAW = DEV && (FEAT & FEAT_DEVMRT);
 #pragma unroll
-            for (int q = 0; q < 19; ++q)
-                f[q] = RAW ? T(F::ldr(n.at(fA, q, cn))) : F::ld(n.at(fA, q, cn), L.off[q]);
+            for (int q = 0; q < 19; ++q) f[q] = F::ld(n.at(fA, q, cn), L.off[q]);
             if (p.noise_amp != 0.f) {
                 const uint32_t cell = uint32_t((z * L.ny + y) * L.nx + x);
                 const float xi = philox_uniform(p.noise_seed, cell, uint32_t(sc_time(p)));
                 uin = uin + T(p.u_in) * T(p.noise_amp) * (T(2) * T(xi) - T(1));
             }
-            if constexpr ((FEAT & FEAT_DEVMRT) != 0) {
+            if constexpr (!DEV && (FEAT & FEAT_DEVMRT) != 0) {
                 bc = type;
             } else {
                 extrap<T>(type, f, T(p.rho_out), uin);
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(SC_BX* SC_BY, sc_min_blocks<S, FEAT>()) k_stre
  * rows) unless L1 still holds it, and a block's operands take 27 KB of the
  * array that L1 shares with shared memory.  So the launch asks for exactly the
  * shared memory of its resident blocks (7: 196 of 228 KB).  512 x 128 x 128,
- * FP32: 316 us; with all of the array as shared memory 433 us, and 376 us with
+ * FP32: 316 us (40 steps with their start 16.3 ms); with all of the array as shared memory 433 us, and 376 us with
  * the network left out altogether; 4, 5, 6, 8 blocks per SM 370, 314, 362,
  * 478 us (FP16 408, 322, 353, 402 and with 7 313 us).  Copying the next
  * tile's pulls into shared memory with cp.async cost more L1 than it hid
@@ -556,11 +557,18 @@ __global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS)
             const unsigned zm = (z == 0) ? L.nz - 1 : z - 1, zp = (z == L.nz - 1) ? 0 : z + 1;
             const NodeIdx<LAY> ni(L, xm, unsigned(x), xp, ym, unsigned(y), yp, zm, unsigned(z), zp);
             if (type >= WEST_INLET && type <= NORTH_OUTLET) {
-                /* the neighbour's stored state; the rebuild is below */
+                /* rebuild from the neighbour's stored post-collision state */
                 const unsigned cn = type == WEST_INLET ? n.c - x + xp : type == EAST_OUTLET ? n.c - x + xm
                                   : type == SOUTH_INLET ? n.c + (yp - y) * pitch : n.c + (ym - y) * pitch;
 #pragma unroll
                 for (int q = 0; q < 19; ++q) f[q] = F::ld(ni.at(fA, q, cn), L.off[q]);
+                float uin = p.u_in;
+                if (p.noise_amp != 0.f) {
+                    const uint32_t cell = uint32_t((z * L.ny + y) * L.nx + x);
+                    const float xi = philox_uniform(p.noise_seed, cell, uint32_t(sc_time(p)));
+                    uin = uin + p.u_in * p.noise_amp * (2.f * xi - 1.f);
+                }
+                extrap<float>(type, f, p.rho_out, uin);
             } else {
 #pragma unroll
                 for (int q = 0; q < 19; ++q) f[q] = F::ld(ni.pull(fA, q), L.off[q]);
@@ -585,19 +593,8 @@ __global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS)
             store19<S, LAY, false>(L, fB, n, gb);
         }
         /* the closure for the whole tile; the collision's moments give
-         * Pi_neq (the projected MRT collision on full populations), and an
-         * inlet's or outlet's rebuild is a change of them */
-        MrtDev<float> mo = mrt_dev_sums<float>(f);
-        if (type >= WEST_INLET && type <= NORTH_OUTLET) {
-            float uin = p.u_in;
-            if (p.noise_amp != 0.f) {
-                const uint32_t cell = uint32_t((t.z * L.ny + y) * L.nx + x);
-                const float xi = philox_uniform(p.noise_seed, cell, uint32_t(sc_time(p)));
-                uin = uin + p.u_in * p.noise_amp * (2.f * xi - 1.f);
-            }
-            mrt_dev_extrap(mo, type, p.rho_out, uin, 0.f, 0.f);
-        }
-        mrt_dev_finish(mo, 0.f);
+         * Pi_neq (the projected MRT collision on full populations) */
+        const MrtDev<float> mo = mrt_dev_moments<float>(f, 0.f);
         float p6[6], xf[sgs::NIN];
         mrt_dev_pi(mo, p6);
         const float sc = -1.5f / mo.rho;
@@ -619,7 +616,7 @@ __global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS)
         if (p.nu) p.nu[n.c] = nu;
         MrtDev<float> mr;
         mr.rho = keep[0], mr.jx = keep[1], mr.jy = keep[2], mr.jz = keep[3], mr.n9 = keep[4], mr.n11 = keep[5];
-        mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8];
+        mr.n13 = keep[6], mr.n14 = keep[7], mr.n15 = keep[8], mr.n1 = 0.f;
         mrt_dev_complete(mr, 0.f);
         mrt_dev_relax(f, mr, 1.f / (tau0 + 3.f * nu));
         if (p.stats_on) {
@@ -639,7 +636,6 @@ __global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS)
 
 /* whether launch_sc_t has a kernel of these features */
 template <class S> inline bool sc_feat_built(int feat) {
-    if (!sc_has_devmrt<S>() && (feat & FEAT_DEVMRT)) return false;
     if (feat & FEAT_NUBUF) return sizeof(S) <= 4 && !(feat & (FEAT_LID | FEAT_CLAMP | FEAT_XBC));
     return feat >= 0 && feat < 32;
 }
@@ -650,7 +646,8 @@ inline cudaError_t launch_sc_t(const Level& L, const StepParams& p, const void* 
                                float* stats, float* mom_export, cudaStream_t s, const uint32_t* links) {
     const dim3 block(SC_BX, SC_BY), grid(L.pitch / SC_BX, (L.ny + SC_BY - 1) / SC_BY, L.nz);
     const int feat = (p.halfway ? FEAT_HALFWAY : 0) | (p.has_lid ? FEAT_LID : 0) | (p.pull_clamp ? FEAT_CLAMP : 0) |
-                     (p.has_xbc ? FEAT_XBC : 0) | (sc_has_devmrt<S>() && p.model == MRT ? FEAT_DEVMRT : 0) | (p.nu_reuse ? FEAT_NUBUF : 0);
+                     (p.has_xbc ? FEAT_XBC : 0) | (p.model == MRT ? FEAT_DEVMRT : 0) |
+                     (p.nu_reuse ? FEAT_NUBUF : 0);
     if (!sc_feat_built<S>(feat)) return cudaErrorInvalidValue;
 #define LBM_SC(FT)                                                                                            \
     case FT:                                                                                                  \
@@ -661,19 +658,12 @@ inline cudaError_t launch_sc_t(const Level& L, const StepParams& p, const void* 
          * without and with the projected MRT */
         LBM_SC(0) LBM_SC(1) LBM_SC(2) LBM_SC(3) LBM_SC(4) LBM_SC(5) LBM_SC(6) LBM_SC(7)
         LBM_SC(8) LBM_SC(9) LBM_SC(10) LBM_SC(11) LBM_SC(12) LBM_SC(13) LBM_SC(14) LBM_SC(15)
+        LBM_SC(16) LBM_SC(17) LBM_SC(18) LBM_SC(19) LBM_SC(20) LBM_SC(21) LBM_SC(22) LBM_SC(23)
+        LBM_SC(24) LBM_SC(25) LBM_SC(26) LBM_SC(27) LBM_SC(28) LBM_SC(29) LBM_SC(30) LBM_SC(31)
         default:
-            if constexpr (sc_has_devmrt<S>()) {
-                switch (feat) {
-                    LBM_SC(16) LBM_SC(17) LBM_SC(18) LBM_SC(19) LBM_SC(20) LBM_SC(21) LBM_SC(22) LBM_SC(23)
-                    LBM_SC(24) LBM_SC(25) LBM_SC(26) LBM_SC(27) LBM_SC(28) LBM_SC(29) LBM_SC(30) LBM_SC(31)
-                    default: break;
-                }
-            }
             /* the steps between refreshes of the learned closure (channels:
              * no lid, no alternate boundaries, no clamped pulls; not FP64) */
-            if constexpr (sizeof(S) == 4) {
-                switch (feat) { LBM_SC(32) LBM_SC(33) default: break; }
-            } else if constexpr (sizeof(S) == 2) {
+            if constexpr (sizeof(S) <= 4) {
                 switch (feat) { LBM_SC(32) LBM_SC(33) LBM_SC(48) LBM_SC(49) default: break; }
             }
     }

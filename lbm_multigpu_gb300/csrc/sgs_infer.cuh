@@ -268,7 +268,7 @@ template <int ROWS> __device__ __forceinline__ float infer_nu(InferSmem<ROWS>& s
     ok = infer_mma_wait(s, ph ^ 1u) && ok;
     /* output layer: y = b3 + w3 . relu(z2) in FP32, from the layer-2
      * accumulators (two completions per call: parities ph, ph ^ 1) */
-    float2 y2 = make_float2(s.b3, 0.f);
+    float y = s.b3;
     const uint32_t w3 = tc::smem_u32(s.w3f);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -279,13 +279,12 @@ template <int ROWS> __device__ __forceinline__ float infer_nu(InferSmem<ROWS>& s
 #pragma unroll
         for (int j = 0; j < 16; j += 4) {
             const float4 w = tc::lds128f(w3 + 4 * (16 * c + j));
-            y2 = __ffma2_rn(make_float2(w.x, w.y), make_float2(fmaxf(__uint_as_float(r[j]), 0.f),
-                                                               fmaxf(__uint_as_float(r[j + 1]), 0.f)), y2);
-            y2 = __ffma2_rn(make_float2(w.z, w.w), make_float2(fmaxf(__uint_as_float(r[j + 2]), 0.f),
-                                                               fmaxf(__uint_as_float(r[j + 3]), 0.f)), y2);
+            y = fmaf(w.x, fmaxf(__uint_as_float(r[j]), 0.f), y);
+            y = fmaf(w.y, fmaxf(__uint_as_float(r[j + 1]), 0.f), y);
+            y = fmaf(w.z, fmaxf(__uint_as_float(r[j + 2]), 0.f), y);
+            y = fmaf(w.w, fmaxf(__uint_as_float(r[j + 3]), 0.f), y);
         }
     }
-    const float y = y2.x + y2.y;
     /* two completions per call leave the parity of the next one at ph */
     if (!ok) {
         if ((t & 31) == 0) atomicExch(err, 2);

@@ -40,24 +40,23 @@ void cell_collide_mrt_dev(int les, float omega, float cs, float u, float* h, int
     const float k = 18.f * 1.41421356f * cs;
     for (int i = 0; i < n; ++i) collide_mrt_dev<float>(h + 19L * i, omega, les != 0, 1.f / omega, k, u);
 }
+/* n steps of one uniform node's FP32 populations: streaming leaves them alone */
+void cell_iterate_mrt_pop(float omega, float cs, float* f, int steps) {
+    const float k = 18.f * 1.41421356f * cs;
+    for (int i = 0; i < steps; ++i) collide_mrt_pop<float>(f, omega, true, 1.f / omega, k);
+}
 void cell_pi_neq_d(const double* f, double* rho, double* p6, int n) {
     for (int i = 0; i < n; ++i) pi_neq<double>(f + 19L * i, rho[i], p6 + 6L * i);
 }
-/* an inlet / outlet rebuild of h + off and the projected collision of it: as part
- * of the collision (fused) or extrap first; U = u */
-void cell_collide_mrt_dev_bc_d(int fused, int type, double omega, double cs, double u, double rho_bc, double u_in,
-                               const double* off, double* h, int n) {
+/* the projected collision of populations, of an inlet's or outlet's (type)
+ * with the rebuild as part of it (fused) or extrap first */
+void cell_collide_mrt_pop_d(int fused, int type, int les, double omega, double cs, double rho_bc, double u_in, double* h,
+                            int n) {
     const double k = 18.0 * 1.4142135623730951 * cs;
     for (int i = 0; i < n; ++i) {
         double* f = h + 19L * i;
-        if (fused) {
-            collide_mrt_dev<double>(f, omega, true, 1.0 / omega, k, u, type, rho_bc, u_in, 1.0);
-        } else {
-            for (int q = 0; q < 19; ++q) f[q] += off[q];
-            extrap<double>(type, f, rho_bc, u_in);
-            for (int q = 0; q < 19; ++q) f[q] -= off[q];
-            collide_mrt_dev<double>(f, omega, true, 1.0 / omega, k, u);
-        }
+        if (!fused && type != FLUID) extrap<double>(type, f, rho_bc, u_in);
+        collide_mrt_pop<double>(f, omega, les != 0, 1.0 / omega, k, fused ? type : int(FLUID), rho_bc, u_in);
     }
 }
 void cell_mrt_dev_pi_d(const double* f, double* rho, double* p6, int n) {

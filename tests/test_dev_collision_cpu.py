@@ -102,17 +102,15 @@ def test_projected_collision_on_full_populations(cellops, les):
 
 
 @pytest.mark.parametrize("type_", [3, 4, 5, 6])  # west inlet, east outlet, south inlet, north outlet
-@pytest.mark.parametrize("u", [0.0, 0.05])
-def test_rebuild_within_the_projected_collision(cellops, type_, u):
+def test_rebuild_within_the_projected_collision(cellops, type_):
     """the inlet / outlet rebuild as a change of the collision's moments
     equals the rebuild of the populations before the collision"""
-    off = _model_eq(cellops, u)
-    _, h = _states(off, 200, 20 + type_, 0.01)
-    g = h.copy()
-    args = [ctypes.c_double(v) for v in (1 / 0.52, 0.01, u, 1.003, 0.047)]
-    for fused, a in ((0, h), (1, g)):
-        cellops.cell_collide_mrt_dev_bc_d(fused, type_, *args, _ptr(off), _ptr(a), len(a))
-    np.testing.assert_allclose(g, h, rtol=0, atol=1e-14)  # FP64 rounding of sums of 19 terms below 1
+    f, _ = _states(np.zeros(19), 200, 20 + type_, 0.01)
+    g = f.copy()
+    args = [ctypes.c_double(v) for v in (1 / 0.52, 0.01, 1.003, 0.047)]
+    for fused, a in ((0, f), (1, g)):
+        cellops.cell_collide_mrt_pop_d(fused, type_, 1, *args, _ptr(a), len(a))
+    np.testing.assert_allclose(g, f, rtol=0, atol=1e-14)  # FP64 rounding of sums of 19 terms below 1
 
 
 def test_moment_stress_equals_pi_neq(cellops):
@@ -126,3 +124,42 @@ def test_moment_stress_equals_pi_neq(cellops):
     cellops.cell_mrt_dev_pi_d(_ptr(f), _ptr(r2), _ptr(p2), n)
     np.testing.assert_allclose(r2, r1, rtol=1e-14)
     np.testing.assert_allclose(p2, p1, rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("les", [0, 1])
+def test_population_collision_equals_mrt_in_fp64(cellops, les):
+    """collide_mrt_pop equals collide_mrt<MRT> in FP64, up to the rounding of
+    LR7's 0.666666667"""
+    f, _ = _states(np.zeros(19), 300, 11 + les, 0.01)
+    g = f.copy()
+    om, cs = 1 / 0.52, 0.01
+    cellops.cell_collide_d(MRT, les, ctypes.c_double(om), ctypes.c_double(cs), ctypes.c_double(0.0), _ptr(f), len(f))
+    cellops.cell_collide_mrt_pop_d(0, 0, les, *[ctypes.c_double(v) for v in (om, cs, 0.0, 0.0)], _ptr(g), len(g))
+    np.testing.assert_allclose(g, f, rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("rho", [0.99, 1.0, 1.01])
+@pytest.mark.parametrize("u", [0.0, 0.05, 0.1])
+def test_full_population_collision_fp32(cellops, rho, u):
+    """FP32 populations through the projected collision: one collision of a
+    sheared state is within a few ulp of FP64, and a uniform flow keeps its
+    mass and momentum (rounding each of 19 populations, at most half an ulp of
+    1/3 = 1.5e-8 apiece, may move the sum until the state is a fixed point: 19
+    x 1.5e-8 = 2.9e-7)"""
+    f64 = _states(np.zeros(19), 200, 31, 0.01)[0]
+    om, cs = 1 / 0.52, 0.01
+    ref, g = f64.copy(), f64.astype(np.float32)
+    cellops.cell_collide_d(MRT, 1, ctypes.c_double(om), ctypes.c_double(cs), ctypes.c_double(0.0), _ptr(ref), len(ref))
+    for row in g:
+        one = np.ascontiguousarray(row)
+        cellops.cell_iterate_mrt_pop(ctypes.c_float(om), ctypes.c_float(cs), _ptr(one), 1)
+        row[:] = one
+    assert np.abs(g - ref).max() < 5e-7
+
+    e = _feq_bgk(rho, np.array([u, 0.3 * u, -0.1 * u])).copy()
+    cellops.cell_collide_d(MRT, 0, ctypes.c_double(1.0), ctypes.c_double(0.0), ctypes.c_double(0.0), _ptr(e), 1)
+    f = e.astype(np.float32)
+    m0, j0 = f.astype(np.float64).sum(), float(np.dot(CX, f.astype(np.float64)))
+    cellops.cell_iterate_mrt_pop(ctypes.c_float(om), ctypes.c_float(cs), _ptr(f), 5000)
+    assert abs(f.astype(np.float64).sum() - m0) < 2.9e-7
+    assert abs(float(np.dot(CX, f.astype(np.float64))) - j0) < 2.9e-7
