@@ -1872,14 +1872,28 @@ int lbm_get_stats(lbm_handle* h, int level, float* stats4) {
     if (!s.stats) return fail(LBM_ERR_STATE, "statistics are off (VELAV: 0)");
     const Level& L = s.L;
     const size_t n = size_t(L.nx) * L.ny * L.nz;
-    std::vector<float> tmp(size_t(L.qstride) * 4);
-    CUDA_TRY(cudaMemcpyAsync(tmp.data(), s.stats, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(cudaStreamSynchronize(h->stream));
-    for (int k = 0; k < 4; ++k)
-        for (int z = 0; z < L.nz; ++z)
-            for (int y = 0; y < L.ny; ++y)
-                memcpy(stats4 + k * n + (size_t(z) * L.ny + y) * L.nx,
-                       tmp.data() + k * L.qstride + size_t(z) * L.plane + size_t(y) * L.pitch, L.nx * sizeof(float));
+    cudaError_t e;
+    if (void* dv = mapped_view(stats4)) {
+        e = launch_pack_rows(L, 4, s.stats, static_cast<float*>(dv), h->stream);
+        ++h->launches;
+    } else {
+        float* d = nullptr;
+        if (staging(h, 4 * n, &d) == LBM_OK) {
+            e = launch_pack_rows(L, 4, s.stats, d, h->stream);
+            ++h->launches;
+            if (e == cudaSuccess) e = cudaMemcpyAsync(stats4, d, 4 * n * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
+        } else {
+            /* no device memory left for the staging buffer: row by row */
+            cudaGetLastError();
+            e = cudaSuccess;
+            for (int k = 0; k < 4 && e == cudaSuccess; ++k)
+                e = cudaMemcpy2DAsync(stats4 + k * n, L.nx * sizeof(float), s.stats + k * L.qstride,
+                                      L.pitch * sizeof(float), L.nx * sizeof(float), size_t(L.ny) * L.nz,
+                                      cudaMemcpyDeviceToHost, h->stream);
+        }
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "get_stats: %s", cudaGetErrorString(e));
     return LBM_OK;
 }
 

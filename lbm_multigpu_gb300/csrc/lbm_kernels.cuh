@@ -276,6 +276,7 @@ cudaError_t launch_dyn_control(const Level& L, const void* f, int y1, float umax
                                float* dpdy_dev, float* hist3, int t, cudaStream_t s);
 cudaError_t launch_fields(const Level& L, const void* f, float* rho, float* u, float* v, float* w, cudaStream_t s);
 cudaError_t launch_pack(const Level& L, const void* f, float* compact, cudaStream_t s);
+cudaError_t launch_pack_rows(const Level& L, int arrays, const float* in, float* compact, cudaStream_t s);
 cudaError_t launch_unpack(const Level& L, const float* compact, void* f, cudaStream_t s);
 cudaError_t launch_audit(const Level& L, const void* f, const uint8_t* mask, double* partials, int npart,
                          double* out4, cudaStream_t s);

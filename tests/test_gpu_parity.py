@@ -1066,3 +1066,25 @@ def test_c3_configured_patch_vs_oracle(product):
     _, jf = moments(ff)
     _, jo = moments(o.ffa)
     assert rel_l2(jf[:, mf != 2], jo[:, mf != 2]) < RTOL
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(31, 13, 5), (33, 12, 6), (64, 12, 5), (70, 24, 6)])
+def test_statistics_readback(product, nx, ny, nz):
+    """the statistics without their row padding, into pageable and into pinned
+    memory: after one step from start_velav 0 the mean is the momentum of the
+    populations (19 FP32 terms below 1/3 each: 19 x 2^-24 at most apart), and
+    nothing is written at solid nodes"""
+    torch = pytest.importorskip("torch")
+    lbm = product
+    text = lbm.make_inputs(nx, ny, nz, obst1=(8.5, 5.5, 0.0), r1=2.0, re=60.0, umax=0.05, tmax=10, les=1, cs=0.01,
+                           geometry="channel_square", velav=1, start_velav=0, start_velfluc=5)
+    with lbm.Solver(text) as s:
+        s.step(1)
+        st, f, mask = s.stats(), s.populations().astype(np.float64), s.mask()
+        pin = torch.empty((4, nz, ny, nx), dtype=torch.float32, pin_memory=True)
+        lbm._check(s._lib.lbm_get_stats(s._h, 0, pin.data_ptr()))
+    np.testing.assert_array_equal(st, pin.numpy())
+    solid = np.isin(mask, [lbm.NODE["WALL"], lbm.NODE["BODY"]])
+    for k, c in enumerate((CX, CY)):
+        np.testing.assert_allclose(st[k][~solid], np.tensordot(c, f, 1)[~solid], rtol=0, atol=19 * 2.0 ** -24)
+    assert not st[:, solid].any() and not st[2:].any()
