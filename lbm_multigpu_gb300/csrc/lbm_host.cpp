@@ -570,7 +570,7 @@ struct StepGraph {
     long long epoch = -1;
     int cur1 = 0;           /* the refinement level's current buffer at the start */
     bool force = false;     /* every step records a force (else none does) */
-    int phase = 0;          /* t modulo the closure's refresh interval at the start */
+    int refresh = -1;       /* the first step that evaluates the closure, -1: none */
     const float* mom = nullptr;
     long long launches = 0; /* kernels of one replay */
 };
@@ -608,8 +608,9 @@ struct lbm_handle {
      * device (step_dev, which a graph advances by its length), so that a
      * batch is captured once and then launched again with one host call; a
      * capture costs the host 1 to 10 us per step, more than a step of a small
-     * domain takes.  By log2 of the length and the buffer it starts from */
-    StepGraph graphs[5][2];
+     * domain takes.  By log2 of the length, the buffer it starts from and
+     * whether a step of it evaluates the closure */
+    StepGraph graphs[5][2][2];
     int* step_dev = nullptr;        /* behind audit_out's four sums */
     int step_dev_val = -1;          /* its value once everything queued so far has run */
     long long epoch = 0;            /* bumped when anything that captured launches carry changes */
@@ -1037,15 +1038,40 @@ bool uses_counter(const lbm_handle* h, bool force) {
     return force || h->cfg.noise != 0.f || h->cfg.velav || h->lv[0].has_xbc || h->lv[1].has_xbc;
 }
 
+/* the first of the k steps from h->t on that evaluates the closure, or -1 */
+int closure_refresh(const lbm_handle* h, int k) {
+    const Config& c = h->cfg;
+    if (!c.sgs_mlp) return -1;
+    const int r = (c.sgs_every - h->t % c.sgs_every) % c.sgs_every;
+    return r < k ? r : -1;
+}
+
+/* Batches begin with the closure's evaluation or end before the next one, so
+ * that a run of any length meets two graphs per length at most, wherever in
+ * the closure's interval it begins (80 x 35 x 53 nodes, an evaluation every 16
+ * steps, calls of 23 steps: 427 us a call with batches cut anywhere, which
+ * were captured anew on each call, 329 us so) */
+bool closure_fits(const lbm_handle* h, int k) {
+    const Config& c = h->cfg;
+    if (!c.sgs_mlp || c.sgs_every <= 1) return true;
+    const int p = h->t % c.sgs_every;
+    return p + k <= c.sgs_every || (p == 0 && k % c.sgs_every == 0);
+}
+
+/* the graphs at hand for k = 2^lg steps from h->t on */
+StepGraph& graph_slot(lbm_handle* h, int lg) {
+    return h->graphs[lg][h->lv[0].cur][closure_refresh(h, 1 << lg) >= 0];
+}
+
 /* the executable graph of k = 2^lg steps from h->t on, when the one at hand
  * can be launched as it is */
 StepGraph* ready_graph(lbm_handle* h, int lg) {
-    StepGraph& g = h->graphs[lg][h->lv[0].cur];
+    StepGraph& g = graph_slot(h, lg);
     const Config& c = h->cfg;
     if (lg == 0 || !graph_ok(h, 1 << lg)) return nullptr;
     if (!g.exec || !g.steady || g.epoch != h->epoch || !steady_batch(h, 1 << lg)) return nullptr;
     if (g.cur1 != h->lv[1].cur || g.mom != h->mom || g.force != (h->t > c.startf)) return nullptr;
-    if (c.sgs_mlp && g.phase != h->t % c.sgs_every) return nullptr;
+    if (g.refresh != closure_refresh(h, 1 << lg)) return nullptr;
     if (g.force && h->t + (1 << lg) - c.startf > h->force_cap) return nullptr;
     return &g;
 }
@@ -1114,12 +1140,12 @@ int run_graph(lbm_handle* h, int lg) {
         h->mom = mom0, h->mom_prev = mom_prev0, h->have_mom = have_mom0, h->launches = launches0;
         h->nu_valid = nu_valid0;
     };
-    StepGraph& sg = h->graphs[lg][cur0];
+    StepGraph& sg = graph_slot(h, lg);
     sg.steady = steady_batch(h, k);
     sg.epoch = h->epoch;
     sg.cur1 = cur1;
     sg.force = t0 > c.startf;
-    sg.phase = c.sgs_mlp ? t0 % c.sgs_every : 0;
+    sg.refresh = closure_refresh(h, k);
     sg.mom = mom0;
     CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LBM_OK;
@@ -1423,9 +1449,10 @@ int lbm_destroy(lbm_handle* h) {
     if (h->ev_fine0) cudaEventDestroy(h->ev_fine0);
     if (h->ev_fine1) cudaEventDestroy(h->ev_fine1);
     if (h->fine) cudaStreamDestroy(h->fine);
-    for (auto& row : h->graphs)
-        for (StepGraph& g : row)
-            if (g.exec) cudaGraphExecDestroy(g.exec);
+    for (auto& length : h->graphs)
+        for (auto& row : length)
+            for (StepGraph& g : row)
+                if (g.exec) cudaGraphExecDestroy(g.exec);
     cudaFree(h->stage);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -1605,7 +1632,7 @@ int lbm_step(lbm_handle* h, int nsteps) {
     int ramp = graph_ok(h, 2) ? 1 : 0;
     for (int left = nsteps; left > 0;) {
         int lg = GRAPH_LG, rc;
-        while ((1 << lg) > left) --lg;
+        while (lg > 0 && ((1 << lg) > left || !closure_fits(h, 1 << lg))) --lg;
         StepGraph* g = ready_graph(h, lg);
         if (!g && lg > ramp) g = ready_graph(h, lg = ramp);
         if (!g) ramp = std::min(ramp + 1, GRAPH_LG);

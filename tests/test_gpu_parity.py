@@ -252,13 +252,15 @@ def test_uniform_step_graphs_are_bit_exact(product, precision):
         np.testing.assert_array_equal(x, y)
 
 
-@pytest.mark.parametrize("kind", ["stats_noise", "no_body", "fp16_late_force", "refined", "new_mask"])
+@pytest.mark.parametrize("kind", ["stats_noise", "no_body", "fp16_late_force", "refined", "new_mask",
+                                  "closure_5", "closure_16"])
 def test_replayed_step_graphs_are_bit_exact(product, kind):
     """graphs launched again without a new capture (the step number on the
     device): calls of several lengths equal single steps in populations,
     statistics and the recorded forces, with statistics and inlet noise, with
     no body, with the force recorded from a later step on, with refinement,
-    and with the mask changed in between"""
+    with the mask changed in between, and with the learned closure evaluated
+    every 5 or 16 steps"""
     lbm = product
     kw = dict(obst1=(18.5, 11.5, 0.0), r1=4.0, re=60.0, umax=0.05, tmax=400, les=1, cs=0.01, bounceback="halfway",
               inlet_noise=0.01, seed=5)
@@ -271,10 +273,14 @@ def test_replayed_step_graphs_are_bit_exact(product, kind):
     elif kind == "refined":
         kw.update(refinement=1, lr_dims=(32, 32, 12), lr_factor=0.5, lr_origin=(12.25, 4.25, 2.25), cf_time="linear",
                   bounceback="fullway")
+    elif kind.startswith("closure"):
+        kw.update(sgs="mlp", sgs_every=int(kind[8:]))
     text = lbm.make_inputs(64, 24, 12, **kw)
     res = []
     for calls in ([16, 16, 5, 33, 16, 1, 48], [1] * 135):
         with lbm.Solver(text) as s:
+            if kind.startswith("closure"):
+                s.set_sgs_mlp(np.fromfile(lbm.LIB_PATH.parent.parent / "data" / "sgs_mlp.bin", np.float32))
             t = 0
             for n in calls:
                 s.step(n)
