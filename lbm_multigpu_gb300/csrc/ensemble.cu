@@ -66,12 +66,12 @@ __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float
 /* The step with the learned closure, as k_stream_collide_mlp: tiles of 32 x 4
  * (one M = 128 MMA per layer) and persistent blocks; the populations stay in
  * registers across the tensor-core round trips.  Eight boxes of sides 32 to 80
- * (1.8 M nodes): about 100 us with 7 blocks per SM and just their shared
+ * (1.8 M nodes): about 100 us with 5 blocks per SM and just their shared
  * memory taken from L1 (one block of 256 rows per SM, what the occupancy API
  * made of kernels with TMEM: 188 us).  The features are rounded to BF16, so
  * the order of operations that leads to them is part of the result: the
  * projected collision (87 us) moves the fields of 50 steps by 1e-5. */
-constexpr int MLP_TY = 4, MLP_ROWS = 32 * MLP_TY, MLP_BLOCKS = 7;
+constexpr int MLP_TY = 4, MLP_ROWS = 32 * MLP_TY, MLP_BLOCKS = 5;
 __global__ void __launch_bounds__(MLP_ROWS, MLP_BLOCKS) k_ens_step_mlp(const Table T, const float* __restrict__ fA,
                                                                        float* __restrict__ fB,
                                                                        const unsigned char* __restrict__ blob,

@@ -477,15 +477,16 @@ __global__ void __launch_bounds__(SC_BX* SC_BY, sc_min_blocks<S, FEAT>()) k_stre
  * sector of a row twice to an SM (q and its opposite are pulled by different
  * rows) unless L1 still holds it, and a block's operands take 27 KB of the
  * array that L1 shares with shared memory.  So the launch asks for exactly the
- * shared memory of its resident blocks (7: 196 of 228 KB).  512 x 128 x 128,
- * FP32: 316 us (40 steps with their start 16.3 ms); with all of the array as shared memory 433 us, and 376 us with
- * the network left out altogether; 4, 5, 6, 8 blocks per SM 370, 314, 362,
- * 478 us (FP16 408, 322, 353, 402 and with 7 313 us).  Copying the next
- * tile's pulls into shared memory with cp.async cost more L1 than it hid
- * (462 us). */
+ * shared memory of its resident blocks (5: 140 of 228 KB).  512 x 128 x 128,
+ * FP32, 40 steps and a read-back: 16.4 ms, with all of the array as shared
+ * memory 21.4 ms.  Five blocks per SM also leave 96 registers a thread and so
+ * no spills; 7 blocks (72 registers) take 16.3 ms there, but 4.56 instead of
+ * 4.00 ms for 50 steps of 211 x 90 x 70 nodes (FP16 / BF16: 4.60 and 4.00 ms;
+ * 4 blocks 4.37, 6 blocks 4.04).  Copying the next tile's pulls into shared
+ * memory with cp.async cost more L1 than it hid. */
 constexpr int MLP_BY = 4; /* tile 32 x 4: one M = 128 MMA per layer */
 constexpr int MLP_ROWS = SC_BX * MLP_BY;
-constexpr int MLP_BLOCKS = 7;
+constexpr int MLP_BLOCKS = 5;
 
 /* the 19 values g of node c into buffer f, as store19 */
 template <int LAY> struct CellIdx {
