@@ -1035,7 +1035,8 @@ bool steady_batch(const lbm_handle* h, int k) {
 
 /* whether any launch of a steady batch reads the counter */
 bool uses_counter(const lbm_handle* h, bool force) {
-    return force || h->cfg.noise != 0.f || h->cfg.velav || h->lv[0].has_xbc || h->lv[1].has_xbc;
+    const bool body = h->lv[h->cfg.refinement ? 1 : 0].nbody > 0; /* else no force is reduced */
+    return (force && body) || h->cfg.noise != 0.f || h->cfg.velav || h->lv[0].has_xbc || h->lv[1].has_xbc;
 }
 
 /* the first of the k steps from h->t on that evaluates the closure, or -1 */
