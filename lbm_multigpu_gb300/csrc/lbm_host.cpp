@@ -1635,8 +1635,10 @@ int lbm_step(lbm_handle* h, int nsteps) {
         int lg = GRAPH_LG, rc;
         while (lg > 0 && ((1 << lg) > left || !closure_fits(h, 1 << lg))) --lg;
         StepGraph* g = ready_graph(h, lg);
-        if (!g && lg > ramp) g = ready_graph(h, lg = ramp);
-        if (!g) ramp = std::min(ramp + 1, GRAPH_LG);
+        if (!g) {
+            if (lg > ramp) g = ready_graph(h, lg = ramp);
+            ramp = std::min(ramp + 1, GRAPH_LG);
+        }
         if (g) rc = replay_graph(h, *g, 1 << lg);
         else if (lg > 0 && graph_ok(h, 1 << lg)) rc = run_graph(h, lg);
         else rc = one_step(h), lg = 0;

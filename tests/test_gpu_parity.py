@@ -1094,3 +1094,16 @@ def test_statistics_readback(product, nx, ny, nz):
     for k, c in enumerate((CX, CY)):
         np.testing.assert_allclose(st[k][~solid], np.tensordot(c, f, 1)[~solid], rtol=0, atol=19 * 2.0 ** -24)
     assert not st[:, solid].any() and not st[2:].any()
+
+
+def test_step_graphs_grow_after_a_short_call(product):
+    """a short call leaves graphs of 2, 4 and 8 steps; a long one after it
+    grows to batches of 16: beside two kernels a step, at most one launch per
+    batch of 16 and one for each of the shorter ones and the counter's start"""
+    lbm = product
+    with lbm.Solver(lbm.make_inputs(64, 24, 12, obst1=(18.5, 11.5, 0.0), r1=4.0, re=60.0, umax=0.05, tmax=1000, les=1,
+                                    cs=0.01, bounceback="halfway")) as s:
+        s.step(20)
+        n0 = s.launch_count()
+        s.step(640)
+        assert s.launch_count() - n0 <= 2 * 640 + 640 // 16 + 12
