@@ -365,13 +365,16 @@ __global__ void __launch_bounds__(GTH) k_mlp_predict(const float* __restrict__ p
 constexpr int SHUFFLE_ROUNDS = 24;
 using U64 = unsigned long long;
 
+__device__ __forceinline__ GridWalk my_walk() { return grid_walk(blockIdx.x, gridDim.x, threadIdx.x, blockDim.x); }
+
 __global__ void k_shuffle_draw(int* __restrict__ H, int n, U64 state) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 1 || i >= n) return;
-    U64 z = state + U64(n - i) * 0x9E3779B97F4A7C15ull;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    H[i] = int((z ^ (z >> 31)) % U64(i + 1));
+    for (GridWalk w = my_walk(); w.at < n; w.at += w.step) {
+        const int i = int(w.at);
+        U64 z = state + U64(n - i) * 0x9E3779B97F4A7C15ull;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        if (i > 0) H[i] = int((z ^ (z >> 31)) % (U64(i) + 1));
+    }
 }
 
 __device__ __forceinline__ void shuffle_enter(const int* __restrict__ H, U64* __restrict__ R, int i, U64 round) {
@@ -395,16 +398,16 @@ __global__ void k_shuffle_enter(const int* __restrict__ H, U64* __restrict__ R, 
                                 const int* __restrict__ count, int n, U64 round) {
     pdl_wait();
     const int m = list ? __ldcg(count) : n - 1;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x)
-        shuffle_enter(H, R, list ? __ldcg(list + j) : j + 1, round);
+    for (GridWalk w = my_walk(); w.at < m; w.at += w.step)
+        shuffle_enter(H, R, list ? __ldcg(list + w.at) : int(w.at) + 1, round);
 }
 __global__ void k_shuffle_swap(const int* __restrict__ H, const U64* __restrict__ R, int* perm,
                                const int* __restrict__ list, const int* __restrict__ count, int n, U64 round,
                                int* __restrict__ left, int* __restrict__ left_count) {
     pdl_wait();
     const int m = list ? __ldcg(count) : n - 1;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-        const int i = list ? __ldcg(list + j) : j + 1;
+    for (GridWalk w = my_walk(); w.at < m; w.at += w.step) {
+        const int i = list ? __ldcg(list + w.at) : int(w.at) + 1;
         const bool due = !shuffle_swap(H, R, perm, i, round);
         const unsigned who = __activemask(), ask = __ballot_sync(who, due);
         if (!due) continue;
@@ -423,11 +426,11 @@ __global__ void __launch_bounds__(1024) k_shuffle_rest(const int* __restrict__ H
     __shared__ int left;
     int m = __ldcg(count);
     for (; m > 0; ++round) {
-        for (int j = threadIdx.x; j < m; j += blockDim.x) shuffle_enter(H, R, __ldcg(list + j), round);
+        for (long long j = threadIdx.x; j < m; j += blockDim.x) shuffle_enter(H, R, __ldcg(list + j), round);
         if (threadIdx.x == 0) left = 0;
         __threadfence();
         __syncthreads();
-        for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        for (long long j = threadIdx.x; j < m; j += blockDim.x) {
             const int i = __ldcg(list + j);
             if (!shuffle_swap(H, R, perm, i, round)) other[atomicAdd(&left, 1)] = i;
         }
@@ -441,8 +444,7 @@ __global__ void __launch_bounds__(1024) k_shuffle_rest(const int* __restrict__ H
     }
 }
 __global__ void k_iota(int* p, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = i;
+    for (GridWalk w = my_walk(); w.at < n; w.at += w.step) p[w.at] = int(w.at);
 }
 
 /* ---- tensor-core self-check: D[128][64] = A[128][K] B[64][K]^T, K = 16 * kc */
@@ -566,18 +568,18 @@ size_t shuffle_scratch_bytes(int n) {
 
 cudaError_t launch_shuffle(int* perm, int n, unsigned long long state, int epoch, void* scratch, cudaStream_t s) {
     using sgs::U64;
-    const int blocks = (n + 255) / 256, wide = blocks < 152 * 8 ? blocks : 152 * 8;
+    const int wide = sgs::groups_of(n, 256, 152 * 8);
     U64* R = static_cast<U64*>(scratch);
     int* H = reinterpret_cast<int*>(R + n);
     int *list = H + n, *other = list + n, *count = other + n;
     cudaError_t e = cudaMemsetAsync(count, 0, (sgs::SHUFFLE_ROUNDS + 1) * sizeof(int), s);
-    if (epoch == 0) sgs::k_iota<<<blocks, 256, 0, s>>>(perm, n);
+    if (epoch == 0) sgs::k_iota<<<wide, 256, 0, s>>>(perm, n);
     /* round numbers have 32 bits: 2^20 for each of 2^12 epochs (some 2.7 ln n
      * are needed), then R is cleared */
     const int era = epoch & 4095;
     if (era == 0 && e == cudaSuccess) e = cudaMemsetAsync(R, 0, size_t(n) * sizeof(U64), s);
     if (e != cudaSuccess) return e;
-    sgs::k_shuffle_draw<<<blocks, 256, 0, s>>>(H, n, state);
+    sgs::k_shuffle_draw<<<wide, 256, 0, s>>>(H, n, state);
     U64 round = (U64(era) << 20) + 1;
     const int* from = nullptr;
     for (int r = 0; r < sgs::SHUFFLE_ROUNDS && e == cudaSuccess; ++r, ++round) {

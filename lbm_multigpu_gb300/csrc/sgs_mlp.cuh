@@ -42,6 +42,21 @@ constexpr int OFF_W1 = 0, OFF_W2 = OFF_W1 + NH * NIN, OFF_B2 = OFF_W2 + NH * NH,
               OFF_B3 = OFF_W3 + NH, NPARAM = OFF_B3 + 1;
 constexpr float P_REF = 0.01f, NU_SCALE = 1e-4f;
 
+/* the elements of an array that one thread of a grid takes: at, at + step, ...
+ * below the array's size.  64 bits: an array holds up to 2^31 - 1 elements, and
+ * the last step goes past its end */
+struct GridWalk {
+    long long at, step;
+};
+__host__ __device__ inline GridWalk grid_walk(unsigned block, unsigned blocks, unsigned thread, unsigned threads) {
+    return {(long long)block * threads + thread, (long long)blocks * threads};
+}
+/* groups of `per` that n elements fill, up to `most` */
+inline int groups_of(long long n, int per, long long most) {
+    const long long b = (n + per - 1) / per;
+    return int(b < 1 ? 1 : b < most ? b : most);
+}
+
 /* features of one node from p_ij (xx, yy, zz, xy, xz, yz), tau0 and
  * inv_t0 = 1 / tau0 (a kernel computes it once) */
 template <class T> __host__ __device__ inline void features(const T p[6], T tau0, T inv_t0, T x[NIN]) {

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "../../lbm_multigpu_gb300/csrc/d3q19.cuh"
+#include "../../lbm_multigpu_gb300/csrc/sgs_mlp.cuh"
 
 using namespace lbm;
 
@@ -69,6 +70,18 @@ void cell_mrt_dev_pi_d(const double* f, double* rho, double* p6, int n) {
 float cell_philox_uniform(uint32_t seed, uint32_t cell, uint32_t step) { return philox_uniform(seed, cell, step); }
 void cell_alt_boundary(int type, float* f, int n, const int* yz, int ny, int nz, float u, int t) {
     for (int i = 0; i < n; ++i) alt_boundary<float>(type, f + 19L * i, 0, yz[2 * i], yz[2 * i + 1], 0, ny, nz, u, t);
+}
+
+/* a grid-stride walk over n elements, `per` a block and `most` blocks: the lowest and the highest index that the
+ * block's thread takes, and how many */
+void cell_grid_walk(long long n, int per, long long most, int block, int thread, long long* out3) {
+    const int blocks = sgs::groups_of(n, per, most);
+    out3[0] = n, out3[1] = -1, out3[2] = 0;
+    for (sgs::GridWalk w = sgs::grid_walk(block < 0 ? blocks - 1 : block, blocks, thread, per); w.at < n; w.at += w.step) {
+        out3[0] = w.at < out3[0] ? w.at : out3[0];
+        out3[1] = w.at > out3[1] ? w.at : out3[1];
+        ++out3[2];
+    }
 }
 
 }  // extern "C"
