@@ -206,7 +206,7 @@ int lbm_mlp_train(const float* d_X, const float* d_T, int n, int batch, int step
     Rng r(seed);
     int pos = n, epoch = 0;
     for (int st = 0; st < steps; ++st) {
-        if (pos + batch > n) {
+        if (batch > n - pos) {
             SGS_TRY(launch_shuffle(idx.p, n, r.s, epoch++, shuffle.p, s), "shuffle launch");
             r.skip(uint64_t(n - 1));
             pos = 0;

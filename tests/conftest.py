@@ -58,6 +58,37 @@ def cellops(tmp_path_factory):
 
 
 @pytest.fixture(scope="session")
+def fakecuda(tmp_path_factory):
+    """the library's host sources over a stand-in for the CUDA runtime and the
+    kernels (test-only, tests/native/fake_cuda.cpp): bookkeeping and error
+    paths without a GPU"""
+    from lbm_multigpu_gb300.build import CSRC, nvcc
+
+    d = tmp_path_factory.mktemp("fakecuda")
+    inc = "-I" + str(Path(nvcc()).resolve().parents[1] / "include")
+    cxx = ["g++", "-O1", "-std=c++17", "-fPIC", inc]
+    srcs = [CSRC / "lbm_host.cpp", CSRC / "lbm_sgs.cpp", CSRC / "lbm_ensemble.cpp", ROOT / "tests" / "native" / "fake_cuda.cpp"]
+    objs = [str(d / (p.stem + ".o")) for p in srcs]
+    for p, r in [(p, subprocess.Popen([*cxx, "-c", str(p), "-o", o])) for p, o in zip(srcs, objs)]:
+        assert r.wait() == 0, p
+    names = {f: {line.split()[-1] for line in subprocess.run(["nm", *f, *objs], capture_output=True, text=True,
+                                                            check=True).stdout.splitlines() if len(line.split()) > 1}
+             for f in (("-u",), ("--defined-only",))}
+    rest = sorted(n for n in names["-u",] - names["--defined-only",] if n.startswith(("cuda", "_ZN3lbm")))
+    stubs = d / "stubs.c"
+    stubs.write_text("".join(f"long {n}(void) {{ return 0; }}\n" for n in rest))
+    out = d / "fakecuda.so"
+    r = subprocess.run(["gcc", "-O1", "-fPIC", "-c", str(stubs), "-o", str(d / "stubs.o")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run(["g++", "-shared", "-o", str(out), *objs, str(d / "stubs.o")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    lib = ctypes.CDLL(str(out))
+    lib.fake_calls.restype = lib.fake_trace.restype = ctypes.c_long
+    lib.lbm_last_error.restype = ctypes.c_char_p
+    return lib
+
+
+@pytest.fixture(scope="session")
 def golden():
     import numpy as np
 

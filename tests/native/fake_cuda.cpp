@@ -1,0 +1,141 @@
+/*
+ * fake_cuda.cpp -- test-only stand-in for the CUDA runtime and the kernel
+ * launchers under the library's host sources (lbm_host.cpp, lbm_sgs.cpp,
+ * lbm_ensemble.cpp), so that their bookkeeping and their error paths run
+ * without a GPU: device memory is host memory, work on a stream is done at
+ * once, kernels do nothing.  Every other symbol that the sources need is a
+ * function that returns 0 (conftest.py generates them).  Not part of the
+ * product library.
+ */
+#include <cuda_runtime_api.h>
+#include <stdint.h>
+#include <string.h>
+#include <sys/mman.h>
+
+#include <map>
+#include <string>
+#include <vector>
+
+namespace {
+std::map<void*, size_t> g_mem;
+std::map<std::string, long> g_calls, g_fail_at;
+std::map<std::string, size_t> g_fail_above;
+std::vector<long long> g_trace;
+const int* g_perm = nullptr; /* the permutation that a shuffle last filled */
+
+/* counts the call; true when a test asked for it to fail */
+bool failing(const char* fn, size_t bytes = 0) {
+    const long n = ++g_calls[fn];
+    if (g_fail_at.count(fn) && g_fail_at[fn] == n) return true;
+    return g_fail_above.count(fn) && bytes > g_fail_above[fn];
+}
+cudaError_t take(void** p, size_t n) {
+    /* address space only: a test may ask for more than the machine has */
+    void* m = mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+    if (m == MAP_FAILED) return cudaErrorMemoryAllocation;
+    g_mem[m] = n ? n : 1;
+    *p = m;
+    return cudaSuccess;
+}
+cudaError_t give(void* p) {
+    if (!p) return cudaSuccess;
+    if (!g_mem.count(p)) return cudaErrorInvalidValue;
+    munmap(p, g_mem[p]);
+    g_mem.erase(p);
+    return cudaSuccess;
+}
+}  // namespace
+
+extern "C" {
+
+/* for the tests: the call number `at` of fn from now on fails (0: none), or every one for more than `bytes` bytes */
+void fake_fail(const char* fn, long at) { g_fail_at[fn] = at ? g_calls[fn] + at : 0; }
+void fake_fail_above(const char* fn, size_t bytes) { g_fail_above[fn] = bytes; }
+long fake_calls(const char* fn) { return g_calls[fn]; }
+size_t fake_blocks() { return g_mem.size(); }
+/* what the launchers below noted */
+long fake_trace(long long* out, long cap) {
+    const long n = long(g_trace.size());
+    for (long i = 0; i < n && i < cap; ++i) out[i] = g_trace[i];
+    return n;
+}
+void fake_reset() {
+    g_calls.clear(), g_fail_at.clear(), g_fail_above.clear(), g_trace.clear(), g_perm = nullptr;
+}
+
+cudaError_t cudaMalloc(void** p, size_t n) { return failing("cudaMalloc", n) ? cudaErrorMemoryAllocation : take(p, n); }
+cudaError_t cudaFree(void* p) { return give(p); }
+cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) {
+    return failing("cudaMallocFromPoolAsync", n) ? cudaErrorMemoryAllocation : take(p, n);
+}
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return give(p); }
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    if (failing("cudaMemcpy", n)) return cudaErrorUnknown;
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+    if (failing("cudaMemcpyAsync", n)) return cudaErrorUnknown;
+    memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemset(void* d, int v, size_t n) { return memset(d, v, n), cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return memset(d, v, n), cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 152, cudaSuccess; }
+cudaError_t cudaDeviceGetStreamPriorityRange(int* a, int* b) { return *a = *b = 0, cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+    return *a = cudaPointerAttributes{}, cudaSuccess;
+}
+const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
+/* one step-graph executable is as good as another: a number */
+static uintptr_t g_next = 0;
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+    return failing("cudaStreamBeginCapture") ? cudaErrorIllegalState : cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
+    *g = reinterpret_cast<cudaGraph_t>(++g_next);
+    return failing("cudaStreamEndCapture") ? cudaErrorUnknown : cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) {
+    if (failing("cudaGraphInstantiate")) return cudaErrorUnknown;
+    *x = reinterpret_cast<cudaGraphExec_t>(++g_next);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphExecUpdate(cudaGraphExec_t, cudaGraph_t, cudaGraphExecUpdateResultInfo*) {
+    return failing("cudaGraphExecUpdate") ? cudaErrorUnknown : cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) {
+    return failing("cudaGraphLaunch") ? cudaErrorUnknown : cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
+    return *s = reinterpret_cast<cudaStream_t>(++g_next), cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t* s, unsigned f, int) { return cudaStreamCreateWithFlags(s, f); }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    return *e = reinterpret_cast<cudaEvent_t>(++g_next), cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t* e) { return cudaEventCreateWithFlags(e, 0); }
+cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) {
+    return *p = reinterpret_cast<cudaMemPool_t>(++g_next), cudaSuccess;
+}
+
+}  // extern "C"
+
+namespace lbm {
+int force_partials() { return 608; }
+int ens_step_resident(int, int) { return 608; }
+int mlp_grad_blocks(int) { return 1; }
+size_t shuffle_scratch_bytes(int n) { return 20 * size_t(n); }
+cudaError_t launch_shuffle(int* perm, int, unsigned long long, int, void*, cudaStream_t) {
+    g_calls["launch_shuffle"]++;
+    g_perm = perm;
+    return cudaSuccess;
+}
+/* notes where the batch begins and its size */
+cudaError_t launch_mlp_grad(const float*, const float*, const float*, const int* idx, int n, float*, int, cudaStream_t) {
+    g_trace.push_back(g_perm ? idx - g_perm : -1); /* -1: nothing filled the permutation yet */
+    g_trace.push_back(n);
+    return cudaSuccess;
+}
+}  // namespace lbm
