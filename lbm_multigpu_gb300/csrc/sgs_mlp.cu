@@ -510,11 +510,12 @@ __global__ void __launch_bounds__(128) k_mlp_predict_tc(const unsigned char* __r
 #if defined(__CUDA_ARCH__)
     InferSmem<128>& s = *reinterpret_cast<InferSmem<128>*>(dsm);
     infer_setup<128>(s, blob);
-    for (int base = blockIdx.x * 128; base < n; base += gridDim.x * 128) {
-        const int i = base + threadIdx.x;
+    /* the block's tiles: the same number of passes for all of its threads */
+    for (GridWalk w = grid_walk(blockIdx.x, gridDim.x, 0, 128); w.at < n; w.at += w.step) {
+        const long long i = w.at + threadIdx.x;
         float x[NIN];
 #pragma unroll
-        for (int k = 0; k < NIN; ++k) x[k] = i < n ? X[size_t(i) * NIN + k] : 0.f;
+        for (int k = 0; k < NIN; ++k) x[k] = i < n ? X[i * NIN + k] : 0.f;
         const float v = infer_nu<128>(s, x, err);
         if (v < 0.f) break; /* a tensor-core wait ran out (block-uniform) */
         if (i < n) nu[i] = v;
@@ -598,9 +599,7 @@ cudaError_t launch_shuffle(int* perm, int n, unsigned long long state, int epoch
 }
 
 cudaError_t launch_mlp_predict_tc(const void* blob, const float* X, int n, float* nu, int* err, cudaStream_t s) {
-    int b = (n + 127) / 128;
-    if (b > 152 * 4) b = 152 * 4;
-    if (b < 1) b = 1;
+    const int b = sgs::groups_of(n, 128, 152 * 4);
     const size_t smem = sgs::infer_dyn_smem<128>();
     static cudaError_t attr = cudaErrorNotReady;
     if (attr == cudaErrorNotReady)

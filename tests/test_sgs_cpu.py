@@ -357,15 +357,19 @@ def test_bf16_inference_error_is_within_the_gpu_tolerance(product):
 
 
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 152 * 8 * 256 + 1, 2_147_172_353, 2_147_172_354, 2 ** 31 - 255, 2 ** 31 - 1])
-def test_grid_walk_stays_inside_the_array(cellops, n):
-    """the index walk of the shuffle's kernels up to the largest sample count
-    (a 32-bit index wraps in the step past the end from n = 2,147,172,354
-    on): every thread stays in 0 .. n - 1 and takes all of its elements"""
-    step = min((n + 255) // 256, 152 * 8) * 256
+@pytest.mark.parametrize("per,most", [(256, 152 * 8), (128, 152 * 4)])
+def test_grid_walk_stays_inside_the_array(cellops, n, per, most):
+    """the index walk of the shuffle's kernels and of the tensor-core
+    prediction (by its blocks' first threads) up to the largest sample count
+    (a 32-bit index wraps in the step past the end from n = 2,147,172,354 and
+    2,147,405,825 on): every thread stays in 0 .. n - 1 and takes all of its
+    elements"""
+    step = min((n + per - 1) // per, most) * per
     last = (n - 1) % step   # the thread that takes element n - 1
-    for block, thread, first in ((0, 0, 0), (last // 256, last % 256, last), (-1, 0, step - 256), (-1, 255, step - 1)):
+    for block, thread, first in ((0, 0, 0), (last // per, last % per, last), (-1, 0, step - per),
+                                 (-1, per - 1, step - 1)):
         out = (ctypes.c_longlong * 3)()
-        cellops.cell_grid_walk(ctypes.c_longlong(n), 256, ctypes.c_longlong(152 * 8), block, thread, out)
+        cellops.cell_grid_walk(ctypes.c_longlong(n), per, ctypes.c_longlong(most), block, thread, out)
         count = max(0, (n - first + step - 1) // step)
         assert out[2] == count
         if count:
