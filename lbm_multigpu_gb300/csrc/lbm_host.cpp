@@ -1141,8 +1141,11 @@ int run_graph(lbm_handle* h, int lg) {
         h->mom = mom0, h->mom_prev = mom_prev0, h->have_mom = have_mom0, h->launches = launches0;
         h->nu_valid = nu_valid0;
     };
+    /* the slot is not ready (steady) while its executable is not of the steps
+     * that it describes, which lasts on every early return */
     StepGraph& sg = graph_slot(h, lg);
-    sg.steady = steady_batch(h, k);
+    sg.steady = false;
+    const bool steady = steady_batch(h, k);
     sg.epoch = h->epoch;
     sg.cur1 = cur1;
     sg.force = t0 > c.startf;
@@ -1150,8 +1153,8 @@ int run_graph(lbm_handle* h, int lg) {
     sg.mom = mom0;
     CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LBM_OK;
-    for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h, sg.steady ? j : -1, j > 0);
-    if (rc == LBM_OK && sg.steady && uses_counter(h, sg.force)) {
+    for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h, steady ? j : -1, j > 0);
+    if (rc == LBM_OK && steady && uses_counter(h, sg.force)) {
         const cudaError_t e = launch_advance_step(h->step_dev, k, h->stream);
         if (e != cudaSuccess) rc = fail(LBM_ERR_CUDA, "step counter: %s", cudaGetErrorString(e));
         ++h->launches;
@@ -1163,7 +1166,6 @@ int run_graph(lbm_handle* h, int lg) {
         if (g) cudaGraphDestroy(g);
         cudaGetLastError();
         restore();
-        sg.steady = false;
         return rc != LBM_OK ? rc : fail(LBM_ERR_CUDA, "step capture: %s", cudaGetErrorString(ec));
     }
     cudaError_t e = cudaSuccess;
@@ -1177,6 +1179,7 @@ int run_graph(lbm_handle* h, int lg) {
     }
     if (!sg.exec) e = cudaGraphInstantiate(&sg.exec, g, 0);
     cudaGraphDestroy(g);
+    sg.steady = steady && e == cudaSuccess;
     rc = e == cudaSuccess ? launch_graph(h, sg, t0, k) : fail(LBM_ERR_CUDA, "step graph: %s", cudaGetErrorString(e));
     if (rc) {
         restore();

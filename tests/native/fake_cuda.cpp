@@ -88,8 +88,14 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
     return *a = cudaPointerAttributes{}, cudaSuccess;
 }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
-/* one step-graph executable is as good as another: a number */
+/* handles are numbers; of a step graph's executable the stand-in keeps when it was last built or updated */
 static uintptr_t g_next = 0;
+static std::map<cudaGraphExec_t, uintptr_t> g_built;
+static uintptr_t g_mark = 0;
+static long g_stale = 0;
+/* from here on: the launches of executables last built before this call */
+void fake_mark() { g_mark = ++g_next, g_stale = 0; }
+long fake_stale_launches() { return g_stale; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
     return failing("cudaStreamBeginCapture") ? cudaErrorIllegalState : cudaSuccess;
 }
@@ -100,13 +106,18 @@ cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) {
     if (failing("cudaGraphInstantiate")) return cudaErrorUnknown;
     *x = reinterpret_cast<cudaGraphExec_t>(++g_next);
+    g_built[*x] = g_next;
     return cudaSuccess;
 }
-cudaError_t cudaGraphExecUpdate(cudaGraphExec_t, cudaGraph_t, cudaGraphExecUpdateResultInfo*) {
-    return failing("cudaGraphExecUpdate") ? cudaErrorUnknown : cudaSuccess;
+cudaError_t cudaGraphExecUpdate(cudaGraphExec_t x, cudaGraph_t, cudaGraphExecUpdateResultInfo*) {
+    if (failing("cudaGraphExecUpdate")) return cudaErrorUnknown;
+    g_built[x] = ++g_next;
+    return cudaSuccess;
 }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) {
-    return failing("cudaGraphLaunch") ? cudaErrorUnknown : cudaSuccess;
+cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t) {
+    if (failing("cudaGraphLaunch")) return cudaErrorUnknown;
+    g_stale += g_built[x] < g_mark;
+    return cudaSuccess;
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     return *s = reinterpret_cast<cudaStream_t>(++g_next), cudaSuccess;

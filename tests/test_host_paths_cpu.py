@@ -37,3 +37,33 @@ def test_batches_stay_inside_the_samples(fake, n, batch):
     int): each lies within the permutation"""
     for start, size in _train(fake, n, batch, 4):
         assert 0 <= start and start + size <= n
+
+
+def _solver(fake, **kw):
+    import lbm_multigpu_gb300 as lbm
+
+    h = ctypes.c_void_p()
+    text = lbm.make_inputs(64, 24, 12, obst1=(18.5, 11.5, 0.0), r1=4.0, re=60.0, umax=0.05, tmax=1000, les=1, cs=0.01,
+                           bounceback="halfway", **kw)
+    assert fake.lbm_create(text.encode(), ctypes.byref(h)) == 0, fake.lbm_last_error()
+    return h
+
+
+@pytest.mark.parametrize("call", ["cudaStreamBeginCapture", "cudaStreamEndCapture", "cudaGraphInstantiate"])
+def test_failed_capture_leaves_no_stale_graph(fake, call):
+    """a capture that fails after a mask change: the next call captures the
+    steps anew instead of launching the graph of the old mask"""
+    h = _solver(fake)
+    mask = np.zeros((12, 24, 64), np.uint8)
+    assert fake.lbm_step(h, 64) == 0
+    assert fake.lbm_set_mask(h, 0, _ptr(mask)) == 0, fake.lbm_last_error()
+    fake.fake_mark()
+    if call == "cudaGraphInstantiate":   # reached when the old executable cannot be updated in place
+        fake.fake_fail(b"cudaGraphExecUpdate", 1)
+    fake.fake_fail(call.encode(), 1)
+    assert fake.lbm_step(h, 64) != 0
+    fake.fake_fail(b"cudaGraphExecUpdate", 0)
+    launches = fake.fake_calls(b"cudaGraphLaunch")
+    assert fake.lbm_step(h, 64) == 0, fake.lbm_last_error()
+    assert fake.fake_calls(b"cudaGraphLaunch") > launches and fake.fake_stale_launches() == 0
+    assert fake.lbm_destroy(h) == 0
