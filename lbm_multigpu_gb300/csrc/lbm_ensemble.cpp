@@ -293,8 +293,9 @@ int lbm_ensemble_init_turbulence(lbm_ensemble* e, uint32_t seed, float u_rms, in
     if (!e || !(u_rms >= 0) || kmax_div < 2 || per_shell < 1) return set_error(LBM_ERR_ARG, "bad argument", cudaSuccess);
     std::vector<ens::Mode> all;
     std::vector<ens::KMode> sorted;
-    for (int m = 0; m < e->T.count; ++m) {
-        ens::Member& M = e->T.m[m];
+    ens::Table T = e->T; /* the ensemble keeps its modes until the new ones are on the device */
+    for (int m = 0; m < T.count; ++m) {
+        ens::Member& M = T.m[m];
         M.mode0 = int(all.size());
         make_modes(M.n, std::max(1, M.n / kmax_div), per_shell, (uint64_t(seed) << 8) + uint64_t(m), u_rms, all);
         M.nmodes = int(all.size()) - M.mode0;
@@ -310,11 +311,16 @@ int lbm_ensemble_init_turbulence(lbm_ensemble* e, uint32_t seed, float u_rms, in
         std::stable_sort(sorted.begin() + M.mode0, sorted.end(),
                          [](const ens::KMode& a, const ens::KMode& b) { return a.k[0] < b.k[0]; });
     }
+    ens::KMode* dev = nullptr;
+    ENS_TRY(cudaMalloc(&dev, std::max<size_t>(1, sorted.size()) * sizeof(ens::KMode)), "modes");
+    if (cudaError_t r = cudaMemcpy(dev, sorted.data(), sorted.size() * sizeof(ens::KMode), cudaMemcpyHostToDevice)) {
+        cudaFree(dev);
+        return set_error(LBM_ERR_CUDA, "modes", r);
+    }
     cudaFree(e->kmodes);
-    e->kmodes = nullptr;
-    ENS_TRY(cudaMalloc(&e->kmodes, std::max<size_t>(1, sorted.size()) * sizeof(ens::KMode)), "modes");
-    ENS_TRY(cudaMemcpy(e->kmodes, sorted.data(), sorted.size() * sizeof(ens::KMode), cudaMemcpyHostToDevice), "modes");
+    e->kmodes = dev;
     e->modes = std::move(all);
+    e->T = T;
     ENS_TRY(launch_ens_init(e->T, e->kmodes, e->f[0], e->stream), "turbulence init");
     e->cur = 0;
     e->steps = 0;

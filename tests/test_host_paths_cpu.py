@@ -67,3 +67,33 @@ def test_failed_capture_leaves_no_stale_graph(fake, call):
     assert fake.lbm_step(h, 64) == 0, fake.lbm_last_error()
     assert fake.fake_calls(b"cudaGraphLaunch") > launches and fake.fake_stale_launches() == 0
     assert fake.lbm_destroy(h) == 0
+
+
+@pytest.mark.parametrize("call", ["cudaMalloc", "cudaMemcpy"])
+@pytest.mark.parametrize("before", [0, 1])
+def test_modes_after_a_failed_initialisation(fake, call, before):
+    """lbm_ensemble_modes after an lbm_ensemble_init_turbulence that failed on
+    the device: the modes of the last field that was made (before: an earlier
+    one with fewer modes), none without one"""
+    h, sizes, tau = ctypes.c_void_p(), np.array([32, 48], np.int32), np.array([0.6, 0.6], np.float32)
+    assert fake.lbm_ensemble_create(2, _ptr(sizes), _ptr(tau), 0, ctypes.c_float(0.01), ctypes.byref(h)) == 0
+
+    def modes(member):
+        n = ctypes.c_int()
+        k, ph, a = np.zeros((4096, 3), np.int32), np.zeros(4096), np.zeros((4096, 3))
+        assert fake.lbm_ensemble_modes(h, member, _ptr(k), _ptr(ph), _ptr(a), 4096, ctypes.byref(n)) == 0
+        return n.value, k[:n.value].copy(), ph[:n.value].copy(), a[:n.value].copy()
+
+    u = ctypes.c_float(0.04)
+    if before:
+        assert fake.lbm_ensemble_init_turbulence(h, 1, u, 16, 2) == 0, fake.lbm_last_error()
+    want = [modes(m) for m in range(2)]
+    assert (want[1][0] > 0) == bool(before)
+    fake.fake_fail(call.encode(), 1)
+    assert fake.lbm_ensemble_init_turbulence(h, 2, u, 4, 24) != 0
+    for m in range(2):
+        got = modes(m)
+        assert got[0] == want[m][0]
+        for x, y in zip(got[1:], want[m][1:]):
+            np.testing.assert_array_equal(x, y)
+    assert fake.lbm_ensemble_destroy(h) == 0
