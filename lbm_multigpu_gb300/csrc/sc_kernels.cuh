@@ -676,11 +676,14 @@ template <class S, bool HW, int LAY>
 static cudaError_t sc_mlp_t(const Level& L, const StepParams& p, const void* fA, void* fB, const uint8_t* mask,
                             float* stats, const uint32_t* links, const void* blob, int* err, cudaStream_t s) {
     const size_t smem = sgs::infer_dyn_smem<MLP_ROWS>();
-    static cudaError_t attr = cudaErrorNotReady;
-    static int grid = 0;
-    if (attr == cudaErrorNotReady)
-        attr = sgs::infer_resident(k_stream_collide_mlp<S, HW, LAY>, MLP_ROWS, smem, sgs::tmem_cols<MLP_ROWS>(),
-                                   MLP_BLOCKS, &grid);
+    static sgs::DeviceGrids grids;
+    int grid = 0;
+    const cudaError_t attr = grids.get(
+        [smem](int* g) {
+            return sgs::infer_resident(k_stream_collide_mlp<S, HW, LAY>, MLP_ROWS, smem, sgs::tmem_cols<MLP_ROWS>(),
+                                       MLP_BLOCKS, g);
+        },
+        &grid);
     if (attr != cudaSuccess) return attr;
     const int ntiles = (L.pitch / SC_BX) * ((L.ny + MLP_BY - 1) / MLP_BY) * L.nz;
     k_stream_collide_mlp<S, HW, LAY><<<grid < ntiles ? grid : ntiles, dim3(SC_BX, MLP_BY), smem, s>>>(

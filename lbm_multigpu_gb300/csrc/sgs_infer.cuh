@@ -24,6 +24,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "sgs_mlp.cuh"
 #include "tc_sm103.cuh"
 
@@ -109,6 +111,30 @@ template <class K> inline cudaError_t infer_resident(K kernel, int threads, size
     *grid = (sms > 0 ? sms : 152) * nb;
     return e;
 }
+
+/* the grid that infer_resident gives a kernel on each device, worked out at its
+ * first launch there: the grid and the attributes that are set with it belong
+ * to the device.  Safe with any threads (two at a device's first launch both
+ * work it out, to the same result) */
+class DeviceGrids {
+public:
+    template <class F> cudaError_t get(F make, int* grid) {
+        int dev = 0;
+        if (cudaError_t e = cudaGetDevice(&dev)) return e;
+        if (dev < 0 || dev >= DEVICES) return cudaErrorInvalidDevice;
+        int g = grid_[dev].load(std::memory_order_acquire);
+        if (!g) {
+            if (cudaError_t e = make(&g)) return e;
+            grid_[dev].store(g, std::memory_order_release);
+        }
+        *grid = g;
+        return cudaSuccess;
+    }
+
+private:
+    static constexpr int DEVICES = 64;
+    std::atomic<int> grid_[DEVICES] = {};
+};
 
 #if defined(__CUDA_ARCH__)
 

@@ -601,9 +601,7 @@ cudaError_t launch_shuffle(int* perm, int n, unsigned long long state, int epoch
 cudaError_t launch_mlp_predict_tc(const void* blob, const float* X, int n, float* nu, int* err, cudaStream_t s) {
     const int b = sgs::groups_of(n, 128, 152 * 4);
     const size_t smem = sgs::infer_dyn_smem<128>();
-    static cudaError_t attr = cudaErrorNotReady;
-    if (attr == cudaErrorNotReady)
-        attr = cudaFuncSetAttribute(sgs::k_mlp_predict_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    const cudaError_t attr = cudaFuncSetAttribute(sgs::k_mlp_predict_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (attr != cudaSuccess) return attr;
     TmemLane lane(s);
     if (lane.status() != cudaSuccess) return lane.status();

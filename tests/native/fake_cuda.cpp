@@ -7,7 +7,7 @@
  * function that returns 0 (conftest.py generates them).  Not part of the
  * product library.
  */
-#include <cuda_runtime_api.h>
+#include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
 #include <sys/mman.h>
@@ -16,11 +16,14 @@
 #include <string>
 #include <vector>
 
+#include "../../lbm_multigpu_gb300/csrc/sgs_infer.cuh"
+
 namespace {
 std::map<void*, size_t> g_mem;
 std::map<std::string, long> g_calls, g_fail_at;
 std::map<std::string, size_t> g_fail_above;
 std::vector<long long> g_trace;
+int g_device = 0;
 const int* g_perm = nullptr; /* the permutation that a shuffle last filled */
 
 /* counts the call; true when a test asked for it to fail */
@@ -63,6 +66,21 @@ void fake_reset() {
     g_calls.clear(), g_fail_at.clear(), g_fail_above.clear(), g_trace.clear(), g_perm = nullptr;
 }
 
+/* the grid of one kernel on a device: 100 (device + 1), or an error when `fails` */
+int fake_device_grid(int device, int fails, int* grid) {
+    static lbm::sgs::DeviceGrids grids;
+    g_device = device;
+    const cudaError_t e = grids.get(
+        [&](int* g) {
+            ++g_calls["grid"];
+            *g = 100 * (device + 1);
+            return fails ? cudaErrorUnknown : cudaSuccess;
+        },
+        grid);
+    g_device = 0;
+    return int(e);
+}
+
 cudaError_t cudaMalloc(void** p, size_t n) { return failing("cudaMalloc", n) ? cudaErrorMemoryAllocation : take(p, n); }
 cudaError_t cudaFree(void* p) { return give(p); }
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t) {
@@ -81,7 +99,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 }
 cudaError_t cudaMemset(void* d, int v, size_t n) { return memset(d, v, n), cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return memset(d, v, n), cudaSuccess; }
-cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { return *d = g_device, cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 152, cudaSuccess; }
 cudaError_t cudaDeviceGetStreamPriorityRange(int* a, int* b) { return *a = *b = 0, cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {

@@ -97,3 +97,14 @@ def test_modes_after_a_failed_initialisation(fake, call, before):
         for x, y in zip(got[1:], want[m][1:]):
             np.testing.assert_array_equal(x, y)
     assert fake.lbm_ensemble_destroy(h) == 0
+
+
+def test_closure_grid_is_of_the_device(fake):
+    """the closure kernel's grid, with the function attributes that go with
+    it, is worked out once on each device; a failure is not kept"""
+    g = ctypes.c_int()
+    assert fake.fake_device_grid(1, 1, ctypes.byref(g)) != 0
+    for device in (0, 1, 0, 1, 63):
+        assert fake.fake_device_grid(device, 0, ctypes.byref(g)) == 0 and g.value == 100 * (device + 1)
+    assert fake.fake_calls(b"grid") == 4
+    assert fake.fake_device_grid(64, 0, ctypes.byref(g)) != 0
