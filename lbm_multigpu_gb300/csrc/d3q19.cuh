@@ -49,9 +49,13 @@ __host__ __device__ constexpr float wq(int q) {
  * operations of the FP64 pipe.  That pipe does 2 operations per clock and SM
  * on this chip and bounds the FP64 kernels, so the seeds change format by
  * integer instructions (same exponent range, mantissa cut to 23 bits).
- * Each step squares the seed's relative error of about 2^-21, so the second
- * leaves the rounding of the last operations.  Arguments outside the FP32
- * range take the library functions; IEEE operations on the host. */
+ * With the seed's relative error d, below 2^-21: the reciprocal's steps square
+ * it (d^2, d^4); the square root's share one half-reciprocal of the seed's
+ * precision, so that after the first, which leaves 1.5 d^2, the second gains
+ * one more factor (1.5 d^3).  Both are far below 2^-53 then, which leaves the
+ * rounding of the last operation: within an ulp of the IEEE result, and equal
+ * to it but for near ties.  Arguments outside the FP32 range take the library
+ * functions; IEEE operations on the host. */
 #ifdef __CUDA_ARCH__
 __device__ __forceinline__ bool fp32_range(double x) {
     /* 2^-100 <= x < 2^100, read from the exponent */
