@@ -33,6 +33,12 @@ __device__ __forceinline__ int find_member(const Table& T, int g) {
     return m;
 }
 
+/* Bound by HBM and by the warps in flight: lanes outside the box go through the
+ * collision too (on the rest state), which takes 48 registers (56 with four
+ * rows and no model); left out of it by a `continue`, the kernel took 56 to 64
+ * and a step longer: 16 boxes of 26 M nodes 606 -> 624 us with Smagorinsky,
+ * 604 -> 612 us without, eight boxes of 7 M 169.0 -> 173.4, 167.6 -> 169.8.
+ * Dependent launches: 2 M nodes 60.9 -> 60.5 us, 0.3 M 11.0 -> 10.8. */
 template <int TY, int SGS>
 __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float* __restrict__ fA,
                                                       float* __restrict__ fB, float cs) {
@@ -46,20 +52,28 @@ __global__ void __launch_bounds__(32 * TY) k_ens_step(const Table T, const float
         const int z = local / per_z, r = local - z * per_z;
         const int y = (r / M.tiles_x) * TY + ty, x = (r % M.tiles_x) * 32 + tx;
         const int n = M.n;
-        if (x >= n || y >= n) continue;
+        const bool live = x < n && y < n;
         const unsigned pitch = unsigned(M.pitch), plane = unsigned(n) * pitch, qs = plane * unsigned(n);
         const float* a = fA + M.off;
         float* b = fB + M.off;
         float f[19];
-        const unsigned c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
-        const unsigned xs[3] = {unsigned(x == 0 ? n - 1 : x - 1), unsigned(x), unsigned(x == n - 1 ? 0 : x + 1)};
-        const unsigned yb[3] = {(y == 0 ? n - 1 : y - 1) * pitch, y * pitch, (y == n - 1 ? 0 : y + 1) * pitch};
-        const unsigned zb[3] = {(z == 0 ? n - 1 : z - 1) * plane, z * plane, (z == n - 1 ? 0 : z + 1) * plane};
+        unsigned c = 0;
+        if (live) {
+            c = unsigned(z) * plane + unsigned(y) * pitch + unsigned(x);
+            const unsigned xs[3] = {unsigned(x == 0 ? n - 1 : x - 1), unsigned(x), unsigned(x == n - 1 ? 0 : x + 1)};
+            const unsigned yb[3] = {(y == 0 ? n - 1 : y - 1) * pitch, y * pitch, (y == n - 1 ? 0 : y + 1) * pitch};
+            const unsigned zb[3] = {(z == 0 ? n - 1 : z - 1) * plane, z * plane, (z == n - 1 ? 0 : z + 1) * plane};
 #pragma unroll
-        for (int q = 0; q < 19; ++q) f[q] = __ldg(a + q * qs + zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]);
+            for (int q = 0; q < 19; ++q) f[q] = __ldg(a + q * qs + zb[1 - cz(q)] + yb[1 - cy(q)] + xs[1 - cx(q)]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 19; ++q) f[q] = wq(q);
+        }
         collide_mrt<MRT>(f, M.omega, SGS == SGS_SMAG, cs, 0.f);
+        if (live) {
 #pragma unroll
-        for (int q = 0; q < 19; ++q) b[q * qs + c] = f[q];
+            for (int q = 0; q < 19; ++q) b[q * qs + c] = f[q];
+        }
     }
 }
 
