@@ -567,6 +567,7 @@ int lbm::set_error(int code, const char* what, cudaError_t e) {
 struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     bool steady = false;
+    bool asked = false;     /* a batch of its kind was run (directly, the first time) */
     long long epoch = -1;
     int cur1 = 0;           /* the refinement level's current buffer at the start */
     bool force = false;     /* every step records a force (else none does) */
@@ -603,13 +604,14 @@ struct lbm_handle {
      * coarse level, so it runs beside the coarse stream-collide on this stream */
     cudaStream_t fine = nullptr;
     cudaEvent_t ev_fine0 = nullptr, ev_fine1 = nullptr;
-    /* lbm_step runs batches of 2, 4, 8 or 16 steps as CUDA graphs, which
-     * removes the gaps between their launches.  The step number lives on the
-     * device (step_dev, which a graph advances by its length), so that a
-     * batch is captured once and then launched again with one host call; a
-     * capture costs the host 1 to 10 us per step, more than a step of a small
-     * domain takes.  By log2 of the length, the buffer it starts from and
-     * whether a step of it evaluates the closure */
+    /* lbm_step runs batches of 4, 8 or 16 steps as CUDA graphs (batch_lg),
+     * which removes the gaps between their launches.  The step number lives on
+     * the device (step_dev, which a graph advances by its length), so that a
+     * batch is captured once and then launched again with one host call.  The
+     * first batch of a kind is run directly: a capture costs the host 1 to 10
+     * us per step and the executable as much again, more than a program that
+     * makes one short call gets back.  By log2 of the length, the buffer it
+     * starts from and whether a step of it evaluates the closure */
     StepGraph graphs[5][2][2];
     int* step_dev = nullptr;        /* behind audit_out's four sums */
     int step_dev_val = -1;          /* its value once everything queued so far has run */
@@ -1114,6 +1116,32 @@ int replay_graph(lbm_handle* h, StepGraph& g, int k) {
     h->launches += g.launches;
     h->t += k;
     return join_side(h);
+}
+
+/* whether a step waits for work on another stream (the force reduction, the
+ * fine level, the closure's kernel), which costs 2 to 4 us between two direct
+ * steps; without it the next step's dependent launch hides the gap */
+bool step_branches(const lbm_handle* h) {
+    return h->cfg.refinement || h->cfg.sgs_mlp || (h->lv[0].nbody > 0 && h->t >= h->cfg.startf);
+}
+
+/* log2 of the batch that lbm_step(n) takes as one graph with `left` steps to
+ * go, 0: a direct step.  A graph's beginning and end cost 8 to 20 us (no
+ * launch reaches over them, the step counter is set and advanced), and a
+ * direct step after one as much again.  So, with a branch in the steps, 16 and 8
+ * where they fit (66 K nodes with a body: 9.0 us a direct step, 7.6 in graphs
+ * of 4, 6.2 of 8, 5.9 of 16; 8.4 M nodes: 186.0, 189.3, 185.0, 184.1), and 4
+ * only with refinement, a dozen launches a step (2 M + 0.4 M nodes: 94.1 us, 87.4
+ * in graphs of 4), in calls that it divides.  Without a branch a run of direct
+ * steps is as fast as its graphs (64^3 cavity: 6.27 us, 6.20 in graphs of 16,
+ * 6.74 of 4), so that only long calls take them. */
+int batch_lg(const lbm_handle* h, int n, int left, bool branch) {
+    for (int lg = GRAPH_LG; lg >= 2; --lg) {
+        const int k = 1 << lg;
+        if (k > left || !closure_fits(h, k) || !graph_ok(h, k)) continue;
+        if (lg == 2 ? h->cfg.refinement && left == k && n % k == 0 : branch || (lg == GRAPH_LG && n >= 4 * k)) return lg;
+    }
+    return 0;
 }
 
 /* k = 2^lg steps captured from the main stream into one graph (the force
@@ -1630,23 +1658,20 @@ int lbm_set_populations(lbm_handle* h, int level, const float* f) {
 int lbm_step(lbm_handle* h, int nsteps) {
     if (!h) return fail(LBM_ERR_ARG, "null handle");
     if (nsteps < 0) return fail(LBM_ERR_ARG, "nsteps %d < 0", nsteps);
-    /* the longest batch that fits, when its graph is at hand; else batches
-     * that grow 2, 4, 8, 16, so that the host captures each while the GPU
-     * runs the one before (after one direct step where graphs need it) */
-    int ramp = graph_ok(h, 2) ? 1 : 0;
+    const bool branch = step_branches(h);
     for (int left = nsteps; left > 0;) {
-        int lg = GRAPH_LG, rc;
-        while (lg > 0 && ((1 << lg) > left || !closure_fits(h, 1 << lg))) --lg;
-        StepGraph* g = ready_graph(h, lg);
-        if (!g) {
-            if (lg > ramp) g = ready_graph(h, lg = ramp);
-            ramp = std::min(ramp + 1, GRAPH_LG);
+        const int lg = batch_lg(h, nsteps, left, branch), k = 1 << lg;
+        int rc = LBM_OK;
+        if (StepGraph* g = ready_graph(h, lg)) {
+            rc = replay_graph(h, *g, k);
+        } else if (lg > 0 && graph_slot(h, lg).asked) {
+            rc = run_graph(h, lg);
+        } else {
+            if (lg > 0) graph_slot(h, lg).asked = true;
+            for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h);
         }
-        if (g) rc = replay_graph(h, *g, 1 << lg);
-        else if (lg > 0 && graph_ok(h, 1 << lg)) rc = run_graph(h, lg);
-        else rc = one_step(h), lg = 0;
         if (rc) return rc;
-        left -= 1 << lg;
+        left -= k;
     }
     return LBM_OK;
 }

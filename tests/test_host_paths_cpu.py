@@ -108,3 +108,16 @@ def test_closure_grid_is_of_the_device(fake):
         assert fake.fake_device_grid(device, 0, ctypes.byref(g)) == 0 and g.value == 100 * (device + 1)
     assert fake.fake_calls(b"grid") == 4
     assert fake.fake_device_grid(64, 0, ctypes.byref(g)) != 0
+
+
+@pytest.mark.parametrize("calls,captures", [([5, 20], 0), ([4, 4, 4], 0), ([8, 8, 8], 1), ([20, 20, 20], 1),
+                                            ([20, 640], 1), ([100], 1)])
+def test_short_calls_capture_nothing_they_do_not_use_again(fake, calls, captures):
+    """a batch is captured when one of its kind comes a second time: a first
+    short call is direct steps, and what is captured is launched again"""
+    h = _solver(fake)
+    for n in calls:
+        assert fake.lbm_step(h, n) == 0, fake.lbm_last_error()
+    assert fake.fake_calls(b"cudaStreamBeginCapture") == captures
+    assert fake.fake_calls(b"cudaGraphLaunch") >= captures
+    assert fake.lbm_destroy(h) == 0
