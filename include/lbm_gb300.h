@@ -239,7 +239,10 @@ int lbm_mlp_grad(const float* d_params, const float* d_X, const float* d_T, int 
  * pointers, async */
 int lbm_mlp_predict(const float* d_params, const float* d_X, int n, float* d_nu, void* stream);
 /* Adam (beta 0.9 / 0.999) over seeded shuffled mini-batches of device
- * samples; params (host) in and out, loss_hist[steps] (host, may be NULL) */
+ * samples; params (host) in and out, loss_hist[steps] (host, may be NULL).
+ * Takes 4 bytes of device memory per sample during the call, from 28,672
+ * samples on 20 more where they are to be had (else the shuffle runs on the
+ * host) */
 int lbm_mlp_train(const float* d_X, const float* d_T, int n, int batch, int steps, float lr, uint32_t seed,
                   float* params, float* loss_hist, void* stream);
 /* the coefficient o of n samples through the tensor-core path the collide

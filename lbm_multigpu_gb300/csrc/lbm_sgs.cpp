@@ -12,7 +12,10 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
+#include <utility>
 #include <vector>
 
 #include "../../include/lbm_gb300.h"
@@ -95,6 +98,13 @@ template <class T> struct DevBuf {
         return cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), n * sizeof(T), pool, s);
     }
 };
+
+/* Samples from which a training epoch's shuffle runs on the device: its 51
+ * launches cost 100 to 150 us whatever the size, the host's loop and copy 10 us
+ * and 6 ns a sample.  A step that begins an epoch, device / host: 4,000 samples
+ * 136 / 39 us, 16,384 157 / 114, 28,672 189 / 189, 65,536 232 / 407; with 16
+ * steps an epoch the two meet at 40,000 (29 / 27 us). */
+constexpr int SHUFFLE_DEVICE = 28672;
 
 uint16_t bf16_rne(float f) {
     uint32_t u;
@@ -197,18 +207,32 @@ int lbm_mlp_train(const float* d_X, const float* d_T, int n, int batch, int step
     SGS_TRY(part.alloc(size_t(nb) * (sgs::NPARAM + 1)), "cudaMalloc");
     SGS_TRY(loss.alloc(size_t(steps > 0 ? steps : 1)), "cudaMalloc");
     SGS_TRY(idx.alloc(size_t(n)), "cudaMalloc");
-    SGS_TRY(shuffle.alloc(shuffle_scratch_bytes(n)), "cudaMalloc");
+    /* the shuffle runs on the device; for few samples, or without the device
+     * memory for its scratch (20 bytes a sample), on the host */
+    std::unique_ptr<int[]> perm;
+    if (n < SHUFFLE_DEVICE || shuffle.alloc(shuffle_scratch_bytes(n)) != cudaSuccess) {
+        cudaGetLastError();
+        perm.reset(new (std::nothrow) int[size_t(n)]);
+        if (!perm) return set_error(LBM_ERR_NOMEM, "training: no host memory for the sample order", cudaSuccess);
+        for (int i = 0; i < n; ++i) perm[i] = i;
+    }
     SGS_TRY(cudaMemcpyAsync(P.p, params, sgs::NPARAM * sizeof(float), cudaMemcpyHostToDevice, s), "params upload");
     SGS_TRY(cudaMemsetAsync(M.p, 0, sgs::NPARAM * sizeof(float), s), "memset");
     SGS_TRY(cudaMemsetAsync(V.p, 0, sgs::NPARAM * sizeof(float), s), "memset");
-    /* epochs over a seeded permutation, shuffled on the device; an epoch takes
-     * n - 1 draws */
+    /* epochs over a seeded permutation; an epoch takes n - 1 draws */
     Rng r(seed);
     int pos = n, epoch = 0;
     for (int st = 0; st < steps; ++st) {
         if (batch > n - pos) {
-            SGS_TRY(launch_shuffle(idx.p, n, r.s, epoch++, shuffle.p, s), "shuffle launch");
-            r.skip(uint64_t(n - 1));
+            if (perm) {
+                for (int i = n - 1; i > 0; --i) std::swap(perm[i], perm[r.next() % (uint64_t(i) + 1)]);
+                SGS_TRY(cudaMemcpyAsync(idx.p, perm.get(), size_t(n) * sizeof(int), cudaMemcpyHostToDevice, s),
+                        "index upload");
+                SGS_TRY(cudaStreamSynchronize(s), "index upload");
+            } else {
+                SGS_TRY(launch_shuffle(idx.p, n, r.s, epoch++, shuffle.p, s), "shuffle launch");
+                r.skip(uint64_t(n - 1));
+            }
             pos = 0;
         }
         SGS_TRY(launch_mlp_grad(P.p, d_X, d_T, idx.p + pos, batch, part.p, nb, s), "gradient launch");

@@ -296,4 +296,16 @@ void orc_sgs_targets(const double* ubar, const double* uu, int cx, int cy, int c
             }
 }
 
+/* one epoch of the mini-batch shuffle of perm[n]: Fisher-Yates from the top
+ * with the next n - 1 draws of splitmix64; returns the generator's state */
+uint64_t orc_shuffle(uint64_t state, int* perm, int n) {
+    for (int i = n - 1; i > 0; --i) {
+        uint64_t z = state += 0x9E3779B97F4A7C15ull;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        std::swap(perm[i], perm[(z ^ (z >> 31)) % (uint64_t(i) + 1)]);
+    }
+    return state;
+}
+
 }  // extern "C"

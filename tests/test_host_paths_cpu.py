@@ -121,3 +121,35 @@ def test_short_calls_capture_nothing_they_do_not_use_again(fake, calls, captures
     assert fake.fake_calls(b"cudaStreamBeginCapture") == captures
     assert fake.fake_calls(b"cudaGraphLaunch") >= captures
     assert fake.lbm_destroy(h) == 0
+
+
+@pytest.mark.parametrize("n,epochs,room", [(1, 3, True), (2, 3, True), (4000, 3, True), (28_671, 2, True),
+                                           (28_672, 2, False), (100_003, 2, False)])
+def test_host_shuffle(fake, n, epochs, room):
+    """with few samples, or without device memory for the device's shuffle,
+    training shuffles on the host, in the order of the oracle's shuffle"""
+    from oracle_bindings import oracle
+
+    if not room:
+        fake.fake_fail_above(b"cudaMallocFromPoolAsync", ctypes.c_size_t(8 * n))
+    batch, P, x = (n + 1) // 2, np.zeros(fake.lbm_mlp_param_count(), np.float32), ctypes.c_void_p(16)
+    per = n // batch   # steps an epoch
+    blocks = fake.fake_blocks()
+    assert fake.lbm_mlp_train(x, x, n, batch, per * epochs, ctypes.c_float(1e-3), 9, _ptr(P), None, None) == 0
+    assert fake.fake_calls(b"launch_shuffle") == 0 and fake.fake_blocks() == blocks
+    got = np.zeros(per * epochs * batch, np.int64)
+    assert fake.fake_trace(_ptr(got), len(got)) == len(got)
+    shuffle = oracle().orc_shuffle
+    shuffle.restype, shuffle.argtypes = ctypes.c_uint64, [ctypes.c_uint64, ctypes.c_void_p, ctypes.c_int]
+    state, perm, want = (9 * 0x9E3779B97F4A7C15 + 0x632BE59BD9B4E019) % 2 ** 64, np.arange(n, dtype=np.int32), []
+    for _ in range(epochs):
+        state = shuffle(state, _ptr(perm), n)
+        want.append(perm[:per * batch].copy())
+    np.testing.assert_array_equal(got, np.concatenate(want))
+
+
+def test_device_shuffle_from_its_size_on(fake):
+    """the rule's other side: with room for its scratch the shuffle of 28,672
+    samples is the device's"""
+    _train(fake, 28_672, 28_672, 3)
+    assert fake.fake_calls(b"launch_shuffle") == 3

@@ -465,3 +465,41 @@ def test_closure_step_graphs_are_bit_exact(product):
             out.append((s.populations(), s.forces(steps)))
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n,batch,steps", [(28_672, 1, 28_672), (60_013, 1, 60_013), (28_672, 14_337, 4_100),
+                                           (28_671, 14_336, 40), (262_144, 200_000, 20)])
+def test_shuffle_over_many_samples_is_fisher_yates(product, n, batch, steps):
+    """the device's shuffle and, one sample below its range, the host's:
+    batches of one give each sample's loss, batches of more than half of the
+    samples (every step an epoch) the mean over the first `batch` of the
+    epoch's order; 4,100 epochs pass the clearing of the scratch.  FP32: the
+    loss of index k is off by 2^-22 (k + 1)^2 at most, a mean of them by a few
+    1e-6 of itself; the mean over another half of the samples is some
+    0.5 / sqrt(batch) = 1e-3 away"""
+    torch = pytest.importorskip("torch")
+    lib = product.library()
+    X = np.zeros((n, NIN), np.float32)
+    X[:, 15] = 1
+    T = ((1 + np.arange(n)) * np.float32(1e-4)).astype(np.float32)
+    P, hist = _params(lib, 3), np.zeros(steps, np.float32)
+    dX, dT = _dev(torch, X), _dev(torch, T)
+    at = lambda t: ctypes.c_void_p(t.data_ptr())
+    o, dP = torch.zeros(n, device="cuda"), _dev(torch, P)
+    assert lib.lbm_mlp_predict(at(dP), at(dX), n, at(o), None) == 0
+    torch.cuda.synchronize()
+    base = float(o[0].item()) / 1e-4
+    assert lib.lbm_mlp_train(at(dX), at(dT), n, batch, steps, ctypes.c_float(1e-30), 9, ptr(P), ptr(hist),
+                             None) == 0, lib.lbm_last_error()
+    shuffle = oracle().orc_shuffle
+    shuffle.restype, shuffle.argtypes = ctypes.c_uint64, [ctypes.c_uint64, ctypes.c_void_p, ctypes.c_int]
+    state, perm = (9 * 0x9E3779B97F4A7C15 + 0x632BE59BD9B4E019) % 2 ** 64, np.arange(n, dtype=np.int32)
+    loss, want = (base - (1 + np.arange(n))) ** 2, []
+    for _ in range(1 if batch == 1 else steps):
+        state = shuffle(state, ptr(perm), n)
+        want.append(loss[perm] if batch == 1 else [loss[perm[:batch]].mean()])
+    want = np.concatenate(want)
+    if batch == 1:   # roots: one apart from sample to sample, off by 2^-23 (k + 1)
+        np.testing.assert_allclose(np.sqrt(hist.astype(np.float64)), np.sqrt(want), rtol=0, atol=0.02 + 1e-6 * n)
+    else:
+        np.testing.assert_allclose(hist, want, rtol=1e-5)
