@@ -221,13 +221,14 @@ __global__ void __launch_bounds__(GTH, 2) k_mlp_grad(const float* __restrict__ p
             gd3 += dy;
         }
         __syncthreads();
-        /* dz2 = dy w3 relu'(z2) */
+        /* dz2 = dy w3 relu'(z2); slopes are factors, so that a dy that is not a
+         * number reaches every weight */
         const float4 dy = ld4(s.dy + q0);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float w3 = s.w3[u0 + j];
-            const float4 d = make_float4(h2[j][0] > 0.f ? dy.x * w3 : 0.f, h2[j][1] > 0.f ? dy.y * w3 : 0.f,
-                                         h2[j][2] > 0.f ? dy.z * w3 : 0.f, h2[j][3] > 0.f ? dy.w * w3 : 0.f);
+            const float4 d = make_float4(dy.x * (h2[j][0] > 0.f ? w3 : 0.f), dy.y * (h2[j][1] > 0.f ? w3 : 0.f),
+                                         dy.z * (h2[j][2] > 0.f ? w3 : 0.f), dy.w * (h2[j][3] > 0.f ? w3 : 0.f));
             *reinterpret_cast<float4*>(s.d2 + (u0 + j) * LS + q0) = d;
             gb2[j] += (d.x + d.y) + (d.z + d.w);
             gw3[j] += (dy.x * h2[j][0] + dy.y * h2[j][1]) + (dy.z * h2[j][2] + dy.w * h2[j][3]);
@@ -244,8 +245,8 @@ __global__ void __launch_bounds__(GTH, 2) k_mlp_grad(const float* __restrict__ p
             const float4 h = ld4(s.h1 + (u0 + j) * LS + q0);
             const bool on = u0 + j != HC;
             *reinterpret_cast<float4*>(s.d1 + (u0 + j) * LS + q0) =
-                make_float4(on && h.x > 0.f ? h2[j][0] : 0.f, on && h.y > 0.f ? h2[j][1] : 0.f,
-                            on && h.z > 0.f ? h2[j][2] : 0.f, on && h.w > 0.f ? h2[j][3] : 0.f);
+                make_float4(h2[j][0] * (on && h.x > 0.f ? 1.f : 0.f), h2[j][1] * (on && h.y > 0.f ? 1.f : 0.f),
+                            h2[j][2] * (on && h.z > 0.f ? 1.f : 0.f), h2[j][3] * (on && h.w > 0.f ? 1.f : 0.f));
         }
         outer_tile<8, 8, 4, 16>(s.d2, r2, s.h1, c2, g2); /* dW2 = dz2 h1^T */
         __syncthreads();

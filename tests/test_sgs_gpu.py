@@ -503,3 +503,28 @@ def test_shuffle_over_many_samples_is_fisher_yates(product, n, batch, steps):
         np.testing.assert_allclose(np.sqrt(hist.astype(np.float64)), np.sqrt(want), rtol=0, atol=0.02 + 1e-6 * n)
     else:
         np.testing.assert_allclose(hist, want, rtol=1e-5)
+
+
+@pytest.mark.parametrize("where", ["nan target", "inf target", "nan feature"])
+def test_mlp_gradient_of_values_that_are_no_numbers(product, where):
+    """one such value among the samples: the gradient is not finite where the
+    oracle's is not (a bad target reaches every weight, also through units
+    whose ReLU is off), and the loss is as the oracle's"""
+    torch = pytest.importorskip("torch")
+    lib = product.library()
+    n = 200
+    P = _params(lib, 7)
+    X, T = _data(n, 2)
+    if where.endswith("target"):
+        T[77] = np.nan if where.startswith("nan") else np.inf
+    else:
+        X[77, 12] = np.nan
+    dP, dX, dT = _dev(torch, P), _dev(torch, X), _dev(torch, T)
+    g = torch.zeros(NPARAM + 1, dtype=torch.float32, device="cuda")
+    at = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert lib.lbm_mlp_grad(at(dP), at(dX), at(dT), n, at(g), at(g[NPARAM:]), None) == 0, lib.lbm_last_error()
+    go, lo = np.zeros(NPARAM), ctypes.c_double()
+    oracle().orc_mlp_grad(ptr(P), ptr(X), ptr(T), n, ptr(go), ctypes.byref(lo))
+    gg = g.cpu().numpy().astype(np.float64)
+    np.testing.assert_array_equal(np.isfinite(gg[:NPARAM]), np.isfinite(go))
+    assert not np.isfinite(go).all() and np.isfinite(gg[NPARAM]) == np.isfinite(lo.value)
