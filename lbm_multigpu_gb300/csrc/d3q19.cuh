@@ -634,14 +634,12 @@ template <class T> __host__ __device__ __forceinline__ void mrt_pop_relax(T f[19
                      ra = make_float2(Ra, Ra), rd = make_float2(Rd, Rd);
         /* E + O w and E - O w, with the density's share r rho */
         auto pair = [&](float2 E, float2 O, float2 w, float2 n, float2 r, T& p0, T& p1, T& m0, T& m1) {
-            float2 P = pfma(O, w, E), M = pfma(O, n, E);
-            if (LAST) P = pfma(rr, r, P), M = pfma(rr, r, M);
+            const float2 P = pfma(rr, r, pfma(O, w, E)), M = pfma(rr, r, pfma(O, n, E));
             p0 = P.x, p1 = P.y, m0 = M.x, m1 = M.y;
         };
         pair(make_float2(ex, ey), make_float2(jx, jy), wa, na, ra, f[1], f[2], f[3], f[4]);
-        f[9] = ez + WA * jz;
-        f[14] = ez - WA * jz;
-        if (LAST) f[9] += Ra * rho, f[14] += Ra * rho;
+        f[9] = ez + WA * jz + Ra * rho;
+        f[14] = ez - WA * jz + Ra * rho;
         /* xy: (5,7), (6,8); xz: (10,17), (12,15); yz: (11,18), (13,16) */
         pair(pfma(make_float2(t13, t13), qq, make_float2(bxy, bxy)), make_float2(jx + jy, jy - jx), wd, nd, rd, f[5], f[6],
              f[7], f[8]);

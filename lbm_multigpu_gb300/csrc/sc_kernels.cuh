@@ -237,10 +237,9 @@ __device__ __forceinline__ bool sc_in_band(const Level& L, const StepParams& p, 
  * the projected collision has by then, and f is its neighbour's as stored */
 template <class S, int LAY, bool DEVMRT, bool NUBUF>
 __device__ __forceinline__ void sc_collide_store(const Level& L, const StepParams& p, S* __restrict__ fB,
-                                                 float* __restrict__ stats, float* __restrict__ mom_export,
-                                                 const NodeIdx<LAY>& n, typename Fmt<S>::T f[19], unsigned c,
-                                                 const int x, const int y, const int z, const int bc,
-                                                 const typename Fmt<S>::T uin) {
+                                                 float* __restrict__ stats, const NodeIdx<LAY>& n,
+                                                 typename Fmt<S>::T f[19], unsigned c, const int x, const int y,
+                                                 const int z, const int bc, const typename Fmt<S>::T uin) {
     using T = typename Fmt<S>::T;
     constexpr bool DEV = LBM_SC_DEV && sizeof(S) == 2;
     const unsigned qs = unsigned(L.qstride);
@@ -427,8 +426,8 @@ __device__ __forceinline__ void sc_finish(const Level& L, const StepParams& p, c
                 for (int q = 0; q < 19; ++q) f[q] -= L.off[q];
             }
         }
-        sc_collide_store<S, LAY, (FEAT & FEAT_DEVMRT) != 0, (FEAT & FEAT_NUBUF) != 0>(L, p, fB, stats, mom_export, n,
-                                                                                      f, c, x, y, z, bc, uin);
+        sc_collide_store<S, LAY, (FEAT & FEAT_DEVMRT) != 0, (FEAT & FEAT_NUBUF) != 0>(L, p, fB, stats, n, f, c,
+                                                                                      x, y, z, bc, uin);
     }
     if (p.exp_nx > 0) sc_export<S>(L, p, mom_export, f, x, y, z);
 }
