@@ -256,7 +256,9 @@ int lbm_mlp_train(const float* d_X, const float* d_T, int n, int batch, int step
  * with it) runs on one internal stream per device, ordered after the
  * caller's stream and before its later work, so such kernels never run side
  * by side: two of them sharing an SM could ask for more than its 512 tensor-
- * memory columns.  Calls from several threads are serialised by a lock. */
+ * memory columns.  (Steps replayed from a handle's or an ensemble's graphs run
+ * on its own stream; the closure's kernels fit an SM in any mixture.)  Calls
+ * from several threads are serialised by a lock, captures of steps included. */
 int lbm_mlp_predict_tc(const float* params, const float* d_X, int n, float* d_nu, void* stream);
 /* the weight blob the tensor-core inference stages in shared memory, from
  * a parameter vector (host memory, lbm_mlp_blob_bytes() bytes):

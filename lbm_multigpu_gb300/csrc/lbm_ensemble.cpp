@@ -116,6 +116,7 @@ cudaError_t build_graph(lbm_ensemble* e) {
     drop_graph(e);
     cudaGraph_t g = nullptr;
     if (cudaError_t r0 = lbm::TmemLane::prepare()) return r0;
+    const lbm::TmemHold hold(e->sgs == ens::SGS_MLP);
     cudaError_t r = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal);
     if (r != cudaSuccess) return r;
     const int saved = e->cur;

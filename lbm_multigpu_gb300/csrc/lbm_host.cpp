@@ -1179,17 +1179,21 @@ int run_graph(lbm_handle* h, int lg) {
     sg.force = t0 > c.startf;
     sg.refresh = closure_refresh(h, k);
     sg.mom = mom0;
-    CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LBM_OK;
-    for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h, steady ? j : -1, j > 0);
-    if (rc == LBM_OK && steady && uses_counter(h, sg.force)) {
-        const cudaError_t e = launch_advance_step(h->step_dev, k, h->stream);
-        if (e != cudaSuccess) rc = fail(LBM_ERR_CUDA, "step counter: %s", cudaGetErrorString(e));
-        ++h->launches;
-    }
-    sg.launches = h->launches - launches0;
     cudaGraph_t g = nullptr;
-    const cudaError_t ec = cudaStreamEndCapture(h->stream, &g);
+    cudaError_t ec;
+    {
+        TmemHold hold(c.sgs_mlp);
+        CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+        for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h, steady ? j : -1, j > 0);
+        if (rc == LBM_OK && steady && uses_counter(h, sg.force)) {
+            const cudaError_t e = launch_advance_step(h->step_dev, k, h->stream);
+            if (e != cudaSuccess) rc = fail(LBM_ERR_CUDA, "step counter: %s", cudaGetErrorString(e));
+            ++h->launches;
+        }
+        sg.launches = h->launches - launches0;
+        ec = cudaStreamEndCapture(h->stream, &g);
+    }
     if (rc != LBM_OK || ec != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         cudaGetLastError();

@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(IFACE_THREADS) k_interp_fc(const RefineParams 
  * created on first use and kept for the life of the process */
 namespace {
 constexpr int LANE_DEVICES = 64;
-std::mutex g_lane_mu[LANE_DEVICES];
+std::recursive_mutex g_lane_mu[LANE_DEVICES];
 cudaStream_t g_lane[LANE_DEVICES] = {};
 cudaEvent_t g_lane_in[LANE_DEVICES] = {}, g_lane_out[LANE_DEVICES] = {};
 }  // namespace
@@ -644,6 +644,17 @@ TmemLane::~TmemLane() {
     if (dev_ < 0) return;
     if (lane_ && cudaEventRecord(done_, lane_) == cudaSuccess) cudaStreamWaitEvent(caller_, done_, 0);
     g_lane_mu[dev_].unlock();
+}
+
+TmemHold::TmemHold(bool wanted) {
+    int dev = 0;
+    if (!wanted || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= LANE_DEVICES) return;
+    g_lane_mu[dev].lock();
+    dev_ = dev;
+}
+
+TmemHold::~TmemHold() {
+    if (dev_ >= 0) g_lane_mu[dev_].unlock();
 }
 
 constexpr int storage_code_f32 = STORE_F32, storage_code_f16 = STORE_F16, storage_code_bf16 = STORE_BF16,

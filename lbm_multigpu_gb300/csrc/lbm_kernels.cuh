@@ -243,8 +243,10 @@ int force_scan_partials();
  * work by events, so that no two of them run at the same time on a device.
  * Each such kernel sizes its shared memory so that its own resident blocks
  * never ask an SM for more than its 512 TMEM columns; two different ones
- * side by side could, and tcgen05.alloc would then wait for columns.  The
- * lane is held (a host mutex) from construction to destruction. */
+ * side by side could, and tcgen05.alloc would then wait for columns (a step
+ * graph's kernels replay on their handle's stream; the closure's 96 registers
+ * a thread keep any mixture of them below 6 blocks an SM).  The lane is held
+ * (a host mutex) from construction to destruction, and by a TmemHold. */
 class TmemLane {
 public:
     explicit TmemLane(cudaStream_t caller);
@@ -262,6 +264,21 @@ private:
     cudaEvent_t done_ = nullptr;
     int dev_ = -1;
     cudaError_t err_ = cudaSuccess;
+};
+
+/* Keeps the current device's lane for the calling thread (TmemLane may be
+ * constructed inside).  Held over a stream capture that uses the lane: the lane
+ * is part of the capture from its first kernel to the end, and another thread's
+ * launch on it in between would break into the capture. */
+class TmemHold {
+public:
+    explicit TmemHold(bool wanted);
+    ~TmemHold();
+    TmemHold(const TmemHold&) = delete;
+    TmemHold& operator=(const TmemHold&) = delete;
+
+private:
+    int dev_ = -1;
 };
 
 /* record an error for lbm_last_error(); returns code (lbm_host.cpp) */

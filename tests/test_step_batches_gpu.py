@@ -40,3 +40,41 @@ def test_batches_equal_single_steps(product, kind):
     assert np.isfinite(res[0][0]).all()
     for a, b in zip(*res):
         np.testing.assert_array_equal(a, b)
+
+
+def test_closure_steps_of_several_threads(product):
+    """handles with the closure, each of its own thread, and an ensemble with
+    it, all capturing graphs: every one has the result of a thread alone"""
+    import threading
+
+    lbm = product
+    text, weights = _kind(lbm, "closure_1_fp32"), np.fromfile(lbm.LIB_PATH.parent.parent / WEIGHTS, np.float32)
+
+    def flow():
+        with lbm.Solver(text) as s:
+            for n in (16, 16, 16, 40):
+                s.step(n)
+            return s.populations()
+
+    def boxes():
+        with lbm.Ensemble([32, 16], 0.55, sgs="mlp") as e:
+            e.set_mlp(weights)
+            e.init_turbulence(3)
+            e.step(40)
+            return e.populations(0)
+
+    want, wrong = {f: f() for f in (flow, boxes)}, []
+
+    def work(f):
+        for _ in range(12):
+            try:
+                np.testing.assert_array_equal(f(), want[f])
+            except Exception as e:   # an error code, or another result
+                wrong.append(str(e)[:200])
+
+    threads = [threading.Thread(target=work, args=(f,)) for f in (flow, flow, flow, boxes)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
