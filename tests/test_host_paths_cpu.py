@@ -153,3 +153,25 @@ def test_device_shuffle_from_its_size_on(fake):
     samples is the device's"""
     _train(fake, 28_672, 28_672, 3)
     assert fake.fake_calls(b"launch_shuffle") == 3
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(31, 13, 5), (33, 12, 6), (64, 12, 5), (70, 24, 6)])
+def test_statistics_without_staging_memory(fake, nx, ny, nz):
+    """lbm_get_stats where the device has no room for the packed copy: row by
+    row, without the padding"""
+    import lbm_multigpu_gb300 as lbm
+
+    h, pitch = ctypes.c_void_p(), (nx + 31) // 32 * 32
+    text = lbm.make_inputs(nx, ny, nz, obst1=(8.5, 5.5, 0.0), r1=2.0, re=60.0, umax=0.05, tmax=10, les=1, cs=0.01,
+                           geometry="channel_square", velav=1, start_velav=0, start_velfluc=5)
+    assert fake.lbm_create(text.encode(), ctypes.byref(h)) == 0, fake.lbm_last_error()
+    assert fake.lbm_step(h, 1) == 0
+    got = np.full((4, nz, ny, nx), -1, np.float32)
+    fake.fake_fail(b"cudaMalloc", 1)
+    assert fake.lbm_get_stats(h, 0, _ptr(got)) == 0, fake.lbm_last_error()
+    assert fake.fake_calls(b"cudaMemcpy2DAsync") == 4
+    np.testing.assert_array_equal(got, np.arange(4 * nz * ny * pitch).reshape(4, nz, ny, pitch)[..., :nx])
+    fake.fake_fail(b"cudaMalloc", 1)
+    fake.fake_fail(b"cudaMemcpy2DAsync", 3)
+    assert fake.lbm_get_stats(h, 0, _ptr(got)) != 0
+    assert fake.lbm_destroy(h) == 0

@@ -528,3 +528,46 @@ def test_mlp_gradient_of_values_that_are_no_numbers(product, where):
     gg = g.cpu().numpy().astype(np.float64)
     np.testing.assert_array_equal(np.isfinite(gg[:NPARAM]), np.isfinite(go))
     assert not np.isfinite(go).all() and np.isfinite(gg[NPARAM]) == np.isfinite(lo.value)
+
+
+def test_training_calls_of_several_threads(product):
+    """training, gradients and tensor-core predictions on streams of their own
+    from several threads, whose scratch comes from one pool: each has the
+    result of a call alone, bit for bit"""
+    import threading
+
+    torch = pytest.importorskip("torch")
+    lib = product.library()
+    X, T = _data(40_000, 5)
+    dX, dT, P0 = _dev(torch, X), _dev(torch, T), _params(lib, 5)
+    at = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def run(stream, n):
+        s = ctypes.c_void_p(stream.cuda_stream)
+        P, g, nu = P0.copy(), torch.zeros(NPARAM, device="cuda"), torch.zeros(n, device="cuda")
+        torch.cuda.synchronize()
+        assert lib.lbm_mlp_train(at(dX), at(dT), n, 3000, 20, ctypes.c_float(1e-3), 4, ptr(P), None, s) == 0
+        dP = _dev(torch, P)
+        torch.cuda.synchronize()
+        assert lib.lbm_mlp_grad(at(dP), at(dX), at(dT), n, at(g), None, s) == 0
+        assert lib.lbm_mlp_predict_tc(ptr(P), at(dX), n, at(nu), s) == 0
+        return P, g.cpu().numpy(), nu.cpu().numpy()
+
+    sizes, wrong = (40_000, 20_000, 30_001), []
+    want = {n: run(torch.cuda.Stream(), n) for n in sizes}
+
+    def work(n):
+        try:
+            stream = torch.cuda.Stream()
+            for _ in range(8):
+                for a, b in zip(run(stream, n), want[n]):
+                    np.testing.assert_array_equal(a, b)
+        except Exception as e:
+            wrong.append(str(e)[:200])
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
