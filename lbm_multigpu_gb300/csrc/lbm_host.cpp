@@ -604,7 +604,7 @@ struct lbm_handle {
      * coarse level, so it runs beside the coarse stream-collide on this stream */
     cudaStream_t fine = nullptr;
     cudaEvent_t ev_fine0 = nullptr, ev_fine1 = nullptr;
-    /* lbm_step runs batches of 4, 8 or 16 steps as CUDA graphs (batch_lg),
+    /* lbm_step runs batches of up to 16 steps as CUDA graphs (batch_lg),
      * which removes the gaps between their launches.  The step number lives on
      * the device (step_dev, which a graph advances by its length), so that a
      * batch is captured once and then launched again with one host call.  The
@@ -1132,16 +1132,28 @@ bool step_branches(const lbm_handle* h) {
  * where they fit (66 K nodes with a body: 9.0 us a direct step, 7.6 in graphs
  * of 4, 6.2 of 8, 5.9 of 16; 8.4 M nodes: 186.0, 189.3, 185.0, 184.1), and 4
  * only with refinement, a dozen launches a step (2 M + 0.4 M nodes: 94.1 us, 87.4
- * in graphs of 4), in calls that it divides.  Without a branch a run of direct
+ * in graphs of 4, 91.4 of 2), in calls that it divides; 2 in calls of 2.  Without a branch a run of direct
  * steps is as fast as its graphs (64^3 cavity: 6.27 us, 6.20 in graphs of 16,
  * 6.74 of 4), so that only long calls take them. */
 int batch_lg(const lbm_handle* h, int n, int left, bool branch) {
-    for (int lg = GRAPH_LG; lg >= 2; --lg) {
+    for (int lg = GRAPH_LG; lg > 0; --lg) {
         const int k = 1 << lg;
         if (k > left || !closure_fits(h, k) || !graph_ok(h, k)) continue;
-        if (lg == 2 ? h->cfg.refinement && left == k && n % k == 0 : branch || (lg == GRAPH_LG && n >= 4 * k)) return lg;
+        if (lg <= 2 ? h->cfg.refinement && left == k && (lg == 2 ? n % k == 0 : n == k)
+                    : branch || (lg == GRAPH_LG && n >= 4 * k))
+            return lg;
     }
     return 0;
+}
+
+/* Whether the host captures 2^lg steps while the GPU runs COVER direct ones:
+ * from 4 MB a population on (256 x 64 x 64 FP32 nodes with a body: 29 us a step,
+ * some 100 us for the capture of 16 and its executable; 2 M nodes with
+ * refinement: 94 us, 180 us for 8).  Not with the closure (16: 500 us). */
+constexpr int COVER = 4;
+bool capture_hides(const lbm_handle* h, int lg) {
+    if (h->cfg.sgs_mlp || h->lv[0].L.qstride * storage_bytes(h->storage) < 4 << 20) return false;
+    return lg >= (h->cfg.refinement ? 3 : GRAPH_LG);
 }
 
 /* k = 2^lg steps captured from the main stream into one graph (the force
@@ -1664,10 +1676,20 @@ int lbm_step(lbm_handle* h, int nsteps) {
     if (nsteps < 0) return fail(LBM_ERR_ARG, "nsteps %d < 0", nsteps);
     const bool branch = step_branches(h);
     for (int left = nsteps; left > 0;) {
-        const int lg = batch_lg(h, nsteps, left, branch), k = 1 << lg;
-        int rc = LBM_OK;
-        if (StepGraph* g = ready_graph(h, lg)) {
+        int lg = batch_lg(h, nsteps, left, branch), rc = LBM_OK;
+        StepGraph* g = ready_graph(h, lg);
+        const bool shorter = !g && lg == GRAPH_LG && !graph_slot(h, lg).asked && capture_hides(h, lg - 1);
+        if (shorter) g = ready_graph(h, --lg);
+        int k = 1 << lg;
+        /* behind a graph of 8 the capture of 16 hides */
+        if (shorter && (g || graph_slot(h, lg).asked)) graph_slot(h, GRAPH_LG).asked = true;
+        if (g) {
             rc = replay_graph(h, *g, k);
+        } else if (lg > 0 && left == nsteps && left >= k + COVER && capture_hides(h, lg)) {
+            /* nothing is queued: some direct steps, behind which the capture hides */
+            graph_slot(h, lg).asked = true;
+            k = COVER;
+            for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h);
         } else if (lg > 0 && graph_slot(h, lg).asked) {
             rc = run_graph(h, lg);
         } else {

@@ -175,3 +175,23 @@ def test_statistics_without_staging_memory(fake, nx, ny, nz):
     fake.fake_fail(b"cudaMemcpy2DAsync", 3)
     assert fake.lbm_get_stats(h, 0, _ptr(got)) != 0
     assert fake.lbm_destroy(h) == 0
+
+
+@pytest.mark.parametrize("refined,calls,captures", [(0, [20], 1), (0, [16], 0), (0, [16, 16], 1), (1, [20], 1), (1, [8], 0),
+                                                    (1, [20, 20], 2)])
+def test_captures_of_large_domains_hide_behind_direct_steps(fake, refined, calls, captures):
+    """from 4 MB a population on the first long call captures behind four
+    direct steps (with refinement the graph of 8), and every step is run"""
+    import lbm_multigpu_gb300 as lbm
+
+    h, kw = ctypes.c_void_p(), {}
+    if refined:
+        kw = dict(refinement=1, lr_dims=(64, 48, 32), lr_factor=0.5, lr_origin=(48.25, 20.25, 16.25))
+    text = lbm.make_inputs(256, 64, 64, obst1=(64.5, 31.5, 0.0), r1=4.0, re=60.0, umax=0.05, tmax=1000, les=1, cs=0.01, **kw)
+    assert fake.lbm_create(text.encode(), ctypes.byref(h)) == 0, fake.lbm_last_error()
+    for n in calls:
+        assert fake.lbm_step(h, n) == 0, fake.lbm_last_error()
+    t = ctypes.c_int()
+    assert fake.lbm_get_time(h, ctypes.byref(t)) == 0 and t.value == sum(calls)
+    assert fake.fake_calls(b"cudaStreamBeginCapture") == captures
+    assert fake.lbm_destroy(h) == 0

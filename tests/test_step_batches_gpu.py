@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-CALLS = [4, 4, 4, 8, 8, 12, 12, 20, 20, 3, 64, 17, 96]
+CALLS = [2, 2, 2, 4, 4, 4, 8, 8, 12, 12, 20, 20, 3, 64, 17, 96]
 WEIGHTS = "data/sgs_mlp.bin"
 
 
