@@ -369,7 +369,7 @@ using U64 = unsigned long long;
 __device__ __forceinline__ GridWalk my_walk() { return grid_walk(blockIdx.x, gridDim.x, threadIdx.x, blockDim.x); }
 
 __global__ void k_shuffle_draw(int* __restrict__ H, int n, U64 state) {
-    for (GridWalk w = my_walk(); w.at < n; w.at += w.step) {
+    for (GridWalk w = my_walk(); w.at < unsigned(n); w.at += w.step) {
         const int i = int(w.at);
         U64 z = state + U64(n - i) * 0x9E3779B97F4A7C15ull;
         z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -399,7 +399,7 @@ __global__ void k_shuffle_enter(const int* __restrict__ H, U64* __restrict__ R, 
                                 const int* __restrict__ count, int n, U64 round) {
     pdl_wait();
     const int m = list ? __ldcg(count) : n - 1;
-    for (GridWalk w = my_walk(); w.at < m; w.at += w.step)
+    for (GridWalk w = my_walk(); w.at < unsigned(m); w.at += w.step)
         shuffle_enter(H, R, list ? __ldcg(list + w.at) : int(w.at) + 1, round);
 }
 __global__ void k_shuffle_swap(const int* __restrict__ H, const U64* __restrict__ R, int* perm,
@@ -407,7 +407,7 @@ __global__ void k_shuffle_swap(const int* __restrict__ H, const U64* __restrict_
                                int* __restrict__ left, int* __restrict__ left_count) {
     pdl_wait();
     const int m = list ? __ldcg(count) : n - 1;
-    for (GridWalk w = my_walk(); w.at < m; w.at += w.step) {
+    for (GridWalk w = my_walk(); w.at < unsigned(m); w.at += w.step) {
         const int i = list ? __ldcg(list + w.at) : int(w.at) + 1;
         const bool due = !shuffle_swap(H, R, perm, i, round);
         const unsigned who = __activemask(), ask = __ballot_sync(who, due);
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(1024) k_shuffle_rest(const int* __restrict__ H
     }
 }
 __global__ void k_iota(int* p, int n) {
-    for (GridWalk w = my_walk(); w.at < n; w.at += w.step) p[w.at] = int(w.at);
+    for (GridWalk w = my_walk(); w.at < unsigned(n); w.at += w.step) p[w.at] = int(w.at);
 }
 
 /* ---- tensor-core self-check: D[128][64] = A[128][K] B[64][K]^T, K = 16 * kc */
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(128) k_mlp_predict_tc(const unsigned char* __r
     InferSmem<128>& s = *reinterpret_cast<InferSmem<128>*>(dsm);
     infer_setup<128>(s, blob);
     /* the block's tiles: the same number of passes for all of its threads */
-    for (GridWalk w = grid_walk(blockIdx.x, gridDim.x, 0, 128); w.at < n; w.at += w.step) {
+    for (GridWalk w = grid_walk(blockIdx.x, gridDim.x, 0, 128); w.at < unsigned(n); w.at += w.step) {
         const long long i = w.at + threadIdx.x;
         float x[NIN];
 #pragma unroll

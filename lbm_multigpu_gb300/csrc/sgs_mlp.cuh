@@ -42,14 +42,15 @@ constexpr int OFF_W1 = 0, OFF_W2 = OFF_W1 + NH * NIN, OFF_B2 = OFF_W2 + NH * NH,
               OFF_B3 = OFF_W3 + NH, NPARAM = OFF_B3 + 1;
 constexpr float P_REF = 0.01f, NU_SCALE = 1e-4f;
 
-/* the elements of an array that one thread of a grid takes: at, at + step, ...
- * below the array's size.  64 bits: an array holds up to 2^31 - 1 elements, and
- * the last step goes past its end */
+/* The elements of an array that one thread of a grid takes: at, at + step, ...
+ * below the array's size.  Unsigned, since an array holds up to 2^31 - 1
+ * elements and the last step goes past its end: with `step` threads in the grid,
+ * at most 2^31, at + step stays below 2^32 */
 struct GridWalk {
-    long long at, step;
+    unsigned at, step;
 };
 __host__ __device__ inline GridWalk grid_walk(unsigned block, unsigned blocks, unsigned thread, unsigned threads) {
-    return {(long long)block * threads + thread, (long long)blocks * threads};
+    return {block * threads + thread, blocks * threads};
 }
 /* groups of `per` that n elements fill, up to `most` */
 inline int groups_of(long long n, int per, long long most) {

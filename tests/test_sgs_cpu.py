@@ -361,7 +361,7 @@ def test_bf16_inference_error_is_within_the_gpu_tolerance(product):
 def test_grid_walk_stays_inside_the_array(cellops, n, per, most):
     """the index walk of the shuffle's kernels and of the tensor-core
     prediction (by its blocks' first threads) up to the largest sample count
-    (a 32-bit index wraps in the step past the end from n = 2,147,172,354 and
+    (a signed 32-bit index wraps in the step past the end from n = 2,147,172,354 and
     2,147,405,825 on): every thread stays in 0 .. n - 1 and takes all of its
     elements"""
     step = min((n + per - 1) // per, most) * per
