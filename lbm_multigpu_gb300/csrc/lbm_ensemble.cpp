@@ -242,7 +242,7 @@ int lbm_ensemble_create(int count, const int* sizes, const float* tau0, int sgs,
     }
     e->nelem = off;
     e->nu = uoff;
-    layout(e, ens::tile_height_ok(8, sgs) ? 8 : 4);
+    layout(e, 4);
     if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(set_error(LBM_ERR_CUDA, "ensemble: stream", cudaSuccess));
     cudaEventCreate(&e->e0);
@@ -263,7 +263,11 @@ int lbm_ensemble_create(int count, const int* sizes, const float* tau0, int sgs,
     cudaMemset(e->u, 0, e->nu * sizeof(float));
     if (launch_ens_init_from(e->T, e->u, e->f[0], e->f[1], e->stream) != cudaSuccess)
         return bail(set_error(LBM_ERR_CUDA, "ensemble: init", cudaGetLastError()));
-    e->grid = std::min(e->T.ntiles, ens_step_resident(e->T.ty, sgs));
+    /* The closure's blocks are persistent; without it one tile of four rows a
+     * block, which the autotuner mostly finds too (4.1 M nodes: 93 us a step, a
+     * persistent grid of tiles of eight rows 100 to 117; 55 K nodes 3.8, 4.4
+     * to 5.4) */
+    e->grid = sgs == ens::SGS_MLP ? std::min(e->T.ntiles, ens_step_resident(e->T.ty, sgs)) : e->T.ntiles;
     if (int rc = sync_check(e)) return bail(rc);
     *out = e;
     return LBM_OK;
