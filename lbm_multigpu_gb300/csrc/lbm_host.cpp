@@ -721,23 +721,33 @@ int upload_mask(lbm_handle* h, int level) {
     std::vector<uint32_t> links(halfway ? size_t(L.qstride) : 0, 0u);
     s.has_lid = std::find(s.hmask.begin(), s.hmask.end(), uint8_t(LID)) != s.hmask.end();
     s.has_xbc = std::any_of(s.hmask.begin(), s.hmask.end(), [](uint8_t v) { return v >= DIR_WEST; });
-    /* rows that hold a solid node: away from them a row is its types alone */
-    std::vector<uint8_t> solid_row(size_t(L.ny) * L.nz);
+    /* rows that hold a solid node, and below where in them: lbm_set_mask of a 512 x
+     * 128 x 128 channel takes 306 ms node by node, 59 with a look at the rows, 24 so;
+     * with walls at both ends of every row (160^3 cavity) 146, 149 and 35 */
+    std::vector<uint8_t> solid_row(size_t(L.ny) * L.nz), solid(L.nx);
     for (size_t r = 0; r < solid_row.size(); ++r) {
         const uint8_t* row = s.hmask.data() + r * L.nx;
         solid_row[r] = std::any_of(row, row + L.nx, [](uint8_t v) { return v == WALL || v == BODY; });
     }
     for (int z = 0; z < L.nz; ++z)
         for (int y = 0; y < L.ny; ++y) {
+            /* x next to which any of the nine rows around this one has a solid
+             * node; elsewhere the node is its type alone */
             bool near_row = false;
             for (int dz = -1; dz <= 1; ++dz)
-                for (int dy = -1; dy <= 1; ++dy) near_row |= solid_row[size_t(nb(z + dz, L.nz)) * L.ny + nb(y + dy, L.ny)] != 0;
-            if (!near_row) {
-                memcpy(pitched.data() + size_t(z) * L.plane + size_t(y) * L.pitch,
-                       s.hmask.data() + (size_t(z) * L.ny + y) * L.nx, L.nx);
-                continue;
-            }
+                for (int dy = -1; dy <= 1; ++dy) {
+                    const size_t r = size_t(nb(z + dz, L.nz)) * L.ny + nb(y + dy, L.ny);
+                    if (!solid_row[r]) continue;
+                    if (!near_row) std::fill(solid.begin(), solid.end(), uint8_t(0));
+                    near_row = true;
+                    const uint8_t* row = s.hmask.data() + r * L.nx;
+                    for (int x = 0; x < L.nx; ++x) solid[x] |= uint8_t(row[x] == WALL) | uint8_t(row[x] == BODY);
+                }
+            memcpy(pitched.data() + size_t(z) * L.plane + size_t(y) * L.pitch, s.hmask.data() + (size_t(z) * L.ny + y) * L.nx,
+                   L.nx);
+            if (!near_row) continue;
             for (int x = 0; x < L.nx; ++x) {
+                if (!(solid[nb(x - 1, L.nx)] | solid[x] | solid[nb(x + 1, L.nx)])) continue;
                 const uint8_t t = type_at(x, y, z);
                 const size_t pc = size_t(z) * L.plane + size_t(y) * L.pitch + x;
                 uint8_t m = t;

@@ -12,6 +12,7 @@
 #include <string.h>
 #include <sys/mman.h>
 
+#include <algorithm>
 #include <map>
 #include <string>
 #include <vector>
@@ -25,6 +26,8 @@ std::map<std::string, long> g_calls, g_fail_at;
 std::map<std::string, size_t> g_fail_above;
 std::vector<long long> g_trace;
 int g_device = 0;
+std::vector<uint8_t> g_mask;                   /* of the last step */
+std::vector<uint32_t> g_links, g_body, g_blinks; /* and of the last force */
 const int* g_perm = nullptr; /* the permutation that a shuffle last filled */
 
 /* counts the call; true when a test asked for it to fail */
@@ -63,7 +66,14 @@ long fake_trace(long long* out, long cap) {
     for (long i = 0; i < n && i < cap; ++i) out[i] = g_trace[i];
     return n;
 }
+long fake_mask(uint8_t* out) { return std::copy(g_mask.begin(), g_mask.end(), out) - out; }
+long fake_words(int which, uint32_t* out, long cap) {
+    const std::vector<uint32_t>& v = which == 0 ? g_links : which == 1 ? g_body : g_blinks;
+    for (long i = 0; i < cap && i < long(v.size()); ++i) out[i] = v[i];
+    return long(v.size());
+}
 void fake_reset() {
+    g_body.clear(), g_blinks.clear();
     g_calls.clear(), g_fail_at.clear(), g_fail_above.clear(), g_trace.clear(), g_perm = nullptr;
 }
 
@@ -159,9 +169,18 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) {
 
 namespace lbm {
 int force_partials() { return 608; }
+cudaError_t launch_force(const Level&, const void*, const unsigned* body, int nbody, double*, unsigned*, double*, cudaStream_t,
+                         const uint32_t* blinks, const int*) {
+    if (!body) return cudaErrorInvalidValue;
+    g_body.assign(body, body + nbody);
+    g_blinks.assign(blinks, blinks ? blinks + nbody : blinks);
+    return cudaSuccess;
+}
 /* every word of the statistics is its own index (below 2^24) */
-cudaError_t launch_stream_collide(const Level& L, const StepParams&, const void*, void*, const uint8_t*, float* stats,
-                                  float*, cudaStream_t, const uint32_t*) {
+cudaError_t launch_stream_collide(const Level& L, const StepParams&, const void*, void*, const uint8_t* mask, float* stats,
+                                  float*, cudaStream_t, const uint32_t* links) {
+    g_mask.assign(mask, mask + L.qstride);
+    g_links.assign(links, links ? links + L.qstride : links);
     for (long long i = 0; stats && i < 4 * L.qstride; ++i) stats[i] = float(i);
     return cudaSuccess;
 }

@@ -195,3 +195,62 @@ def test_captures_of_large_domains_hide_behind_direct_steps(fake, refined, calls
     assert fake.lbm_get_time(h, ctypes.byref(t)) == 0 and t.value == sum(calls)
     assert fake.fake_calls(b"cudaStreamBeginCapture") == captures
     assert fake.lbm_destroy(h) == 0
+
+
+@pytest.mark.parametrize("dims", [(64, 24, 6), (33, 7, 5), (31, 5, 3), (70, 9, 4)])
+@pytest.mark.parametrize("bounceback", ["halfway", "fullway"])
+@pytest.mark.parametrize("edge", ["wrap", "clamp"])
+@pytest.mark.parametrize("what", ["walls", "sparse", "body", "none"])
+def test_uploaded_mask_against_brute_force(fake, dims, bounceback, edge, what):
+    """the flag of nodes next to a solid one, their links, and the force list
+    with its links to the body, against a look at all 18 neighbours"""
+    import lbm_multigpu_gb300 as lbm
+    from oracle_bindings import CX, CY, CZ
+
+    nx, ny, nz = dims
+    N, rng = lbm.NODE, np.random.default_rng(nx)
+    m = np.zeros((nz, ny, nx), np.uint8)
+    if what == "walls":      # at both ends of every row
+        m[:, :, 0] = m[:, :, -1] = N["WALL"]
+        m[nz // 2, ny // 2, nx // 2] = N["BODY"]
+    elif what == "sparse":
+        r = rng.random(m.shape)
+        m[r < 0.02], m[r > 0.98], m[(r > 0.5) & (r < 0.52)] = N["WALL"], N["BODY"], N["WEST_INLET"]
+    elif what == "body":
+        m[1:3, 2:4, 5:9] = N["BODY"]
+    h, pitch = ctypes.c_void_p(), (nx + 31) // 32 * 32
+    text = lbm.make_inputs(nx, ny, nz, obst1=(8.5, 2.5, 0.0), r1=1.0, re=60.0, umax=0.05, tmax=10, les=1, cs=0.01,
+                           bounceback=bounceback, edge_pull=edge)
+    assert fake.lbm_create(text.encode(), ctypes.byref(h)) == 0, fake.lbm_last_error()
+    assert fake.lbm_set_mask(h, 0, _ptr(m)) == 0 and fake.lbm_step(h, 2) == 0, fake.lbm_last_error()
+    solid, body = np.isin(m, [N["WALL"], N["BODY"]]), m == N["BODY"]
+    links, blinks = np.zeros(m.shape, np.uint32), np.zeros(m.shape, np.uint32)
+    ax = [np.arange(n) for n in (nz, ny, nx)]
+    take = (lambda i, n: np.clip(i, 0, n - 1)) if edge == "clamp" else (lambda i, n: i % n)
+    for q in range(1, 19):
+        at = np.ix_(take(ax[0] - int(CZ[q]), nz), take(ax[1] - int(CY[q]), ny), take(ax[2] - int(CX[q]), nx))
+        links |= (solid[at] & ~solid).astype(np.uint32) << q
+        blinks |= (body[at] & ~solid).astype(np.uint32) << q
+    got = np.zeros((nz, ny, pitch), np.uint8)
+    assert fake.fake_mask(_ptr(got)) == got.size
+    np.testing.assert_array_equal(got[..., :nx], m | np.where(links != 0, 0x80, 0).astype(np.uint8))
+    assert (got[..., nx:] == N["WALL"]).all()
+
+    def words(which):
+        n = fake.fake_words(which, None, 0)
+        w = np.zeros(n, np.uint32)
+        fake.fake_words(which, _ptr(w), n)
+        return w
+
+    if bounceback == "halfway":
+        np.testing.assert_array_equal(words(0).reshape(nz, ny, pitch)[..., :nx], links)
+        assert not words(0).reshape(nz, ny, pitch)[..., nx:].any()
+        listed = blinks != 0
+        np.testing.assert_array_equal(words(2), blinks[listed])
+    else:
+        listed = body
+        assert words(2).size == 0
+    at = np.zeros((nz, ny, pitch), np.uint32)
+    at.reshape(-1)[:] = np.arange(at.size)
+    np.testing.assert_array_equal(words(1), at[..., :nx][listed])
+    assert fake.lbm_destroy(h) == 0
