@@ -778,19 +778,21 @@ int upload_mask(lbm_handle* h, int level) {
         CUDA_TRY(cudaMalloc(&s.links, links.size() * sizeof(uint32_t)));
         CUDA_TRY(cudaMemcpy(s.links, links.data(), links.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     }
+    /* the list counts only once it is whole on the device, with its links */
+    s.nbody = 0;
     cudaFree(s.body);
     s.body = nullptr;
-    s.nbody = int(list.size());
+    cudaFree(s.blinks);
+    s.blinks = nullptr;
     if (!list.empty()) {
         CUDA_TRY(cudaMalloc(&s.body, list.size() * sizeof(unsigned)));
         CUDA_TRY(cudaMemcpy(s.body, list.data(), list.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
     }
-    cudaFree(s.blinks);
-    s.blinks = nullptr;
     if (!blist.empty()) {
         CUDA_TRY(cudaMalloc(&s.blinks, blist.size() * sizeof(uint32_t)));
         CUDA_TRY(cudaMemcpy(s.blinks, blist.data(), blist.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     }
+    s.nbody = int(list.size());
     return LBM_OK;
 }
 

@@ -254,3 +254,28 @@ def test_uploaded_mask_against_brute_force(fake, dims, bounceback, edge, what):
     at.reshape(-1)[:] = np.arange(at.size)
     np.testing.assert_array_equal(words(1), at[..., :nx][listed])
     assert fake.lbm_destroy(h) == 0
+
+
+@pytest.mark.parametrize("bounceback", ["halfway", "fullway"])
+@pytest.mark.parametrize("nth", [1, 2, 3])
+def test_failed_mask_upload_leaves_no_half_force_list(fake, bounceback, nth):
+    """lbm_set_mask that fails in one of its allocations: no later step
+    reduces a force over a list that is not on the device, or over one without
+    its links"""
+    h, mask = ctypes.c_void_p(), np.zeros((12, 24, 64), np.uint8)
+    import lbm_multigpu_gb300 as lbm
+
+    text = lbm.make_inputs(64, 24, 12, obst1=(18.5, 11.5, 0.0), r1=4.0, re=60.0, umax=0.05, tmax=1000, les=1, cs=0.01,
+                           bounceback=bounceback)
+    assert fake.lbm_create(text.encode(), ctypes.byref(h)) == 0 and fake.lbm_step(h, 3) == 0
+    mask[3:5, 6:9, 20:24] = lbm.NODE["BODY"]
+    fake.fake_fail(b"cudaMalloc", nth)
+    allocations = {"halfway": 3, "fullway": 1}[bounceback]
+    assert (fake.lbm_set_mask(h, 0, _ptr(mask)) != 0) == (nth <= allocations)
+    launches = fake.fake_calls(b"launch_force")
+    fake.lbm_step(h, 2)
+    if fake.fake_calls(b"launch_force") > launches:   # both parts of the list are there
+        assert fake.fake_words(1, None, 0) > 0
+        assert (fake.fake_words(2, None, 0) > 0) == (bounceback == "halfway")
+    assert fake.fake_calls(b"null body list") == 0
+    assert fake.lbm_destroy(h) == 0
