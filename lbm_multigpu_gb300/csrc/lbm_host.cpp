@@ -1142,16 +1142,19 @@ bool step_branches(const lbm_handle* h) {
  * launch reaches over them, the step counter is set and advanced), and a
  * direct step after one as much again.  So, with a branch in the steps, 16 and 8
  * where they fit (66 K nodes with a body: 9.0 us a direct step, 7.6 in graphs
- * of 4, 6.2 of 8, 5.9 of 16; 8.4 M nodes: 186.0, 189.3, 185.0, 184.1), and 4
- * and 2 only with refinement, a dozen launches a step (2 M + 0.4 M nodes: 94.1 us,
- * 87.4 in graphs of 4, 91.4 of 2), in calls that end with one.  Without a
- * branch a run of direct steps is as fast as its graphs (64^3 cavity: 6.27 us,
- * 6.20 in graphs of 16, 6.74 of 4), so that only long calls take them. */
+ * of 4, 6.2 of 8, 5.9 of 16; 8.4 M nodes: 186.0, 189.3, 185.0, 184.1), 4 to end a
+ * longer call of less than half a million nodes (36 steps of 54 K BF16 nodes: 274
+ * us with direct ones instead, 261 so; 1 M nodes lose 1 %), and 4 and 2 with
+ * refinement, a dozen launches a step (2 M + 0.4 M nodes: 94.1 us, 87.4 in graphs
+ * of 4, 91.4 of 2), in calls that end with one.  Without a branch a run of direct
+ * steps is as fast as its graphs (64^3 cavity: 6.27 us, 6.20 in graphs of 16,
+ * 6.74 of 4), so that only long calls take them. */
 int batch_lg(const lbm_handle* h, int n, int left, bool branch) {
     for (int lg = GRAPH_LG; lg > 0; --lg) {
         const int k = 1 << lg;
         if (k > left || !closure_fits(h, k) || !graph_ok(h, k)) continue;
-        if (lg <= 2 ? h->cfg.refinement && n % 2 == 0 : branch || (lg == GRAPH_LG && n >= 4 * k)) return lg;
+        const bool last = lg == 2 && left == k && n % k == 0 && n > k && h->lv[0].L.qstride < 1 << 19;
+        if (lg > 2 ? branch || (lg == GRAPH_LG && n >= 4 * k) : h->cfg.refinement ? n % 2 == 0 : branch && last) return lg;
     }
     return 0;
 }

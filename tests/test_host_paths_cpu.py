@@ -110,7 +110,7 @@ def test_closure_grid_is_of_the_device(fake):
     assert fake.fake_device_grid(64, 0, ctypes.byref(g)) != 0
 
 
-@pytest.mark.parametrize("calls,captures", [([5, 20], 0), ([4, 4, 4], 0), ([8, 8, 8], 1), ([20, 20, 20], 1),
+@pytest.mark.parametrize("calls,captures", [([5, 20], 0), ([4, 4, 4], 0), ([8, 8, 8], 1), ([20, 20, 20], 2),
                                             ([20, 640], 1), ([100], 1)])
 def test_short_calls_capture_nothing_they_do_not_use_again(fake, calls, captures):
     """a batch is captured when one of its kind comes a second time: a first
