@@ -1159,11 +1159,12 @@ int batch_lg(const lbm_handle* h, int n, int left, bool branch) {
     return 0;
 }
 
-/* Whether the host captures 2^lg steps while the GPU runs COVER direct ones:
+/* The direct steps behind which the host captures 2^lg steps, and whether it can:
  * from 4 MB a population on (256 x 64 x 64 FP32 nodes with a body: 29 us a step,
- * some 100 us for the capture of 16 and its executable; 2 M nodes with
- * refinement: 94 us, 180 us for 8).  Not with the closure (16: 500 us). */
-constexpr int COVER = 4;
+ * some 100 us for the capture of 16 and its executable, several times that for
+ * the first of a process; 2 M nodes with refinement: 94 us, 180 us for 8).  Not
+ * with the closure (16: 500 us). */
+int cover_steps(const lbm_handle* h) { return h->cfg.refinement ? 4 : 8; }
 bool capture_hides(const lbm_handle* h, int lg) {
     if (h->cfg.sgs_mlp || h->lv[0].L.qstride * storage_bytes(h->storage) < 4 << 20) return false;
     return lg >= (h->cfg.refinement ? 3 : GRAPH_LG);
@@ -1698,10 +1699,10 @@ int lbm_step(lbm_handle* h, int nsteps) {
         if (shorter && (g || graph_slot(h, lg).asked)) graph_slot(h, GRAPH_LG).asked = true;
         if (g) {
             rc = replay_graph(h, *g, k);
-        } else if (lg > 0 && left == nsteps && left >= k + COVER && capture_hides(h, lg)) {
+        } else if (lg > 0 && left == nsteps && left >= k + cover_steps(h) && capture_hides(h, lg)) {
             /* nothing is queued: some direct steps, behind which the capture hides */
             graph_slot(h, lg).asked = true;
-            k = COVER;
+            k = cover_steps(h);
             for (int j = 0; j < k && rc == LBM_OK; ++j) rc = one_step(h);
         } else if (lg > 0 && graph_slot(h, lg).asked) {
             rc = run_graph(h, lg);

@@ -177,11 +177,11 @@ def test_statistics_without_staging_memory(fake, nx, ny, nz):
     assert fake.lbm_destroy(h) == 0
 
 
-@pytest.mark.parametrize("refined,calls,captures", [(0, [20], 1), (0, [16], 0), (0, [16, 16], 1), (1, [20], 1), (1, [8], 0),
+@pytest.mark.parametrize("refined,calls,captures", [(0, [24], 1), (0, [20], 0), (0, [16, 16], 1), (1, [20], 1), (1, [8], 0),
                                                     (1, [20, 20], 2)])
 def test_captures_of_large_domains_hide_behind_direct_steps(fake, refined, calls, captures):
-    """from 4 MB a population on the first long call captures behind four
-    direct steps (with refinement the graph of 8), and every step is run"""
+    """from 4 MB a population on the first long call captures behind eight
+    direct steps (with refinement four, the graph of 8), and every step is run"""
     import lbm_multigpu_gb300 as lbm
 
     h, kw = ctypes.c_void_p(), {}
